@@ -1,4 +1,5 @@
-"""Generate sdft_twiddles.cuh: exp(-2 pi i t/R), t = 0..R-1, for the in-register DFTs.
+"""Generate sdft_twiddles.cuh: exp(-2 pi i t/R), t = 0..R-1, for the in-register DFTs,
+and sdft_tw_edges.cuh: the same for every compile-time FFT edge, in constant memory.
 
 Each value is computed in 50-digit decimal arithmetic (pi by Machin's
 formula, cos and sin by their Taylor series) and rounded once to the nearest
@@ -6,11 +7,14 @@ double (float(Decimal) rounds correctly), so every constant is the correctly
 rounded double of the exact twiddle.
 
   python gen_twiddles.py > sdft_twiddles.cuh
+  python gen_twiddles.py edges > sdft_tw_edges.cuh
 """
+import sys
 from decimal import Decimal, getcontext
 
 getcontext().prec = 50
 RADICES = (6, 8, 9, 12, 16, 24, 32)
+EDGES = (12, 16, 18, 24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128)
 
 
 def _atan_inv(n):
@@ -74,5 +78,47 @@ def main():
     print("}  // namespace sdft")
 
 
+def edges():
+    off = {}
+    vals = []
+    for n in EDGES:
+        off[n] = len(vals)
+        vals += zip(*twiddles(n))
+    print(f"""// sdft_tw_edges.cuh -- exp(-2 pi i t/N) of the compile-time FFT edges in constant
+// memory: the warps of a pass read one twiddle index at a time, which the constant
+// cache broadcasts without a shared-memory wavefront (generated by gen_twiddles.py;
+// correctly rounded doubles, and those rounded to float).
+#pragma once
+#include <cuda_runtime.h>
+namespace sdft {{
+constexpr int kTwTotal = {len(vals)};
+// offset of edge n's table, -1 without one
+constexpr int tw_off(int n) {{
+  switch (n) {{""")
+    for n in EDGES:
+        print(f"    case {n}: return {off[n]};")
+    print("""    default: return -1;
+  }
+}""")
+    print("static __constant__ double2 c_twd[kTwTotal] = {")
+    print(",\n".join(f"    {{{r!r}, {i!r}}}" for r, i in vals))
+    print("};")
+    print("static __constant__ float2 c_twf[kTwTotal] = {")
+    print(",\n".join(f"    {{(float){r!r}, (float){i!r}}}" for r, i in vals))
+    print("};")
+    print("""template <int N, typename C> struct TwC;
+template <int N> struct TwC<N, float2> {
+  static constexpr int off = tw_off(N);
+  static_assert(off >= 0, "edge without a constant twiddle table");
+  __device__ __forceinline__ float2 operator()(int t) const { return c_twf[off + t]; }
+};
+template <int N> struct TwC<N, double2> {
+  static constexpr int off = tw_off(N);
+  static_assert(off >= 0, "edge without a constant twiddle table");
+  __device__ __forceinline__ double2 operator()(int t) const { return c_twd[off + t]; }
+};
+}  // namespace sdft""")
+
+
 if __name__ == "__main__":
-    main()
+    edges() if sys.argv[1:] == ["edges"] else main()

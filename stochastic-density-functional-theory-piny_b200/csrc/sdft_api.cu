@@ -415,7 +415,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   // inside a loop the previous stage C already packed and c-transformed `cur`
   // into the column scratch; this step's stage C does the same for OUT when
   // another application follows
-  const bool fuse = ctx->fast && ctx->track_omax && !is_fp64(ctx);
+  const bool fuse = ctx->fast && ctx->track_omax && ctx->g.kc_contig;
   const bool have_x = fuse && ctx->x_vec == cur && ctx->x_n == nstate;
   e.Xnext = (fuse && e.pack_next && e.OUT) ? ctx->d_x : nullptr;
   int nl = 3;
@@ -654,7 +654,6 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   if (cudaSetDevice(device) != cudaSuccess) return fail(set_error(SDFT_ERR_CUDA, "cudaSetDevice failed"));
   if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess)
     return fail(set_error(SDFT_ERR_CUDA, "stream create failed"));
-  if (init_const_twiddles()) return fail(set_error(SDFT_ERR_CUDA, "constant twiddle tables"));
   std::vector<int> cpg, cpc, colab;
   int r = build_columns(ctx, cpg, cpc, colab);
   if (r) return fail(r);
@@ -706,7 +705,8 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   g.plane_nt = default_plane_threads(ctx);
   g.ncoef = ncoef; g.ngp = ctx->ngp;
   g.ncols = ctx->cols.ncols; g.ncols_pad = ctx->cols.ncols_pad; g.ncp = ctx->cols.ncp; g.kamax = ctx->cols.kamax;
-  g.nbatch = (g.ncp + kCPB - 1) / kCPB;
+  const int cpb = ctx->fast ? col_cpb(n3) : kCPB;
+  g.nbatch = (g.ncp + cpb - 1) / cpb;
   g.cp_gstart = ctx->d_cp_gstart; g.cp_gcount = ctx->d_cp_gcount; g.col_ab = ctx->d_col_ab;
   g.gkc = ctx->d_gkc; g.ak2 = ctx->d_ak2;
   g.tw1 = ctx->d_tw; g.tw2 = ctx->d_tw + n1; g.tw3 = ctx->d_tw + n1 + n2;
@@ -733,6 +733,50 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
     CKF(cudaMemcpyAsync(ctx->d_kb_rng, rng.data(), n1 * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
     CKF(cudaStreamSynchronize(ctx->st));  // (rng is a local)
     g.kb_rng = ctx->d_kb_rng;
+  }
+  // the column-stage CTAs' points and the kc range of each column (a mirror
+  // column's is the negated one; the (0,0) column holds both halves and G = 0)
+  if (ctx->fast) {
+    std::vector<int> start(g.nbatch + 1, 0);
+    std::vector<int2> items, rng(g.ncols);
+    items.reserve(ncoef);
+    g.kc_contig = 1;
+    auto wrap = [n3](int k) { return k < 0 ? k + n3 : k; };
+    for (int cp = 0; cp < g.ncp; cp++) {
+      const bool zc = cp == g.ncp - 1;
+      const int l = 2 * (cp % cpb), lm = zc ? l : l + 1;
+      auto item = [&](int gi, int k, unsigned flag) {
+        const unsigned m = (unsigned)wrap(k) | (unsigned)wrap(-k) << 8 | (unsigned)l << 16 | (unsigned)lm << 24 | flag;
+        items.push_back(make_int2(gi, (int)m));
+      };
+      int lo = n3, hi = -n3;
+      for (int e = 0; e < cpc[cp]; e++) {
+        const int gi = cpg[cp] + e;
+        item(gi, kc[gi], 0u);
+        lo = std::min(lo, kc[gi]);
+        hi = std::max(hi, kc[gi]);
+      }
+      if (zc) {  // kc > 0 only: its points 1..hi, their mirrors and 0 fill [-hi, hi]
+        item(ncoef - 1, 0, 0x80000000u);
+        hi = std::max(hi, 0);
+        if (hi != cpc[cp]) g.kc_contig = 0;
+        rng[2 * cp] = make_int2(-hi, hi);
+      } else {
+        if (hi - lo + 1 != cpc[cp]) g.kc_contig = 0;
+        rng[2 * cp] = make_int2(lo, hi);
+        rng[2 * cp + 1] = make_int2(-hi, -lo);
+      }
+      start[cp / cpb + 1] = (int)items.size();
+    }
+    if (!g.kc_contig) std::fill(rng.begin(), rng.end(), make_int2(-n3, n3));
+    DMF(ctx->d_item_start, start.size() * sizeof(int));
+    DMF(ctx->d_items, items.size() * sizeof(int2));
+    DMF(ctx->d_kc_rng, rng.size() * sizeof(int2));
+    CKF(cudaMemcpyAsync(ctx->d_item_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+    CKF(cudaMemcpyAsync(ctx->d_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
+    CKF(cudaMemcpyAsync(ctx->d_kc_rng, rng.data(), rng.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
+    CKF(cudaStreamSynchronize(ctx->st));  // (the vectors are locals)
+    g.item_start = ctx->d_item_start; g.items = ctx->d_items; g.kc_rng = ctx->d_kc_rng;
   }
 
   // orbital blocks (zero padded)
@@ -768,7 +812,7 @@ extern "C" int sdft_ctx_destroy(sdft_ctx *ctx) {
                   ctx->d_twf, ctx->d_vp, ctx->d_vks_tmp, ctx->d_pj, ctx->d_bk, ctx->d_w, ctx->d_z,
                   ctx->d_zwork, ctx->d_chi, ctx->d_b1, ctx->d_b2, ctx->d_fnl, ctx->d_acc, ctx->d_coef,
                   ctx->d_x, ctx->d_dots, ctx->d_mom, ctx->d_rho_part, ctx->d_rho, ctx->d_neg, ctx->d_noise_scratch,
-                  ctx->d_enl, ctx->d_red, ctx->d_kb_rng,
+                  ctx->d_enl, ctx->d_red, ctx->d_kb_rng, ctx->d_item_start, ctx->d_items, ctx->d_kc_rng,
                   ctx->d_err, ctx->d_pj_dig, ctx->d_bk_dig, ctx->d_c_dig,
                   ctx->d_z_dig, ctx->d_pj_sc, ctx->d_bk_sc, ctx->d_c_sc, ctx->d_z_sc, ctx->d_rowmax,
                   ctx->d_oz_part, ctx->d_kb_rs, ctx->d_kb_rc, ctx->d_gk, ctx->d_zsave, ctx->d_rowmax3};

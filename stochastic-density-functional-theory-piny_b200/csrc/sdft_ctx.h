@@ -62,6 +62,8 @@ struct sdft_ctx {
   double *d_enl = nullptr;
   double *d_red = nullptr;  // reduction partials + scalars (Lanczos, energies)
   int2 *d_kb_rng = nullptr;  // per plane row: signed kb range of its sphere columns
+  int *d_item_start = nullptr;                    // column-stage CTAs' items (DevGeom)
+  int2 *d_items = nullptr, *d_kc_rng = nullptr;
   // state
   int resident = 0;          // orbitals in d_chi
   int filtered = 0;          // orbitals with results in d_acc

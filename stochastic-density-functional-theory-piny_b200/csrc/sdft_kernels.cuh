@@ -7,7 +7,11 @@
 namespace sdft {
 
 // Column-pair batch of the column stages.
-constexpr int kCPB = 8;          // column pairs per CTA (16 columns)
+constexpr int kCPB = 8;          // column pairs per CTA (16 columns), generic path
+// column pairs per CTA of the compile-time-edge column stages: 1.1 to 1.6
+// thousand points, so that a transform pass has one or two units per thread of
+// 128 and the item phase one or two points, at every edge
+constexpr int col_cpb(int n3) { return n3 >= 72 ? 8 : (n3 >= 48 ? 16 : 32); }
 constexpr int kColThreads = 256; // threads of the column stages
 
 // Device view of the G sphere and FFT grid.
@@ -17,7 +21,11 @@ struct DevGeom {
   int ncoef;            // half sphere + G=0 (last)
   int ngp;              // pitch of one re (or im) block of an orbital
   int ncols, ncols_pad, ncp, kamax;
-  int nbatch;           // ceil(ncp / kCPB)
+  int nbatch;           // column-stage CTAs per orbital pair: ceil(ncp / pairs per CTA)
+  const int *item_start; // [nbatch + 1] first item of each column-stage CTA (compile-time-edge path)
+  const int2 *items;    // the CTAs' sphere points (ColItem, sdft_cols.cuh)
+  const int2 *kc_rng;   // [ncols] signed kc range of each column, or the whole line (kc_contig = 0)
+  int kc_contig;        // every column's points fill its kc range
   const int2 *kb_rng;   // [n1] per plane row a: signed kb range [x, y] of its sphere columns
   int kb_contig;        // every row's columns fill its kb range (else kb_rng is not used)
   int plane_nt;         // FP32 plane stage threads per CTA: 256 or 128

@@ -1,8 +1,8 @@
 // sdft_kernels2.cu -- fast-path FFT stages with compile-time grid edges.
 //
 // Same stage split as sdft_kernels.cu (A: pack + c-FFT, B: plane FFTs x V,
-// C: c-FFT + unpack/epilogue) but every 1-D transform is the two-pass
-// factorised FFT of sdft_fft2.cuh:
+// C: c-FFT + unpack/epilogue; A and C are in sdft_cols.cuh) but every 1-D
+// transform is the two-pass factorised FFT of sdft_fft2.cuh:
 //   stage A writes the c-transformed columns in the permuted real-space
 //   order r = pos_N3(ic) (X row r);
 //   stage B forward-transforms b then a (natural -> permuted), multiplies by
@@ -17,56 +17,9 @@
 #include "sdft_internal.h"
 #include "sdft_kernels.cuh"
 #include "sdft_kernels2.cuh"
+#include "sdft_tw_edges.cuh"
 
 namespace sdft {
-
-// exp(-2 pi i t/N) of every compile-time FFT edge in constant memory (the
-// warps of the plane passes read one twiddle index at a time, which the
-// constant cache broadcasts without a shared-memory wavefront); offsets of
-// the edges 12, 16, 24, 32, 36, 48, 64, 72, 96, 128
-constexpr int kTwEdges[] = {12, 16, 24, 32, 36, 48, 64, 72, 96, 128};
-constexpr int kTwTotal = 528;
-constexpr int tw_off(int n) {
-  int o = 0;
-  for (int e : kTwEdges) {
-    if (e == n) return o;
-    o += e;
-  }
-  return -1;
-}
-template <int N> struct TwOff {
-  static constexpr int value = tw_off(N);
-  static_assert(value >= 0, "edge without a constant twiddle table");
-};
-__constant__ float2 c_twf[kTwTotal];
-__constant__ double2 c_twd[kTwTotal];
-
-template <int N, typename C> struct TwC;
-template <int N> struct TwC<N, float2> {
-  __device__ __forceinline__ float2 operator()(int t) const { return c_twf[TwOff<N>::value + t]; }
-};
-template <int N> struct TwC<N, double2> {
-  __device__ __forceinline__ double2 operator()(int t) const { return c_twd[TwOff<N>::value + t]; }
-};
-
-int init_const_twiddles() {
-  static bool done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-  if (done[dev]) return 0;
-  float2 hf[kTwTotal];
-  double2 hd[kTwTotal];
-  for (int e : kTwEdges)
-    for (int t = 0; t < e; t++) {  // the same values as the context's twiddle tables
-      const double a = 2.0 * M_PI * (double)t / (double)e;
-      hd[tw_off(e) + t] = make_double2(std::cos(a), -std::sin(a));
-      hf[tw_off(e) + t] = make_float2((float)std::cos(a), (float)-std::sin(a));
-    }
-  if (cudaMemcpyToSymbol(c_twf, hf, sizeof hf) != cudaSuccess) return 1;
-  if (cudaMemcpyToSymbol(c_twd, hd, sizeof hd) != cudaSuccess) return 1;
-  done[dev] = true;
-  return 0;
-}
 
 template <typename T> __device__ __forceinline__ const typename CT<T>::type *twp(const DevGeom &g, int d);
 template <> __device__ __forceinline__ const double2 *twp<double>(const DevGeom &g, int d) {
@@ -74,374 +27,6 @@ template <> __device__ __forceinline__ const double2 *twp<double>(const DevGeom 
 }
 template <> __device__ __forceinline__ const float2 *twp<float>(const DevGeom &g, int d) {
   return d == 1 ? g.tw1f : (d == 2 ? g.tw2f : g.tw3f);
-}
-
-// ---------------------------------------------------------------------------
-// stage A
-// ---------------------------------------------------------------------------
-template <typename T, int N3>
-__global__ void __launch_bounds__(kColThreads)
-kf_stage_a(DevGeom g, const double *__restrict__ C, int nstate, int pair0, typename CT<T>::type *__restrict__ X) {
-  using C2 = typename CT<T>::type;
-  constexpr int P3 = N3 + 1;
-  __shared__ __align__(16) C2 buf[2 * kCPB * P3];
-  const int tid = threadIdx.x;
-  const int cp0 = blockIdx.x * kCPB;
-  const int cp1 = min(cp0 + kCPB, g.ncp);
-  const int col0 = 2 * cp0;
-  const int ncl = min(2 * cp1, g.ncols) - col0;
-  const int p = pair0 + blockIdx.y;
-  const int s1 = 2 * p, s2 = 2 * p + 1;
-  const bool has2 = s2 < nstate;
-  for (int i = tid; i < ncl * P3; i += kColThreads) buf[i] = cmk<C2>(0.0, 0.0);
-  __syncthreads();
-  const size_t o1 = (size_t)s1 * 2 * g.ngp, o2 = (size_t)s2 * 2 * g.ngp;
-  const int warp = tid >> 5, lane = tid & 31;
-  for (int cp = cp0 + warp; cp < cp1; cp += kColThreads / 32) {
-    const int lc = 2 * (cp - cp0);
-    const bool zc = (cp == g.ncp - 1);
-    const int lm = zc ? lc : lc + 1;
-    const int gs = g.cp_gstart[cp], gc = g.cp_gcount[cp];
-    for (int e = lane; e < gc; e += 32) {
-      const int gi = gs + e;
-      const int kc = g.gkc[gi];
-      const double a = C[o1 + gi], b = C[o1 + g.ngp + gi];
-      const double c = has2 ? C[o2 + gi] : 0.0, d = has2 ? C[o2 + g.ngp + gi] : 0.0;
-      const int kd = kc < 0 ? kc + N3 : kc;
-      const int km = kc > 0 ? N3 - kc : -kc;
-      buf[lc * P3 + kd] = cmk<C2>(a - d, b + c);
-      buf[lm * P3 + km] = cmk<C2>(a + d, -b + c);
-    }
-    if (zc && lane == 0) {
-      const int g0 = g.ncoef - 1;
-      buf[lc * P3] = cmk<C2>(C[o1 + g0], has2 ? C[o2 + g0] : 0.0);
-    }
-  }
-  __syncthreads();
-  dif<N3, 1, +1>(buf, Lines1{P3}, ncl, TwC<N3, C2>{}, tid, kColThreads);
-  C2 *Xp = X + (size_t)blockIdx.y * N3 * g.ncols_pad;
-  for (int i = tid; i < N3 * ncl; i += kColThreads) {
-    const int r = i / ncl, cl = i - r * ncl;
-    Xp[(size_t)r * g.ncols_pad + col0 + cl] = buf[cl * P3 + r];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// stage C
-// ---------------------------------------------------------------------------
-struct Dots2 { double d0, d1, d2; };
-
-// Writes OUT for orbital s at G index gi and returns the written pair in
-// (wr, wi).
-// HOT: a filter step (Chebyshev or Newton, no moment dots): the noise,
-// H-psi and dot branches are compiled out, which keeps the hot instance
-// within 64 registers without spills.
-template <bool HOT>
-__device__ __forceinline__ void epilogue2(const DevGeom &g, const EpiArgs &e, int s, int gi, bool g0, double fr,
-                                          double fi, Dots2 &dt, double &mx, double &wr, double &wi) {
-  const size_t o = (size_t)s * 2 * g.ngp + gi;
-  if (!HOT && e.mode == EPI_NOISE) {
-    e.OUT[o] = fr;
-    e.OUT[o + g.ngp] = fi;
-    mx = fmax(mx, fmax(absmax_key_d(fr), absmax_key_d(fi)));
-    wr = fr; wi = fi;
-    return;
-  }
-  const double cr = e.C[o], ci = e.C[o + g.ngp];
-  if (e.FNL) {
-    fr += e.FNL[o];
-    fi += e.FNL[o + g.ngp];
-  } else if (e.FNLf) {
-    fr += (double)e.FNLf[o];
-    fi += (double)e.FNLf[o + g.ngp];
-  }
-  if (!g0) {
-    const double k2 = 2.0 * g.ak2[gi];
-    fr -= k2 * cr;
-    fi -= k2 * ci;
-  } else {
-    fi = 0.0;
-  }
-  if (!HOT && e.mode == EPI_HPSI) {
-    e.OUT[o] = fr;
-    e.OUT[o + g.ngp] = fi;
-    mx = fmax(mx, fmax(absmax_key_d(fr), absmax_key_d(fi)));
-    wr = fr; wi = fi;
-    return;
-  }
-  const double sc = g0 ? e.s2 : e.s1;
-  double nr = sc * fr + e.pre * cr;
-  double ni = g0 ? 0.0 : (e.s1 * fi + e.pre * ci);
-  if (e.mode == EPI_CHEBK || e.mode == EPI_MOMK) {
-    nr -= e.PREV[o];
-    if (!g0) ni -= e.PREV[o + g.ngp];
-  }
-  e.OUT[o] = nr;
-  e.OUT[o + g.ngp] = ni;
-  mx = fmax(mx, fmax(absmax_key_d(nr), absmax_key_d(ni)));
-  wr = nr; wi = ni;
-  if (e.ACC) {
-    for (int imu = 0; imu < e.nmu; imu++) {
-      double *A = e.ACC + imu * e.acc_stride;
-      const double a = e.acoef[imu];
-      if (e.acoef0) {
-        const double a0 = e.acoef0[imu];
-        A[o] = a0 * cr + a * nr;
-        A[o + g.ngp] = a0 * ci + a * ni;
-      } else if (e.acoefp) {
-        const double ap = e.acoefp[imu];
-        A[o] += ap * cr + a * nr;
-        A[o + g.ngp] += ap * ci + a * ni;
-      } else {
-        A[o] += a * nr;
-        A[o + g.ngp] += a * ni;
-      }
-    }
-  }
-  if (!HOT && e.dots) {
-    const double wr = g0 ? 1.0 : 2.0;
-    const double xr = e.CHI[o], xi = e.CHI[o + g.ngp];
-    dt.d0 += wr * xr * nr + 2.0 * xi * ni;
-    if (e.mode == EPI_MOMK) {
-      dt.d1 += wr * nr * cr + 2.0 * ni * ci;
-      dt.d2 += wr * nr * nr + 2.0 * ni * ni;
-    } else if (e.ndots > 1) {
-      dt.d1 += wr * xr * xr + 2.0 * xi * xi;
-    }
-  }
-}
-
-// X is not __restrict__: with e.Xnext the CTA overwrites its own columns of
-// the same scratch (read into shared memory at the start) for the next step.
-// Filter-step epilogue for both orbitals of a pair at G index gi: every load
-// of both orbitals is issued before any store (OUT may alias PREV, so a load
-// placed after a store could not be moved above it), which doubles the loads
-// in flight per thread.  Same arithmetic as epilogue2 for CHEB1 / CHEBK /
-// NEWTON without dots; returns the written values (a: s1, b: s2).
-__device__ __forceinline__ void epilogue_pair_hot(const DevGeom &g, const EpiArgs &e, int s1, bool has2, int gi,
-                                                  bool g0, double f1r, double f1i, double f2r, double f2i,
-                                                  double &mx1, double &mx2, double &ar, double &ai, double &br,
-                                                  double &bi) {
-  const size_t n = g.ngp;
-  const size_t o1 = (size_t)s1 * 2 * n + gi, o2 = o1 + 2 * n;
-  const bool rec = e.mode == EPI_CHEBK;
-  const bool acc1 = e.ACC && e.nmu == 1 && !e.acoef0;
-  double c1r = e.C[o1], c1i = e.C[o1 + n], c2r = 0.0, c2i = 0.0;
-  double x1r = 0.0, x1i = 0.0, x2r = 0.0, x2i = 0.0;
-  double p1r = 0.0, p1i = 0.0, p2r = 0.0, p2i = 0.0;
-  double q1r = 0.0, q1i = 0.0, q2r = 0.0, q2i = 0.0;
-  if (has2) { c2r = e.C[o2]; c2i = e.C[o2 + n]; }
-  if (e.FNLf) {
-    x1r = e.FNLf[o1]; x1i = e.FNLf[o1 + n];
-    if (has2) { x2r = e.FNLf[o2]; x2i = e.FNLf[o2 + n]; }
-  } else if (e.FNL) {
-    x1r = e.FNL[o1]; x1i = e.FNL[o1 + n];
-    if (has2) { x2r = e.FNL[o2]; x2i = e.FNL[o2 + n]; }
-  }
-  if (rec) {
-    p1r = e.PREV[o1]; p1i = e.PREV[o1 + n];
-    if (has2) { p2r = e.PREV[o2]; p2i = e.PREV[o2 + n]; }
-  }
-  if (acc1) {
-    q1r = e.ACC[o1]; q1i = e.ACC[o1 + n];
-    if (has2) { q2r = e.ACC[o2]; q2i = e.ACC[o2 + n]; }
-  }
-  const double k2 = g0 ? 0.0 : 2.0 * g.ak2[gi];
-  f1r += x1r - k2 * c1r;
-  f2r += x2r - k2 * c2r;
-  f1i += x1i - k2 * c1i;
-  f2i += x2i - k2 * c2i;
-  const double sc = g0 ? e.s2 : e.s1;
-  ar = sc * f1r + e.pre * c1r;
-  br = sc * f2r + e.pre * c2r;
-  ai = g0 ? 0.0 : (e.s1 * f1i + e.pre * c1i);
-  bi = g0 ? 0.0 : (e.s1 * f2i + e.pre * c2i);
-  if (rec) {
-    ar -= p1r;
-    br -= p2r;
-    if (!g0) { ai -= p1i; bi -= p2i; }
-  }
-  e.OUT[o1] = ar;
-  e.OUT[o1 + n] = ai;
-  mx1 = fmax(mx1, fmax(absmax_key_d(ar), absmax_key_d(ai)));
-  if (has2) {
-    e.OUT[o2] = br;
-    e.OUT[o2 + n] = bi;
-    mx2 = fmax(mx2, fmax(absmax_key_d(br), absmax_key_d(bi)));
-  }
-  if (!e.ACC) return;
-  if (acc1) {
-    const double a = e.acoef[0];
-    const double ap = e.acoefp ? e.acoefp[0] : 0.0;
-    e.ACC[o1] = q1r + ap * c1r + a * ar;
-    e.ACC[o1 + n] = q1i + ap * c1i + a * ai;
-    if (has2) {
-      e.ACC[o2] = q2r + ap * c2r + a * br;
-      e.ACC[o2 + n] = q2i + ap * c2i + a * bi;
-    }
-    return;
-  }
-  for (int k = 0; k < (has2 ? 2 : 1); k++) {
-    const size_t o = k ? o2 : o1;
-    const double cr = k ? c2r : c1r, ci = k ? c2i : c1i, nr = k ? br : ar, ni = k ? bi : ai;
-    for (int imu = 0; imu < e.nmu; imu++) {
-      double *A = e.ACC + imu * e.acc_stride;
-      const double a = e.acoef[imu];
-      if (e.acoef0) {
-        const double a0 = e.acoef0[imu];
-        A[o] = a0 * cr + a * nr;
-        A[o + n] = a0 * ci + a * ni;
-      } else if (e.acoefp) {
-        const double ap = e.acoefp[imu];
-        A[o] += ap * cr + a * nr;
-        A[o + n] += ap * ci + a * ni;
-      } else {
-        A[o] += a * nr;
-        A[o + n] += a * ni;
-      }
-    }
-  }
-}
-
-// 6 CTAs/SM (40 registers, some spilled): latency-bound, the extra resident
-// CTAs measured 4 % faster than 4 CTAs/SM at equal clocks
-// (256 threads x 6 measured ahead of 384 x 4 and 320 x 5: 0.98 against 1.10 and 1.08 ms)
-constexpr int kCThreads = 256, kCMinB = 6;
-template <typename T, int N3, bool HOT>
-__global__ void __launch_bounds__(kCThreads, kCMinB)
-kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
-  using C2 = typename CT<T>::type;
-  constexpr int P3 = N3 + 1;
-  __shared__ __align__(16) C2 buf[2 * kCPB * P3];
-  // packed OUT columns for the next step (e.Xnext; FP32 columns only: the
-  // FP64 instance has no room for a second buffer in static shared memory)
-  constexpr bool kCanPack = sizeof(T) == 4;
-  __shared__ __align__(16) C2 nbuf[kCanPack ? 2 * kCPB * P3 : 1];
-  __shared__ double red[kCThreads / 32][3];
-  const int tid = threadIdx.x;
-  const int cp0 = blockIdx.x * kCPB;
-  const int cp1 = min(cp0 + kCPB, g.ncp);
-  const int col0 = 2 * cp0;
-  const int ncl = min(2 * cp1, g.ncols) - col0;
-  const int p = e.pair0 + blockIdx.y;
-  const int s1 = 2 * p, s2 = 2 * p + 1;
-  const bool has2 = s2 < e.nstate;
-  const C2 *Xp = X + (size_t)blockIdx.y * N3 * g.ncols_pad;
-  for (int i = tid; i < N3 * ncl; i += kCThreads) {
-    const int r = i / ncl, cl = i - r * ncl;
-    buf[cl * P3 + r] = Xp[(size_t)r * g.ncols_pad + col0 + cl];
-  }
-  const bool pack = kCanPack && e.Xnext != nullptr;
-  if (pack)
-    for (int i = tid; i < ncl * P3; i += kCThreads) nbuf[i] = cmk<C2>(0.0, 0.0);
-  // first item (point) of each column pair in the CTA's item list
-  __shared__ int pref[kCPB + 1];
-  if (tid == 0) {
-    int s = 0;
-    for (int k = 0; k < cp1 - cp0; k++) {
-      pref[k] = s;
-      s += g.cp_gcount[cp0 + k] + (cp0 + k == g.ncp - 1 ? 1 : 0);
-    }
-    pref[cp1 - cp0] = s;
-  }
-  __syncthreads();
-  dit<N3, 1, -1>(buf, Lines1{P3}, ncl, TwC<N3, C2>{}, tid, kCThreads);
-  Dots2 dt{0.0, 0.0, 0.0};
-  double mx1 = 0.0, mx2 = 0.0;
-  const int warp = tid >> 5, lane = tid & 31;
-  const double invN = e.invN;
-  const bool noise = !HOT && (e.mode == EPI_NOISE);
-  // one point en of column pair cp
-  auto item = [&](int cp, int en) {
-    const int lc = 2 * (cp - cp0);
-    const bool zc = (cp == g.ncp - 1);
-    const int lm = zc ? lc : lc + 1;
-    const int gs = g.cp_gstart[cp], gc = g.cp_gcount[cp];
-    {
-      if (en < gc) {
-        const int gi = gs + en;
-        const int kc = g.gkc[gi];
-        const int kd = kc < 0 ? kc + N3 : kc;
-        const int km = kc > 0 ? N3 - kc : -kc;
-        const C2 F = buf[lc * P3 + kd], Fm = buf[lm * P3 + km];
-        const double tr = (double)F.x * invN, ti = (double)F.y * invN;
-        const double trc = (double)Fm.x * invN, tic = (double)Fm.y * invN;
-        double f1r, f1i, f2r, f2i;
-        if (!noise) {
-          f1r = -(2.0 * (tr + trc));
-          f1i = -(2.0 * (ti - tic));
-          f2r = -(2.0 * (ti + tic));
-          f2i = -(2.0 * (-tr + trc));
-        } else {
-          f1r = -0.5 * (tr + trc);
-          f1i = -0.5 * (ti - tic);
-          f2r = -0.5 * (ti + tic);
-          f2i = -0.5 * (trc - tr);
-        }
-        double ar, ai, cr2 = 0.0, ci2 = 0.0;
-        if constexpr (HOT) {
-          epilogue_pair_hot(g, e, s1, has2, gi, false, f1r, f1i, f2r, f2i, mx1, mx2, ar, ai, cr2, ci2);
-        } else {
-          epilogue2<HOT>(g, e, s1, gi, false, f1r, f1i, dt, mx1, ar, ai);
-          if (has2) epilogue2<HOT>(g, e, s2, gi, false, f2r, f2i, dt, mx2, cr2, ci2);
-        }
-        if (pack) {  // stage A's packing of the pair (c1 + i c2) at +kc and -kc
-          nbuf[lc * P3 + kd] = cmk<C2>(ar - ci2, ai + cr2);
-          nbuf[lm * P3 + km] = cmk<C2>(ar + ci2, -ai + cr2);
-        }
-      } else {
-        const int g0 = g.ncoef - 1;
-        const C2 F = buf[lc * P3];
-        const double tr = (double)F.x * invN, ti = (double)F.y * invN;
-        const double m = noise ? -1.0 : -2.0;
-        double ar, ai, cr2 = 0.0, ci2 = 0.0;
-        if constexpr (HOT) {
-          epilogue_pair_hot(g, e, s1, has2, g0, true, m * tr, 0.0, m * ti, 0.0, mx1, mx2, ar, ai, cr2, ci2);
-        } else {
-          epilogue2<HOT>(g, e, s1, g0, true, m * tr, 0.0, dt, mx1, ar, ai);
-          if (has2) epilogue2<HOT>(g, e, s2, g0, true, m * ti, 0.0, dt, mx2, cr2, ci2);
-        }
-        if (pack) nbuf[lc * P3] = cmk<C2>(ar, cr2);
-      }
-    }
-  };
-  {  // the CTA's points dealt out over all threads
-    const int tot = pref[cp1 - cp0];
-    for (int it = tid; it < tot; it += kCThreads) {
-      int k = 0;
-      while (k + 1 < cp1 - cp0 && it >= pref[k + 1]) k++;
-      item(cp0 + k, it - pref[k]);
-    }
-  }
-  if (e.omax) {
-    __shared__ double mred[kCThreads / 32][2];
-    omax_flush(e.omax, s1, s2, has2, mx1, mx2, mred);
-  }
-  if (!HOT && e.dots) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      dt.d0 += __shfl_down_sync(0xffffffffu, dt.d0, off);
-      dt.d1 += __shfl_down_sync(0xffffffffu, dt.d1, off);
-      dt.d2 += __shfl_down_sync(0xffffffffu, dt.d2, off);
-    }
-    if (lane == 0) { red[warp][0] = dt.d0; red[warp][1] = dt.d1; red[warp][2] = dt.d2; }
-    __syncthreads();
-    if (tid == 0) {
-      double a = 0.0, b = 0.0, c = 0.0;
-      for (int w = 0; w < kCThreads / 32; w++) { a += red[w][0]; b += red[w][1]; c += red[w][2]; }
-      double *dst = e.dots + ((size_t)p * g.nbatch + blockIdx.x) * 3;
-      dst[0] = a; dst[1] = b; dst[2] = c;
-    }
-  }
-  if (pack) {  // the next application's stage A: forward c-transform, store columns
-    __syncthreads();
-    dif<N3, 1, +1>(nbuf, Lines1{P3}, ncl, TwC<N3, C2>{}, tid, kCThreads);
-    C2 *Xn = reinterpret_cast<C2 *>(e.Xnext) + (size_t)blockIdx.y * N3 * g.ncols_pad;
-    for (int i = tid; i < N3 * ncl; i += kCThreads) {
-      const int r = i / ncl, cl = i - r * ncl;
-      Xn[(size_t)r * g.ncols_pad + col0 + cl] = nbuf[cl * P3 + r];
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -766,8 +351,7 @@ static void plan3(int n3, int &r1, int &r2) {
 
 template <typename T>
 bool fast_stage_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
-  dim3 grid(g.nbatch, npairs);
-#define LA(N) kf_stage_a<T, N><<<grid, kColThreads, 0, st>>>(g, C, nstate, pair0, (typename CT<T>::type *)X)
+#define LA(N) cols_launch_a<T, N>(g, C, nstate, pair0, npairs, X, st)
   SDFT_FOR_N3(LA);
 #undef LA
   return true;
@@ -775,13 +359,7 @@ bool fast_stage_a(const DevGeom &g, const double *C, int nstate, int pair0, int 
 
 template <typename T>
 bool fast_stage_c(const DevGeom &g, const void *X, const EpiArgs &e, int npairs, cudaStream_t st) {
-  dim3 grid(g.nbatch, npairs);
-  const bool hot = e.dots == nullptr && (e.mode == EPI_CHEB1 || e.mode == EPI_CHEBK || e.mode == EPI_NEWTON);
-#define LC(N)                                                                                \
-  do {                                                                                       \
-    if (hot) kf_stage_c<T, N, true><<<grid, kCThreads, 0, st>>>(g, (const typename CT<T>::type *)X, e);  \
-    else kf_stage_c<T, N, false><<<grid, kCThreads, 0, st>>>(g, (const typename CT<T>::type *)X, e);     \
-  } while (0)
+#define LC(N) cols_launch_c<T, N>(g, X, e, npairs, st)
   SDFT_FOR_N3(LC);
 #undef LC
   return true;
@@ -799,7 +377,7 @@ template <typename T>
 bool fast_stage_b(const DevGeom &g, void *X, const T *Vp, int npairs, cudaStream_t st) {
   dim3 grid(g.n3, npairs);
   const size_t sm = pl_smem<T>(g.n1, g.n2);
-  const bool small = std::is_same<T, float>::value && g.plane_nt == 128;
+  [[maybe_unused]] const bool small = g.plane_nt == 128;
   // the j1 = 3, 4 band skipped where both edges factor with R1 = 8 and the
   // sphere is narrower than 3/8 of them (DevGeom::prune34)
 #define LBP(NT_, MB_)                                                                                     \
@@ -813,8 +391,12 @@ bool fast_stage_b(const DevGeom &g, void *X, const T *Vp, int npairs, cudaStream
     constexpr int A = A_, B = B_;                                                                         \
     constexpr bool ok34 = Plan<A>::R1 == 8 && Plan<B>::R1 == 8;                                           \
     const int pm = ok34 ? g.prune34 : 0;                                                                  \
-    if (small) LBP(128, 6);                                                                               \
-    else LBP(PlaneCfg<T>::NT, PlaneCfg<T>::MINB);                                                         \
+    if constexpr (std::is_same<T, float>::value) {                                                        \
+      if (small) LBP(128, 6);                                                                             \
+      else LBP(PlaneCfg<T>::NT, PlaneCfg<T>::MINB);                                                       \
+    } else {                                                                                              \
+      LBP(PlaneCfg<T>::NT, PlaneCfg<T>::MINB);                                                            \
+    }                                                                                                     \
   } while (0)
   SDFT_FOR_PLANE(LB);
 #undef LB

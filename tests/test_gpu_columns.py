@@ -1,0 +1,58 @@
+"""The compile-time-edge FFT stages against the run-time-size ones (the same
+library with SDFT_GENERIC_FFT=1 at context creation), over grids, precisions,
+orbital counts and G lists, including one whose columns have gaps.
+
+Both paths transform with the same arithmetic precision; FP64 results agree to
+a few hundred roundings (1e-12), FP32 transforms (2^-24 per operation, about
+30 operations deep and a handful of applications) to 5e-6."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(wl, grid, reps, holes):
+    s = wl.make_system(reps, grid, strain=(0.01, -0.015, 0.005), disp_sigma=0.05, seed=3)
+    if holes:  # drop interior points of some columns (the list stays grouped by column)
+        drop = np.flatnonzero((s["kc"][:-1] == 1) & (s["kb"][:-1] % 3 == 1))
+        assert len(drop)
+        for k in ("ka", "kb", "kc"):
+            s[k] = np.delete(s[k], drop)
+        s["ncoef"] = len(s["ka"])
+    return s
+
+
+def _results(pkg, s, prec, ns):
+    ctx = pkg.Context(*s["grid"], s["ka"], s["kb"], s["kc"], s["hmat"], precision=prec, max_states=ns)
+    ctx.set_vks(s["vks"])
+    ctx.set_kb(s["kb_desc"])
+    out = {}
+    cr, ci = ctx.genNoiseOrbitalReal(ns, seed=5.0)
+    out["noise"] = np.concatenate([cr, ci])
+    out["hpsi"] = np.concatenate(ctx.calc_coef_force(cr, ci))
+    ec = np.linspace(1.0, 0.2, 14)
+    sre, sim, mom = ctx.filterChebyPolyHerm(cr, ci, ec, 2, 2.0 / 17.5, 2.75, store_moments=True)
+    out["filter"] = np.concatenate(sre + sim)
+    out["stored moments"] = mom[:7]
+    out["one mu"] = np.concatenate(sum(ctx.filterChebyPolyHerm(cr, ci, ec[:6], 1, 2.0 / 17.5, 2.75), []))
+    out["newton"] = np.concatenate(sum(ctx.filterNewtonPolyHerm(cr, ci, ec[:5], np.linspace(-2, 2, 5), 1, 4.0 / 17.5,
+                                                                2.75), []))
+    out["moments"] = ctx.calcChebyMoments(cr, ci, 8, 2.0 / 17.5, 2.75)
+    out["density"] = ctx.rhoCalcRealStoHybrid(cr, ci)
+    ctx.close()
+    return out
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("grid,reps,ns,holes", [
+    ((24, 24, 24), 1, 1, False), ((24, 24, 24), 1, 5, True), ((48, 24, 72), (2, 1, 3), 4, False),
+    ((72, 72, 24), (3, 3, 1), 2, False), ((24, 72, 48), (1, 3, 2), 3, True), ((96, 96, 96), 2, 2, False)])
+def test_compile_time_edges_match_run_time_sizes(pkg, wl, monkeypatch, prec, grid, reps, ns, holes):
+    s = _system(wl, grid, reps, holes)
+    fast = _results(pkg, s, prec, ns)
+    monkeypatch.setenv("SDFT_GENERIC_FFT", "1")
+    slow = _results(pkg, s, prec, ns)
+    for k, v in slow.items():
+        assert rel_l2(fast[k], v) < (1e-12 if prec == 0 or k in ("noise", "density") else 5e-6), k
