@@ -13,7 +13,7 @@ import sys
 from decimal import Decimal, getcontext
 
 getcontext().prec = 50
-RADICES = (6, 8, 9, 12, 16, 24, 32)
+RADICES = (9, 16)
 EDGES = (12, 16, 18, 24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128)
 
 

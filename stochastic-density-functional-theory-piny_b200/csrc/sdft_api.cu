@@ -232,8 +232,11 @@ static int fp64_chunk(sdft_ctx *ctx, int npairs, int *chunk) {
   int r = ensure_x(ctx, std::max(npairs, 2));
   if (r) return r;
   const size_t per = (size_t)ctx->n3 * ctx->cols.ncols_pad * sizeof(double2);
-  *chunk = (int)std::min<size_t>((size_t)npairs, ctx->x_bytes / per);
-  return *chunk >= 1 ? SDFT_OK : set_error(SDFT_ERR_STATE, "column scratch too small");
+  const int fit = (int)std::min<size_t>((size_t)npairs, ctx->x_bytes / per);
+  if (fit < 1) return set_error(SDFT_ERR_STATE, "column scratch too small");
+  const int n = (npairs + fit - 1) / fit;  // as few chunks, evenly filled
+  *chunk = (npairs + n - 1) / n;
+  return SDFT_OK;
 }
 
 static int ensure_coef(sdft_ctx *ctx, size_t n) {
@@ -1191,34 +1194,43 @@ extern "C" int sdft_cheby_moments(sdft_ctx *ctx, int nstate, const double *cre, 
   return moments_core(ctx, nstate, L, scale, emean, moments);
 }
 
+// Partial density grids: pair groups (compile-time-edge path; room for the
+// most that any orbital count of the context takes, so that the buffer never
+// moves under a captured graph), or one grid per pair.
+static int ensure_rho_part(sdft_ctx *ctx, int npairs) {
+  const int n = ctx->fast ? fast_density_max_groups(ctx->g, ctx->npairs_max) : npairs;
+  if (n <= ctx->rho_split) return SDFT_OK;
+  int r = grow(ctx, (void **)&ctx->d_rho_part, (size_t)ctx->rho_split * ctx->N * 8, (size_t)n * ctx->N * sizeof(double));
+  if (!r) ctx->rho_split = n;
+  return r;
+}
+
 // Density of the orbitals held in `vec`.
 static int density_core(sdft_ctx *ctx, const double *vec, int nstate, double scale) {
   int r, chunk;
   const int npairs = (nstate + 1) / 2;
   if ((r = fp64_chunk(ctx, npairs, &chunk))) return r;
-  const int nsplit = npairs;  // one |psi|^2 plane set per pair, summed in pair order
-  if (nsplit > ctx->rho_split) {
-    if ((r = grow(ctx, (void **)&ctx->d_rho_part, (size_t)ctx->rho_split * ctx->N * 8,
-                  (size_t)nsplit * ctx->N * sizeof(double))))
-      return r;
-    ctx->rho_split = nsplit;
-  }
+  const int nsplit = ctx->fast ? fast_density_groups(ctx->g, chunk) : npairs;
+  if ((r = ensure_rho_part(ctx, npairs))) return r;
   if (!ctx->d_rho) DM(ctx->d_rho, (size_t)ctx->N * sizeof(double));
   // one transform per pair (against 2 per pair per filter step): FP64 in
   // every precision, in chunks of pairs that fit the column scratch
   for (int p0 = 0; p0 < npairs; p0 += chunk) {
     const int np = std::min(chunk, npairs - p0);
-    double *part = ctx->d_rho_part + (size_t)p0 * ctx->N;
     if (ctx->fast) {
       { TScope ts(ctx, 0); fast_stage_a<double>(ctx->g, vec, nstate, p0, np, ctx->d_x, ctx->st); }
-      { TScope ts(ctx, 5); fast_stage_b_density<double>(ctx->g, ctx->d_x, np, part, ctx->st); }
+      { TScope ts(ctx, 5); fast_stage_b_density(ctx->g, ctx->d_x, np, nsplit, p0 > 0, ctx->d_rho_part, ctx->st); }
     } else {
       { TScope ts(ctx, 0); launch_stage_a<double>(ctx->g, vec, nstate, p0, np, ctx->d_x, ctx->st); }
-      { TScope ts(ctx, 5); launch_stage_b_density<double>(ctx->g, ctx->d_x, np, np, part, ctx->st); }
+      { TScope ts(ctx, 5); launch_stage_b_density<double>(ctx->g, ctx->d_x, np, np, ctx->d_rho_part + (size_t)p0 * ctx->N, ctx->st); }
     }
     ctx->launches += 2;
   }
-  { TScope ts(ctx, 7); launch_density_reduce(ctx->d_rho_part, nsplit, ctx->N, scale, ctx->d_rho, ctx->st); }
+  {
+    TScope ts(ctx, 7);
+    if (ctx->fast) fast_density_reduce(ctx->g, ctx->d_rho_part, nsplit, scale, ctx->d_rho, ctx->st);
+    else launch_density_reduce(ctx->d_rho_part, nsplit, ctx->N, scale, ctx->d_rho, ctx->st);
+  }
   ctx->launches += 1;
   CK(cudaGetLastError());
   return SDFT_OK;
@@ -1285,7 +1297,7 @@ static int noise_core(sdft_ctx *ctx, int nstate, double seed, int np_states, int
     e.OUT = ctx->d_chi;
     e.invN = 1.0 / (double)ctx->N;
     if (ctx->fast) {
-      { TScope ts(ctx, 6); fast_stage_b_noise<double>(ctx->g, ctx->d_neg, nstate, p0, np, ctx->d_x, ctx->st); }
+      { TScope ts(ctx, 6); fast_stage_b_noise(ctx->g, ctx->d_neg, nstate, p0, np, ctx->d_x, ctx->st); }
       { TScope ts(ctx, 2); fast_stage_c<double>(ctx->g, ctx->d_x, e, np, ctx->st); }
     } else {
       { TScope ts(ctx, 6); launch_stage_b_noise<double>(ctx->g, ctx->d_neg, nstate, p0, np, ctx->d_x, ctx->st); }
@@ -1485,7 +1497,7 @@ out:
 extern "C" int sdft_ctx_set_plane_threads(sdft_ctx *ctx, int nt) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   if (nt != 0 && nt != 128 && nt != 256) return set_error(SDFT_ERR_ARG, "plane_threads: 0 (default), 128 or 256");
-  if (nt == 128 && (is_fp64(ctx) || !ctx->fast))
+  if (nt == 128 && (is_fp64(ctx) || !ctx->fast || !plane_size_settable(ctx->n1, ctx->n2, ctx->n3)))
     return set_error(SDFT_ERR_UNSUPPORTED, "plane_threads: 128 exists for the FP32 fast plane stage only");
   ctx->g.plane_nt = nt == 0 ? default_plane_threads(ctx) : nt;
   return SDFT_OK;
@@ -1546,13 +1558,9 @@ static int prepare_filter(sdft_ctx *ctx, int nstate, int L) {
   if ((r = ensure_coef(ctx, (size_t)L))) return r;
   if ((r = ensure_acc(ctx, 1))) return r;
   const int npairs = (nstate + 1) / 2;
-  if ((r = ensure_x(ctx, std::max(npairs, 2)))) return r;  // as fp64_chunk needs it
-  if (npairs > ctx->rho_split) {
-    if ((r = grow(ctx, (void **)&ctx->d_rho_part, (size_t)ctx->rho_split * ctx->N * 8,
-                  (size_t)npairs * ctx->N * sizeof(double))))
-      return r;
-    ctx->rho_split = npairs;
-  }
+  int chunk;
+  if ((r = fp64_chunk(ctx, npairs, &chunk))) return r;  // also sizes the column scratch
+  if ((r = ensure_rho_part(ctx, npairs))) return r;
   if (!ctx->d_rho && (r = dmalloc(ctx, (void **)&ctx->d_rho, (size_t)ctx->N * sizeof(double)))) return r;
   return SDFT_OK;
 }

@@ -1,4 +1,5 @@
-// sdft_cols_b.cu -- column stages of the edges 72, 96.
+// sdft_cols_b.cu -- column stages of the edges 16, 72, 96.
+#include "sdft_kernels2.cuh"
 #include "sdft_cols.cuh"
 
 namespace sdft {
@@ -7,6 +8,7 @@ namespace sdft {
   template void cols_launch_a<double, N>(const DevGeom &, const double *, int, int, int, void *, cudaStream_t); \
   template void cols_launch_c<float, N>(const DevGeom &, const void *, const EpiArgs &, int, cudaStream_t);     \
   template void cols_launch_c<double, N>(const DevGeom &, const void *, const EpiArgs &, int, cudaStream_t);
+SDFT_COLS(16)
 SDFT_COLS(72)
 SDFT_COLS(96)
 }  // namespace sdft

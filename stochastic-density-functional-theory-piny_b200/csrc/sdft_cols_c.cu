@@ -1,0 +1,15 @@
+// sdft_cols_c.cu -- column stages of the edges 18, 27, 32, 36.
+#include "sdft_kernels2.cuh"
+#include "sdft_cols.cuh"
+
+namespace sdft {
+#define SDFT_COLS(N)                                                                                        \
+  template void cols_launch_a<float, N>(const DevGeom &, const double *, int, int, int, void *, cudaStream_t);  \
+  template void cols_launch_a<double, N>(const DevGeom &, const double *, int, int, int, void *, cudaStream_t); \
+  template void cols_launch_c<float, N>(const DevGeom &, const void *, const EpiArgs &, int, cudaStream_t);     \
+  template void cols_launch_c<double, N>(const DevGeom &, const void *, const EpiArgs &, int, cudaStream_t);
+SDFT_COLS(18)
+SDFT_COLS(27)
+SDFT_COLS(32)
+SDFT_COLS(36)
+}  // namespace sdft

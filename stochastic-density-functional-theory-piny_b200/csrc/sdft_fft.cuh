@@ -22,8 +22,8 @@ template <> struct CT<float> { using type = float2; };
 template <typename C> __device__ __forceinline__ C cmk(double r, double i) {
   C c; c.x = (decltype(c.x))r; c.y = (decltype(c.y))i; return c;
 }
-// FP32 complex arithmetic on the packed f32x2 pipe (sm_100): one
-// instruction per complex add/sub/scale, two per complex multiply.
+// FP32 complex adds, subtracts and scalings as packed f32x2 instructions
+// (sm_100): one issue slot each.
 __device__ __forceinline__ unsigned long long pk2(float x, float y) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -49,11 +49,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk2(a.x, a.y)), "l"(pk2(b.x, b.y)));
   return upk2(r);
 }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a.x, a.y)), "l"(pk2(b.x, b.y)), "l"(pk2(c.x, c.y)));
-  return upk2(r);
-}
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return add2(a, b); }
@@ -62,9 +57,9 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return sub2(a, b); 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// (a.x b.x - a.y b.y, a.x b.y + a.y b.x) = a.x (b.x, b.y) + a.y (-b.y, b.x)
+// four scalar instructions: the packed form needs moves to duplicate and swap halves
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return fma2(make_float2(a.y, a.y), make_float2(-b.y, b.x), mul2(make_float2(a.x, a.x), b));
+  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
 }
 // s * (a.x, a.y) for a real s
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }

@@ -25,25 +25,44 @@
 
 namespace sdft {
 
+// R1 x R2 of every edge with a compile-time plan
 template <int N> struct Plan;
-template <> struct Plan<12> { static constexpr int R1 = 4, R2 = 3; };
-template <> struct Plan<16> { static constexpr int R1 = 4, R2 = 4; };
-template <> struct Plan<24> { static constexpr int R1 = 4, R2 = 6; };
-template <> struct Plan<32> { static constexpr int R1 = 4, R2 = 8; };
-template <> struct Plan<36> { static constexpr int R1 = 6, R2 = 6; };
-template <> struct Plan<48> { static constexpr int R1 = 8, R2 = 6; };
-template <> struct Plan<64> { static constexpr int R1 = 8, R2 = 8; };
-template <> struct Plan<72> { static constexpr int R1 = 8, R2 = 9; };
-template <> struct Plan<96> { static constexpr int R1 = 8, R2 = 12; };
-template <> struct Plan<128> { static constexpr int R1 = 8, R2 = 16; };
+#define SDFT_PLAN(N, A, B) \
+  template <> struct Plan<N> { static constexpr int R1 = A, R2 = B; };
+SDFT_PLAN(12, 4, 3)
+SDFT_PLAN(16, 4, 4)
+SDFT_PLAN(18, 3, 6)
+SDFT_PLAN(24, 4, 6)
+SDFT_PLAN(27, 3, 9)
+SDFT_PLAN(32, 4, 8)
+SDFT_PLAN(36, 6, 6)
+SDFT_PLAN(48, 8, 6)
+SDFT_PLAN(54, 6, 9)
+SDFT_PLAN(64, 8, 8)
+SDFT_PLAN(72, 8, 9)
+SDFT_PLAN(81, 9, 9)
+SDFT_PLAN(96, 8, 12)
+SDFT_PLAN(108, 9, 12)
+SDFT_PLAN(128, 8, 16)
+#undef SDFT_PLAN
+// X(N) for every such edge
+#define SDFT_EDGES(X) \
+  X(12) X(16) X(18) X(24) X(27) X(32) X(36) X(48) X(54) X(64) X(72) X(81) X(96) X(108) X(128)
 
-// position of (frequency or real-space) index k after a dif() pass pair
-template <int N> __device__ __forceinline__ int pos(int k) {
-  return Plan<N>::R2 * (k % Plan<N>::R1) + k / Plan<N>::R1;
-}
-// index stored at position p
-template <int N> __device__ __forceinline__ int ipos(int p) {
-  return (p % Plan<N>::R2) * Plan<N>::R1 + p / Plan<N>::R2;
+// the plan of edge n at run time (r1 = 0: no plan)
+struct PlanRt {
+  int r1, r2;
+  // position of index k after a dif() pass pair, and the index at position p
+  __host__ __device__ __forceinline__ int pos(int k) const { return r2 * (k % r1) + k / r1; }
+  __host__ __device__ __forceinline__ int ipos(int p) const { return (p % r2) * r1 + p / r2; }
+};
+inline PlanRt plan_rt(int n) {
+  switch (n) {
+#define SDFT_P(N) case N: return PlanRt{Plan<N>::R1, Plan<N>::R2};
+    SDFT_EDGES(SDFT_P)
+#undef SDFT_P
+    default: return PlanRt{0, 0};
+  }
 }
 
 template <int R> __device__ __forceinline__ double twc_re(int t);
@@ -51,26 +70,132 @@ template <int R> __device__ __forceinline__ double twc_im(int t);
 #define SDFT_TW(R)                                                                         \
   template <> __device__ __forceinline__ double twc_re<R>(int t) { return kTw##R##re[t]; } \
   template <> __device__ __forceinline__ double twc_im<R>(int t) { return kTw##R##im[t]; }
-SDFT_TW(6)
-SDFT_TW(8)
 SDFT_TW(9)
-SDFT_TW(12)
 SDFT_TW(16)
-SDFT_TW(24)
-SDFT_TW(32)
 #undef SDFT_TW
 
-template <int R> struct F1 { static constexpr int A = (R % 4 == 0 && R > 4) ? 4 : ((R % 3 == 0) ? 3 : 2); };
+// The register DFTs count instructions, not only flops: the plane stage is
+// bound by issue slots.  A packed f32x2 add is one slot but two cycles of the
+// FP32 pipe (measured: 37.0 T element-adds/s packed, 36.2 scalar), and an
+// operand that needs its halves swapped, negated or duplicated first costs
+// moves; so plain complex adds and subtracts are packed, and everything with
+// a rotation or a twiddle is scalar, fused into multiply-adds where it can be.
 
-// In-register R-point DFT, natural order in and out, sign DIR.
-template <int R, int DIR, typename C> __device__ __forceinline__ void dftr(C *v) {
+// a + DIR i b and a - DIR i b
+template <int DIR, typename C> __device__ __forceinline__ C add_i(C a, C b) {
+  C r;
+  if (DIR > 0) { r.x = a.x - b.y; r.y = a.y + b.x; } else { r.x = a.x + b.y; r.y = a.y - b.x; }
+  return r;
+}
+template <int DIR, typename C> __device__ __forceinline__ C sub_i(C a, C b) { return add_i<-DIR>(a, b); }
+// a + s b with s = exp(DIR 2 pi i/8) sqrt(2) b folded in: g = b (1 + DIR i)
+template <int DIR, typename C> __device__ __forceinline__ C rot8(C b) { return add_i<DIR>(b, b); }
+__device__ __forceinline__ double2 axpy(double s, double2 x, double2 y) { return make_double2(fma(s, x.x, y.x), fma(s, x.y, y.y)); }
+__device__ __forceinline__ float2 axpy(float s, float2 x, float2 y) { return make_float2(fmaf(s, x.x, y.x), fmaf(s, x.y, y.y)); }
+// w b with the compile-time twiddle w = exp(DIR 2 pi i e/R)
+template <int R, int DIR, typename C> __device__ __forceinline__ C twmul(C b, int e) {
+  using T = decltype(b.x);
+  if (e == 0) return b;
+  if (4 * e == R) return mul_i<DIR>(b);
+  if (8 * e == R || 8 * e == 3 * R) {  // (+-1 + DIR i) / sqrt(2)
+    const T h = (T)0.70710678118654752440084436210485;
+    const C g = 8 * e == R ? rot8<DIR>(b) : mul_i<DIR>(rot8<DIR>(b));
+    C r;
+    r.x = g.x * h; r.y = g.y * h;
+    return r;
+  }
+  C w;
+  w.x = (T)twc_re<R>(e);
+  w.y = (T)(DIR < 0 ? twc_im<R>(e) : -twc_im<R>(e));
+  return cmul(b, w);
+}
+
+template <int DIR, typename C> __device__ __forceinline__ void dft3(C &v0, C &v1, C &v2) {
+  using T = decltype(v0.x);
+  const T hs = (T)(DIR * 0.86602540378443864676372317075294);  // sqrt(3)/2
+  const C s = cadd(v1, v2), d = csub(v1, v2);
+  const C m = axpy((T)-0.5, s, v0);
+  v0 = cadd(v0, s);
+  v1.x = m.x - hs * d.y; v1.y = m.y + hs * d.x;
+  v2.x = m.x + hs * d.y; v2.y = m.y - hs * d.x;
+}
+template <int DIR, typename C> __device__ __forceinline__ void dft4(C &v0, C &v1, C &v2, C &v3) {
+  const C a0 = cadd(v0, v2), a1 = csub(v0, v2), b0 = cadd(v1, v3), b1 = csub(v1, v3);
+  v0 = cadd(a0, b0);
+  v2 = csub(a0, b0);
+  v1 = add_i<DIR>(a1, b1);
+  v3 = sub_i<DIR>(a1, b1);
+}
+// 8 points; Z34: v[3] and v[4] are zero on input (never read)
+template <int DIR, bool Z34, typename C> __device__ __forceinline__ void dft8(C *v) {
+  using T = decltype(v[0].x);
+  const T h = (T)0.70710678118654752440084436210485;
+  const C s0 = Z34 ? v[0] : cadd(v[0], v[4]), d0 = Z34 ? v[0] : csub(v[0], v[4]);
+  const C s1 = cadd(v[1], v[5]), d1 = csub(v[1], v[5]);
+  const C s2 = cadd(v[2], v[6]), d2 = csub(v[2], v[6]);
+  const C s3 = Z34 ? v[7] : cadd(v[3], v[7]);
+  const C a0 = cadd(s0, s2), a1 = csub(s0, s2), b0 = cadd(s1, s3), b1 = csub(s1, s3);
+  C f0, f1;  // d1 +- DIR i d3
+  if (Z34) {  // d3 = -v[7]
+    f0 = sub_i<DIR>(d1, v[7]);
+    f1 = add_i<DIR>(d1, v[7]);
+  } else {
+    const C d3 = csub(v[3], v[7]);
+    f0 = add_i<DIR>(d1, d3);
+    f1 = sub_i<DIR>(d1, d3);
+  }
+  const C e0 = add_i<DIR>(d0, d2), e1 = sub_i<DIR>(d0, d2);
+  const C g0 = rot8<DIR>(f0), g1 = mul_i<DIR>(rot8<DIR>(f1));
+  v[0] = cadd(a0, b0);
+  v[4] = csub(a0, b0);
+  v[2] = add_i<DIR>(a1, b1);
+  v[6] = sub_i<DIR>(a1, b1);
+  v[1] = axpy(h, g0, e0);
+  v[5] = axpy(-h, g0, e0);
+  v[3] = axpy(h, g1, e1);
+  v[7] = axpy(-h, g1, e1);
+}
+
+// In-register R-point DFT, natural order in and out, sign DIR.  6 and 12 are
+// coprime products: the prime-factor maps (Good 1958) n = N2 n1 + N1 n2, k = k1
+// mod N1 = k2 mod N2 leave no twiddles between the factors.
+template <int R, int DIR, bool Z34 = false, typename C> __device__ __forceinline__ void dftr(C *v) {
+  static_assert(!Z34 || R == 8, "zero inputs 3 and 4 exist for 8 points");
   if constexpr (R == 1) {
     return;
-  } else if constexpr (R == 2 || R == 3 || R == 4) {
-    dft_small<R, DIR>(v);
+  } else if constexpr (R == 2) {
+    const C a = v[0], b = v[1];
+    v[0] = cadd(a, b);
+    v[1] = csub(a, b);
+  } else if constexpr (R == 3) {
+    dft3<DIR>(v[0], v[1], v[2]);
+  } else if constexpr (R == 4) {
+    dft4<DIR>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 6) {
+    // rows n2: n = 3 n1 + 2 n2 mod 6; the 3-point outputs k2 = k mod 3
+    C a[3] = {cadd(v[0], v[3]), cadd(v[2], v[5]), cadd(v[4], v[1])};
+    C b[3] = {csub(v[0], v[3]), csub(v[2], v[5]), csub(v[4], v[1])};
+    dft3<DIR>(a[0], a[1], a[2]);
+    dft3<DIR>(b[0], b[1], b[2]);
+    v[0] = a[0]; v[4] = a[1]; v[2] = a[2];
+    v[3] = b[0]; v[1] = b[1]; v[5] = b[2];
+  } else if constexpr (R == 8) {
+    dft8<DIR, Z34>(v);
+  } else if constexpr (R == 12) {
+    // n = 3 n1 + 4 n2 mod 12, n1 < 4, n2 < 3
+    dft4<DIR>(v[0], v[3], v[6], v[9]);
+    dft4<DIR>(v[4], v[7], v[10], v[1]);
+    dft4<DIR>(v[8], v[11], v[2], v[5]);
+    dft3<DIR>(v[0], v[4], v[8]);   // k1 = 0: k = 0, 4, 8 for k2 = 0, 1, 2
+    dft3<DIR>(v[3], v[7], v[11]);  // k1 = 1: k = 9, 1, 5
+    dft3<DIR>(v[6], v[10], v[2]);  // k1 = 2: k = 6, 10, 2
+    dft3<DIR>(v[9], v[1], v[5]);   // k1 = 3: k = 3, 7, 11
+    const C t9 = v[3], t1 = v[7], t5 = v[11], t3 = v[9], t7 = v[1], t11 = v[5];
+    v[9] = t9; v[1] = t1; v[5] = t5;
+    v[3] = t3; v[7] = t7; v[11] = t11;
   } else {
-    constexpr int A = F1<R>::A, B = R / A;
-    using T = decltype(v[0].x);
+    static_assert(R == 9 || R == 16, "register DFT size");
+    constexpr int A = R == 9 ? 3 : 4, B = R / A;
     C y[R];
 #pragma unroll
     for (int j2 = 0; j2 < B; j2++) {
@@ -79,17 +204,7 @@ template <int R, int DIR, typename C> __device__ __forceinline__ void dftr(C *v)
       for (int j1 = 0; j1 < A; j1++) t[j1] = v[j2 + B * j1];
       dftr<A, DIR>(t);
 #pragma unroll
-      for (int k1 = 0; k1 < A; k1++) {
-        const int e = j2 * k1;  // < R
-        if (e == 0) {
-          y[j2 + B * k1] = t[k1];
-        } else {
-          C w;
-          w.x = (T)twc_re<R>(e);
-          w.y = (T)(DIR < 0 ? twc_im<R>(e) : -twc_im<R>(e));
-          y[j2 + B * k1] = cmul(t[k1], w);
-        }
-      }
+      for (int k1 = 0; k1 < A; k1++) y[j2 + B * k1] = twmul<R, DIR>(t[k1], j2 * k1);
     }
 #pragma unroll
     for (int k1 = 0; k1 < A; k1++) {
@@ -104,7 +219,7 @@ template <int R, int DIR, typename C> __device__ __forceinline__ void dftr(C *v)
 }
 
 // Line addressing for the two-pass FFTs.  base(l) is the offset of line l,
-// ES the element stride (compile time).
+// ES the element stride (0: given at run time, es_rt).
 struct Lines1 {  // lines at l*ls
   int ls;
   __device__ __forceinline__ int base(int l) const { return l * ls; }
@@ -172,7 +287,8 @@ template <int R1> __device__ __forceinline__ constexpr bool band34(bool p34, int
 // natural -> permuted.  twN: exp(-2 pi i t/N) (shared-memory table or accessor).
 template <int N, int ES, int DIR, bool P34 = false, typename C, typename LM, typename TW, typename MK = AllElems>
 __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN, int tid, int nthr,
-                                    const MK &mask = MK{}) {
+                                    const MK &mask = MK{}, int es_rt = ES) {
+  const int es = ES ? ES : es_rt;
   constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
   static_assert(!P34 || R1 == 8, "the j1 = 3, 4 band needs R1 = 8");
   if (nl > 0) {
@@ -186,15 +302,15 @@ __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN,
 #pragma unroll
       for (int j1 = 0; j1 < R1; j1++) {
         const int k = j2 + R2 * j1;
-        v[j1] = (!band34<R1>(P34, j1) && in(k)) ? p[k * ES] : cmk<C>(0.0, 0.0);
+        v[j1] = (!band34<R1>(P34, j1) && in(k)) ? p[k * es] : cmk<C>(0.0, 0.0);
       }
-      dftr<R1, DIR>(v);
-      p[j2 * ES] = v[0];
+      dftr<R1, DIR, P34>(v);
+      p[j2 * es] = v[0];
 #pragma unroll
       for (int k1 = 1; k1 < R1; k1++) {
         C w = tw_at<C>(twN, j2 * k1);
         if (DIR > 0) w.y = -w.y;
-        p[(j2 + R2 * k1) * ES] = cmul(v[k1], w);
+        p[(j2 + R2 * k1) * es] = cmul(v[k1], w);
       }
     }
   }
@@ -204,13 +320,13 @@ __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN,
     for (UnitIter it(tid, nthr, nl); it.j < R1; it.next()) {
       const int l = it.l, k1 = it.j;
       if (!lm.valid(l)) continue;
-      C *p = buf + lm.base(l) + R2 * k1 * ES;
+      C *p = buf + lm.base(l) + R2 * k1 * es;
       C v[R2];
 #pragma unroll
-      for (int j = 0; j < R2; j++) v[j] = p[j * ES];
+      for (int j = 0; j < R2; j++) v[j] = p[j * es];
       dftr<R2, DIR>(v);
 #pragma unroll
-      for (int j = 0; j < R2; j++) p[j * ES] = v[j];
+      for (int j = 0; j < R2; j++) p[j * es] = v[j];
     }
   }
   __syncthreads();
@@ -219,7 +335,8 @@ __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN,
 // permuted -> natural
 template <int N, int ES, int DIR, bool P34 = false, typename C, typename LM, typename TW, typename MK = AllElems>
 __device__ __forceinline__ void dit(C *buf, const LM &lm, int nl, const TW &twN, int tid, int nthr,
-                                    const MK &mask = MK{}) {
+                                    const MK &mask = MK{}, int es_rt = ES) {
+  const int es = ES ? ES : es_rt;
   constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
   static_assert(!P34 || R1 == 8, "the j1 = 3, 4 band needs R1 = 8");
   if (nl > 0) {
@@ -227,17 +344,17 @@ __device__ __forceinline__ void dit(C *buf, const LM &lm, int nl, const TW &twN,
     for (UnitIter it(tid, nthr, nl); it.j < R1; it.next()) {
       const int l = it.l, k1 = it.j;
       if (!lm.valid(l)) continue;
-      C *p = buf + lm.base(l) + R2 * k1 * ES;
+      C *p = buf + lm.base(l) + R2 * k1 * es;
       C v[R2];
 #pragma unroll
-      for (int j = 0; j < R2; j++) v[j] = p[j * ES];
+      for (int j = 0; j < R2; j++) v[j] = p[j * es];
       dftr<R2, DIR>(v);
       p[0] = v[0];
 #pragma unroll
       for (int j2 = 1; j2 < R2; j2++) {
         C w = tw_at<C>(twN, j2 * k1);
         if (DIR > 0) w.y = -w.y;
-        p[j2 * ES] = cmul(v[j2], w);
+        p[j2 * es] = cmul(v[j2], w);
       }
     }
   }
@@ -250,13 +367,13 @@ __device__ __forceinline__ void dit(C *buf, const LM &lm, int nl, const TW &twN,
       C *p = buf + lm.base(l);
       C v[R1];
 #pragma unroll
-      for (int k1 = 0; k1 < R1; k1++) v[k1] = p[(R2 * k1 + j2) * ES];
+      for (int k1 = 0; k1 < R1; k1++) v[k1] = p[(R2 * k1 + j2) * es];
       dftr<R1, DIR>(v);
       const auto out = mask.line(l);
 #pragma unroll
       for (int j1 = 0; j1 < R1; j1++) {
         const int k = j2 + R2 * j1;
-        if (!band34<R1>(P34, j1) && out(k)) p[k * ES] = v[j1];
+        if (!band34<R1>(P34, j1) && out(k)) p[k * es] = v[j1];
       }
     }
   }

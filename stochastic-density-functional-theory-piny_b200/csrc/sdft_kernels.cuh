@@ -11,7 +11,7 @@ constexpr int kCPB = 8;          // column pairs per CTA (16 columns), generic p
 // column pairs per CTA of the compile-time-edge column stages: 1.1 to 1.6
 // thousand points, so that a transform pass has one or two units per thread of
 // 128 and the item phase one or two points, at every edge
-constexpr int col_cpb(int n3) { return n3 >= 72 ? 8 : (n3 >= 48 ? 16 : 32); }
+constexpr int col_cpb(int n3) { return n3 >= 72 ? 8 : (n3 >= 36 ? 16 : 32); }
 constexpr int kColThreads = 256; // threads of the column stages
 
 // Device view of the G sphere and FFT grid.
