@@ -14,7 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib", "libsdft_b200.so")
 BUILD = os.path.join(HERE, "_build")
-SOURCES = ["sdft_host.cpp", "sdft_api.cu", "sdft_kernels.cu", "sdft_kernels2.cu", "sdft_planes.cu",
+SOURCES = ["sdft_host.cpp", "sdft_api.cu", "sdft_kernels.cu", "sdft_plane_b_f32.cu", "sdft_plane_b_f64.cu",
+           "sdft_planes.cu",
            "sdft_cols_a.cu", "sdft_cols_b.cu", "sdft_cols_c.cu", "sdft_cols_d.cu", "sdft_cols_e.cu", "sdft_kb.cu", "sdft_gemm_oz.cu",
            "sdft_noalloc.cu", "sdft_noise.cu", "sdft_lanczos.cu",
            "sdft_mixer.cu", "sdft_xc.cu", "sdft_vks.cu"]

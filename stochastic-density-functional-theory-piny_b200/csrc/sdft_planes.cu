@@ -4,8 +4,9 @@
 //
 // A kernel per pair of edges would need 15 x 15 instances; switching inside
 // the kernel costs two uniform branches per transform and the registers of
-// the largest radix.  64 x 64 planes, 48 pairs, FP32: the Stockham kernel with
-// run-time radices took 415 us per launch.
+// the largest radix.  64 x 64 planes, 49 pairs, FP32, per launch: 58 us (an
+// instance of their own 46.8, so the common pairs have one; the Stockham kernel
+// with run-time radices 415).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "sdft_kernels2.cuh"
@@ -191,6 +192,11 @@ __global__ void kf_vks_perm(const double *__restrict__ v, T *__restrict__ Vp, in
 // dispatch
 // ---------------------------------------------------------------------------
 bool fast_supported(int n1, int n2, int n3) { return plan_rt(n1).r1 && plan_rt(n2).r1 && plan_rt(n3).r1; }
+
+bool plane_size_settable(int n1, int n2, int n3) {
+  auto small = [](int n) { return n == 24 || n == 48 || n == 72; };
+  return (small(n3) || n3 == 96) && ((small(n1) && small(n2)) || (n1 == 96 && n2 == 96));
+}
 
 template <typename T>
 void fast_stage_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {

@@ -1,5 +1,5 @@
 // sdft_planes.cuh -- pieces shared by the plane kernels (compile-time edge
-// pairs in sdft_kernels2.cu, run-time pairs in sdft_planes.cu).
+// pairs in sdft_plane_b.cuh, run-time pairs in sdft_planes.cu).
 #pragma once
 #include "sdft_fft2.cuh"
 #include "sdft_kernels.cuh"
