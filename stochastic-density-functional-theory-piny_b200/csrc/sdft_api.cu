@@ -367,24 +367,21 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
 static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true) {
   if (ctx->P == 0) return SDFT_OK;
   if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back);
-  const int spad = (int)rup(nstate, 64);
   const int K1 = 2 * ctx->ngp;
-  // split K of the projection so that >= ~2 waves of CTAs exist
-  const int tiles = (ctx->Ppad / 128) * (spad / 64);
-  int split = 1;
-  while (tiles * split < 2 * 148 && split < 64 && (K1 / 16) / (split * 2) >= 8 &&
-         (size_t)(split * 2) * spad * ctx->Ppad <= ctx->zwork_elems)
-    split *= 2;
-  if (ctx->gemm_split > 0) {  // tuned override, within the workspace and K
-    split = std::min(ctx->gemm_split, std::max(1, K1 / 16));
-    while (split > 1 && (size_t)split * spad * ctx->Ppad > ctx->zwork_elems) split--;
+  // K of the back projection: the projector rows up to a multiple of 16 (the
+  // padding columns of Bk and Z are zero)
+  const int K2 = (int)rup(ctx->P, 16);
+  if (ctx->plan_n != nstate || ctx->plan_split != ctx->gemm_split) {
+    ctx->plan1 = plan_gemm_nt_f64(ctx->Ppad, K1, ctx->P, nstate, ctx->gemm_split, ctx->zwork_elems);
+    ctx->plan2 = plan_gemm_nt_f64(K1, K2, K1, nstate, 0, 0);
+    ctx->plan_n = nstate;
+    ctx->plan_split = ctx->gemm_split;
   }
   {
     TScope ts(ctx, 3);
-    launch_gemm_nt_f64(ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, ctx->Ppad, spad, K1, ctx->P, nstate,
-                       split, ctx->d_zwork, ctx->st);
+    ctx->launches += launch_gemm_nt_f64(ctx->plan1, ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, K1, ctx->P, nstate,
+                                        ctx->d_zwork, ctx->st);
   }
-  ctx->launches += split > 1 ? 2 : 1;
   if (want_enl) {
     launch_enl(ctx->d_z, ctx->Ppad, ctx->d_w, ctx->P, nstate, ctx->d_enl, ctx->st);
     ctx->launches += 2;
@@ -392,10 +389,9 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
   if (!back) return SDFT_OK;
   {
     TScope ts(ctx, 4);
-    launch_gemm_nt_f64(ctx->d_bk, ctx->Ppad, ctx->d_z, ctx->Ppad, ctx->d_fnl, K1, ctx->Mpad2, spad,
-                       ctx->Ppad, K1, nstate, 1, nullptr, ctx->st);
+    ctx->launches += launch_gemm_nt_f64(ctx->plan2, ctx->d_bk, ctx->Ppad, ctx->d_z, ctx->Ppad, ctx->d_fnl, K1, K2, K1,
+                                        nstate, nullptr, ctx->st);
   }
-  ctx->launches++;
   return SDFT_OK;
 }
 
@@ -708,7 +704,12 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   g.plane_nt = default_plane_threads(ctx);
   g.ncoef = ncoef; g.ngp = ctx->ngp;
   g.ncols = ctx->cols.ncols; g.ncols_pad = ctx->cols.ncols_pad; g.ncp = ctx->cols.ncp; g.kamax = ctx->cols.kamax;
-  const int cpb = ctx->fast ? col_cpb(n3) : kCPB;
+  // fewer columns per CTA where the context's orbitals make fewer than two
+  // CTAs per SM of the default size: 8 atoms, 16 orbitals, FP64, 24 CTAs of 32
+  // column pairs took 7.6 us per stage C, 88 of 8 pairs 3.9
+  int cpb = ctx->fast ? col_cpb(n3) : kCPB;
+  if (ctx->fast && (long long)ctx->npairs_max * ((g.ncp + cpb - 1) / cpb) < 2 * 148) cpb = kCPBSmall;
+  g.cpb = cpb;
   g.nbatch = (g.ncp + cpb - 1) / cpb;
   g.cp_gstart = ctx->d_cp_gstart; g.cp_gcount = ctx->d_cp_gcount; g.col_ab = ctx->d_col_ab;
   g.gkc = ctx->d_gkc; g.ak2 = ctx->d_ak2;

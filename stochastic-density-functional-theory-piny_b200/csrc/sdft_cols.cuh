@@ -39,8 +39,8 @@ namespace sdft {
 // 65.7 us at N3 = 24 with moment dots (19.3 now).  Bound: 2.98 GB at 96^3,
 // 0.65 of the copy bandwidth.
 // FP64: 128 x 5 46.5 us at 72^3 and 32 pairs, 256 x 3 53.3, 192 x 4 49.0.
-template <typename T, int N3> struct ColCfg {
-  static constexpr int CPB = col_cpb(N3), NL = 2 * CPB;
+template <typename T, int N3, int CPB> struct ColCfg {
+  static constexpr int NL = 2 * CPB;
   static constexpr int NT = 128;
   static constexpr int MINB = sizeof(T) == 4 ? 8 : 5;
   static constexpr int P3 = N3 | 1;
@@ -56,9 +56,9 @@ template <int N> __device__ __forceinline__ bool in_kc(int2 r, int k) {
 
 // Forward c-transform of the CTA's lines, natural -> permuted rows stored to
 // the column scratch (phases 4 and 5).
-template <typename T, int N3, typename C2 = typename CT<T>::type>
+template <typename T, int N3, int CPB, typename C2 = typename CT<T>::type>
 __device__ __forceinline__ void col_forward(C2 *buf, const int2 *rng, int ncl, C2 *Xo, int pitch, int tid) {
-  using G = ColCfg<T, N3>;
+  using G = ColCfg<T, N3, CPB>;
   constexpr int R1 = Plan<N3>::R1, R2 = Plan<N3>::R2, NL = G::NL, NT = G::NT, P3 = G::P3;
   const TwC<N3, C2> tw{};
 #pragma unroll 1
@@ -104,11 +104,11 @@ struct ColItem {
       : gi(m.x), kd(m.y & 0xff), km((m.y >> 8) & 0xff), lc((m.y >> 16) & 0xff), lm((m.y >> 24) & 0x7f), g0(m.y < 0) {}
 };
 
-template <typename T, int N3>
-__global__ void __launch_bounds__(ColCfg<T, N3>::NT)
+template <typename T, int N3, int CPB>
+__global__ void __launch_bounds__(ColCfg<T, N3, CPB>::NT)
 kf_stage_a(DevGeom g, const double *__restrict__ C, int nstate, int pair0, typename CT<T>::type *__restrict__ X) {
   using C2 = typename CT<T>::type;
-  using G = ColCfg<T, N3>;
+  using G = ColCfg<T, N3, CPB>;
   constexpr int P3 = G::P3, NL = G::NL, NT = G::NT;
   __shared__ __align__(16) C2 buf[NL * P3];
   __shared__ int2 rng[NL];
@@ -132,7 +132,7 @@ kf_stage_a(DevGeom g, const double *__restrict__ C, int nstate, int pair0, typen
     buf[m.lc * P3 + m.kd] = cmk<C2>(a - d, b + c);
   }
   __syncthreads();
-  col_forward<T, N3>(buf, rng, ncl, X + (size_t)blockIdx.y * N3 * g.ncols_pad + col0, g.ncols_pad, tid);
+  col_forward<T, N3, CPB>(buf, rng, ncl, X + (size_t)blockIdx.y * N3 * g.ncols_pad + col0, g.ncols_pad, tid);
 }
 
 // Epilogue of both orbitals of a pair at G index gi: every load of both
@@ -257,11 +257,11 @@ __device__ __forceinline__ void epilogue_pair(const DevGeom &g, const EpiArgs &e
 
 // X is not __restrict__: with e.Xnext the CTA overwrites its own columns of
 // the same scratch (read into shared memory in phase 1) for the next step.
-template <typename T, int N3, int KIND>
-__global__ void __launch_bounds__(ColCfg<T, N3>::NT, ColCfg<T, N3>::MINB)
+template <typename T, int N3, int CPB, int KIND>
+__global__ void __launch_bounds__(ColCfg<T, N3, CPB>::NT, ColCfg<T, N3, CPB>::MINB)
 kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
   using C2 = typename CT<T>::type;
-  using G = ColCfg<T, N3>;
+  using G = ColCfg<T, N3, CPB>;
   constexpr int R1 = Plan<N3>::R1, R2 = Plan<N3>::R2, P3 = G::P3, NL = G::NL, NT = G::NT, NW = NT / 32;
   __shared__ __align__(16) C2 buf[NL * P3];
   __shared__ int2 rng[NL];
@@ -360,23 +360,39 @@ kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
     for (int w = 0; w < NW; w++) a += red[w][tid];
     e.dots[((size_t)(s1 >> 1) * g.nbatch + blockIdx.x) * 3 + tid] = a;
   }
-  if (e.Xnext) col_forward<T, N3>(buf, rng, ncl, reinterpret_cast<C2 *>(e.Xnext) + xoff, g.ncols_pad, tid);
+  if (e.Xnext) col_forward<T, N3, CPB>(buf, rng, ncl, reinterpret_cast<C2 *>(e.Xnext) + xoff, g.ncols_pad, tid);
 }
 
-template <typename T, int N3>
-void cols_launch_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
-  kf_stage_a<T, N3><<<dim3(g.nbatch, npairs), ColCfg<T, N3>::NT, 0, st>>>(g, C, nstate, pair0,
-                                                                         (typename CT<T>::type *)X);
+template <typename T, int N3, int CPB>
+void cols_launch_a_n(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
+  kf_stage_a<T, N3, CPB><<<dim3(g.nbatch, npairs), ColCfg<T, N3, CPB>::NT, 0, st>>>(g, C, nstate, pair0,
+                                                                                   (typename CT<T>::type *)X);
 }
 
-template <typename T, int N3>
-void cols_launch_c(const DevGeom &g, const void *X, const EpiArgs &e, int npairs, cudaStream_t st) {
+template <typename T, int N3, int CPB>
+void cols_launch_c_n(const DevGeom &g, const void *X, const EpiArgs &e, int npairs, cudaStream_t st) {
   using C2 = typename CT<T>::type;
   const dim3 grid(g.nbatch, npairs);
-  constexpr int NT = ColCfg<T, N3>::NT;
-  if (e.mode == EPI_HPSI || e.mode == EPI_NOISE) kf_stage_c<T, N3, COL_RAW><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
-  else if (e.dots) kf_stage_c<T, N3, COL_DOTS><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
-  else kf_stage_c<T, N3, COL_STEP><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
+  constexpr int NT = ColCfg<T, N3, CPB>::NT;
+  if (e.mode == EPI_HPSI || e.mode == EPI_NOISE) kf_stage_c<T, N3, CPB, COL_RAW><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
+  else if (e.dots) kf_stage_c<T, N3, CPB, COL_DOTS><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
+  else kf_stage_c<T, N3, CPB, COL_STEP><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
+}
+
+// the CPB instance that the context's item table was made for
+template <typename T, int N3>
+void cols_launch_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
+  constexpr int CPB = col_cpb(N3);
+  if constexpr (CPB > kCPBSmall)
+    if (g.cpb == kCPBSmall) return cols_launch_a_n<T, N3, kCPBSmall>(g, C, nstate, pair0, npairs, X, st);
+  cols_launch_a_n<T, N3, CPB>(g, C, nstate, pair0, npairs, X, st);
+}
+template <typename T, int N3>
+void cols_launch_c(const DevGeom &g, const void *X, const EpiArgs &e, int npairs, cudaStream_t st) {
+  constexpr int CPB = col_cpb(N3);
+  if constexpr (CPB > kCPBSmall)
+    if (g.cpb == kCPBSmall) return cols_launch_c_n<T, N3, kCPBSmall>(g, X, e, npairs, st);
+  cols_launch_c_n<T, N3, CPB>(g, X, e, npairs, st);
 }
 
 }  // namespace sdft

@@ -40,6 +40,8 @@ struct sdft_ctx {
   double *d_zsave = nullptr;
   unsigned long long *d_rowmax3 = nullptr;  // row maxima of i G_d c, d = x, y, z (3 s_pad words)
   size_t zwork_elems = 0;
+  sdft::GemmPlan plan1, plan2;        // FP64 projection / back projection for plan_n orbitals and
+  int plan_n = 0, plan_split = 0;     // the gemm_split they were made with (0 orbitals: none)
   // orbital blocks
   double *d_chi = nullptr, *d_b1 = nullptr, *d_b2 = nullptr, *d_fnl = nullptr;
   double *d_acc = nullptr;

@@ -463,6 +463,7 @@ __global__ void k_reduce_slice(const double *__restrict__ part, int split, size_
   for (int m = threadIdx.x; m < ldo; m += blockDim.x) {
     double s = 0.0;
     if (m < Mst)
+#pragma unroll 8
       for (int z = 0; z < split; z++) s += part[z * stride + (size_t)n * ldo + m];
     out[(size_t)n * ldo + m] = s;
     mx = fmax(mx, absmax_key(s));

@@ -175,10 +175,19 @@ static void kb_release(sdft_ctx *ctx) {
   ctx->d_rowmax3 = nullptr;
   ctx->kb_natm = 0;
   ctx->P = 0;
+  ctx->plan_n = 0;
   ctx->oz = false;
   ctx->dev_bytes -= ctx->kb_bytes;
   ctx->kb_bytes = 0;
 }
+
+// Below kOzMinWork the mixed contexts keep the FP64 matrices and the DMMA
+// GEMM too: the digit path's four kernels (digits, GEMM, reduction + digits,
+// GEMM) are then mostly latency.  Time per filter step, digits / DMMA: 8 atoms
+// x 16 orbitals (P K S = 8.5e5) 40.5 / 25.6 us; 16 x 256 (5.5e7) 99.7 / 82.1;
+// 32 x 96 (8.1e7) 70.2 / 59.6; 64 x 32 (1.1e8) 60.8 / 60.0; 48 x 64 (1.2e8)
+// 72.9 / 75.8; 64 x 128 (4.3e8) 114.8 / 146.4.
+static constexpr double kOzMinWork = 9e7;
 
 static int kb_build(sdft_ctx *ctx, const sdft_kb_desc *kb) {
   if (!kb || kb->natm == 0) return SDFT_OK;
@@ -311,7 +320,8 @@ static int kb_build(sdft_ctx *ctx, const sdft_kb_desc *kb) {
   ctx->kb_natm = kb->natm;
   ctx->Ppad = Ppad;
   ctx->Mpad2 = Mpad2;
-  if ((ctx->prec == SDFT_PREC_MIXED || ctx->prec == SDFT_PREC_MIXED_FAST) && gemm_oz_available()) {
+  if ((ctx->prec == SDFT_PREC_MIXED || ctx->prec == SDFT_PREC_MIXED_FAST) && gemm_oz_available() &&
+      (double)P * K1 * ctx->max_states >= kOzMinWork) {
     // digit form of the projector matrices for the INT8 tensor-core GEMMs
     const int S = (ctx->max_states + 127) / 128 * 128;
     const int Kp = (K1 + 63) / 64 * 64;

@@ -16,6 +16,7 @@
 //            dots (stodft/calc-chempot-chebyshev.c:722-842).
 // The KB projection / back projection run as DMMA FP64 GEMMs.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdio>
 #include "sdft_fft.cuh"
 #include "sdft_internal.h"
@@ -389,10 +390,16 @@ k_stage_c(DevGeom g, const typename CT<T>::type *__restrict__ X, EpiArgs e) {
 
 // ============================================================================
 // DMMA FP64 NT GEMM: out[n*ldo+m] = sum_p A[m*lda+p] B[n*ldb+p]
-// Block tile 128(m) x 64(n) x 16(k), 8 warps as 4(m) x 2(n), warp tile
-// 32 x 32 = 4 x 4 mma.m8n8k4 tiles; cp.async double-buffered smem.
+// Block tile BM(m) x BN(n) x 16(k), warp tile WM x WN of mma.m8n8k4, a ring of
+// ST shared-memory stages filled by cp.async.
+//
+// The tile follows the shape.  A 128 x 64 x 16 step is 2100 cycles of an SM's
+// FP64 rate, so on small systems one such tile runs long after the other SMs
+// are idle, and few orbitals leave most of its columns empty; for a handful of
+// orbitals the projector matrix streams from memory, which wants deep rings
+// rather than wide tiles.  plan_gemm_nt_f64 picks tile and split.
 // ============================================================================
-constexpr int GBM = 128, GBN = 64, GBK = 16, GPITCH = GBK + 4;
+constexpr int GBK = 16, GPITCH = GBK + 4;
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -408,88 +415,102 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(256)
+template <int BM, int BN, int WM, int WN, int ST> struct GemmTile {
+  static constexpr int WARPS_N = BN / WN, NT = BM / WM * WARPS_N * 32;
+  static constexpr size_t SMEM = sizeof(double) * ST * (BM + BN) * GPITCH;
+};
+
+template <int BM, int BN, int WM, int WN, int ST>
+__global__ void __launch_bounds__(GemmTile<BM, BN, WM, WN, ST>::NT)
 k_gemm_nt_f64(const double *__restrict__ A, int lda, const double *__restrict__ B, int ldb,
               double *__restrict__ out, int ldo, int K, int Mst, int Nst, int kchunk,
               size_t split_stride) {
+  using G = GemmTile<BM, BN, WM, WN, ST>;
+  constexpr int NT = G::NT, FM = WM / 8, FN = WN / 8;
   extern __shared__ __align__(16) unsigned char gsm[];
-  double (*As)[GBM][GPITCH] = reinterpret_cast<double (*)[GBM][GPITCH]>(gsm);
-  double (*Bs)[GBN][GPITCH] = reinterpret_cast<double (*)[GBN][GPITCH]>(gsm + sizeof(double) * 2 * GBM * GPITCH);
+  double *As = reinterpret_cast<double *>(gsm), *Bs = As + ST * BM * GPITCH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int m0 = blockIdx.x * GBM, n0 = blockIdx.y * GBN;
+  const int wm = warp / G::WARPS_N, wn = warp % G::WARPS_N;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int kbeg = blockIdx.z * kchunk;
-  const int kend = min(K, kbeg + kchunk);
-  const int nk = (kend - kbeg) / GBK;
-  double acc[4][4][2];
+  const int nk = (min(K, kbeg + kchunk) - kbeg) / GBK;
+  double acc[FM][FN][2];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < FM; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < FN; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  auto load_tile = [&](int buf, int k0) {
-    // A: 128 rows x 8 chunks(16B); B: 64 rows x 8 chunks
+  auto load_tile = [&](int kt) {  // rows of 8 chunks of 16 B
+    const int st = kt % ST, k0 = kbeg + kt * GBK;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int c = tid + i * 256;
+    for (int c = tid; c < BM * 8; c += NT) {
       const int r = c >> 3, q = c & 7;
-      cp_async16(&As[buf][r][q * 2], A + (size_t)(m0 + r) * lda + k0 + q * 2);
+      cp_async16(As + (st * BM + r) * GPITCH + q * 2, A + (size_t)(m0 + r) * lda + k0 + q * 2);
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int c = tid + i * 256;
+    for (int c = tid; c < BN * 8; c += NT) {
       const int r = c >> 3, q = c & 7;
-      cp_async16(&Bs[buf][r][q * 2], B + (size_t)(n0 + r) * ldb + k0 + q * 2);
+      cp_async16(Bs + (st * BN + r) * GPITCH + q * 2, B + (size_t)(n0 + r) * ldb + k0 + q * 2);
     }
-    cp_async_commit();
   };
-  if (nk > 0) load_tile(0, kbeg);
+#pragma unroll
+  for (int kt = 0; kt < ST - 1; kt++) {  // (an empty group where K is shorter: the counts stay in step)
+    if (kt < nk) load_tile(kt);
+    cp_async_commit();
+  }
   for (int kt = 0; kt < nk; kt++) {
-    const int cur = kt & 1;
-    if (kt + 1 < nk) {
-      load_tile(cur ^ 1, kbeg + (kt + 1) * GBK);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+    cp_async_wait<ST - 2>();
+    __syncthreads();  // stage kt is in, and every warp is done with stage kt - 1
+    if (kt + ST - 1 < nk) load_tile(kt + ST - 1);
+    cp_async_commit();
+    const double *a = As + ((kt % ST) * BM + wm * WM + (lane >> 2)) * GPITCH + (lane & 3);
+    const double *b = Bs + ((kt % ST) * BN + wn * WN + (lane >> 2)) * GPITCH + (lane & 3);
 #pragma unroll
     for (int kk = 0; kk < GBK / 4; kk++) {
-      double af[4], bf[4];
+      double af[FM], bf[FN];
 #pragma unroll
-      for (int i = 0; i < 4; i++) af[i] = As[cur][wm * 32 + i * 8 + (lane >> 2)][kk * 4 + (lane & 3)];
+      for (int i = 0; i < FM; i++) af[i] = a[i * 8 * GPITCH + kk * 4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) bf[j] = Bs[cur][wn * 32 + j * 8 + (lane >> 2)][kk * 4 + (lane & 3)];
+      for (int j = 0; j < FN; j++) bf[j] = b[j * 8 * GPITCH + kk * 4];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < FM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        for (int j = 0; j < FN; j++) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
     }
-    __syncthreads();
   }
   double *o = out + (size_t)blockIdx.z * split_stride;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int m = m0 + wm * 32 + i * 8 + (lane >> 2);
+  for (int i = 0; i < FM; i++) {
+    const int m = m0 + wm * WM + i * 8 + (lane >> 2);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < FN; j++) {
 #pragma unroll
       for (int v = 0; v < 2; v++) {
-        const int n = n0 + wn * 32 + j * 8 + (lane & 3) * 2 + v;
+        const int n = n0 + wn * WN + j * 8 + (lane & 3) * 2 + v;
         if (m < Mst && n < Nst) o[(size_t)n * ldo + m] = acc[i][j][v];
       }
     }
   }
 }
 
-__global__ void k_split_reduce(const double *__restrict__ work, int split, size_t stride, int ldo,
-                               int Mst, int Nst, double *__restrict__ out) {
-  const size_t total = (size_t)Mst * Nst;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int n = (int)(i / Mst), m = (int)(i - (size_t)n * Mst);
-    const size_t idx = (size_t)n * ldo + m;
-    double s = 0.0;
-    for (int z = 0; z < split; z++) s += work[z * stride + idx];
+// Split partials summed per output: kRedZ threads share the splits of one output
+// (each a contiguous run, in order), then their sums are added in order.
+constexpr int kRedZ = 8;
+__global__ void __launch_bounds__(32 * kRedZ)
+k_split_reduce(const double *__restrict__ work, int split, size_t stride, int ldo, int Mst, double *__restrict__ out) {
+  const int m = blockIdx.x * 32 + threadIdx.x, z = threadIdx.y;
+  const size_t idx = (size_t)blockIdx.y * ldo + m;
+  const int z0 = split * z / kRedZ, z1 = split * (z + 1) / kRedZ;
+  __shared__ double sh[kRedZ][32];
+  double s = 0.0;
+  if (m < Mst) {
+#pragma unroll 4
+    for (int i = z0; i < z1; i++) s += work[i * stride + idx];
+  }
+  sh[z][threadIdx.x] = s;
+  __syncthreads();
+  if (z == 0 && m < Mst) {
+    for (int i = 1; i < kRedZ; i++) s += sh[i][threadIdx.x];
     out[idx] = s;
   }
 }
@@ -682,25 +703,76 @@ void launch_density_reduce(const double *rho_part, int nsplit, int N, double sca
   k_density_reduce<<<grid1d(N, 256), 256, 0, st>>>(rho_part, nsplit, N, scale, rho);
 }
 
-void launch_gemm_nt_f64(const double *A, int lda, const double *B, int ldb, double *out, int ldo, int M,
-                        int N, int K, int Mst, int Nst, int split, double *work, cudaStream_t st) {
-  if (split < 1) split = 1;
-  int kchunk = (K / GBK + split - 1) / split * GBK;
-  split = (K + kchunk - 1) / kchunk;
-  dim3 grid(M / GBM, N / GBN, split);
-  const size_t sm = sizeof(double) * 2 * (GBM + GBN) * GPITCH;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_gemm_nt_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
+// Tile shapes of the FP64 GEMM, with the share of the FP64 rate each sustains.
+// 512 atoms, 256 orbitals (projection and back projection, per launch): 64 x 64
+// as four 32 x 32 warps 3.20 ms (34 TFLOP/s; the 128 x 64 tile of eight warps it
+// replaces 3.35), 64 x 32 3.48, 128 x 32 3.33; 216 atoms, 64 orbitals: 187, 213,
+// 207, 188 us.  8 atoms, 16 orbitals: 32 x 16 2.1 us against 15.5 of 128 x 64;
+// 512 atoms, one orbital: 128 x 8 284 us (6.0 TB/s of projector) against 1650.
+struct GemmShape { int bm, bn; double eff; };
+constexpr GemmShape kGemmShapes[] = {{64, 64, 1.0}, {64, 32, 0.92}, {32, 16, 0.85},
+                                     {128, 16, 0.9}, {128, 8, 0.85}, {32, 8, 0.8}};
+
+// Microseconds of one GEMM with a tile shape and split: the longest of one
+// CTA's chain (1 us of start and end, an iteration no shorter than 0.18 us),
+// the SM's FP64 rate (62 multiply-adds a cycle at 1.9 GHz) and its share of
+// the copy bandwidth (44 GB/s), plus the reduction of split partials.
+static double gemm_cost(GemmShape t, int M, int N, int K, int split) {
+  const int it = (K / GBK + split - 1) / split;
+  const long long ctas = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * split;
+  const double per_sm = (double)((ctas + 147) / 148);
+  const double mma = (double)t.bm * t.bn * GBK / (62.0 * 1900.0 * t.eff);
+  const double mem = (double)(t.bm + t.bn) * GBK * 8.0 / 44000.0;
+  const double chain = 1.0 + it * std::max(0.18, mma);
+  double us = std::max(chain, 1.0 + per_sm * it * std::max(mma, mem));
+  if (split > 1) us += 2.0 + 16.0 * (double)split * M * N / 4e6;
+  return us;
+}
+
+template <int BM, int BN, int WM, int WN, int ST>
+static void launch_gemm_tile(const double *A, int lda, const double *B, int ldb, double *out, int ldo, int K, int Mst,
+                             int Nst, int kchunk, int split, size_t stride, cudaStream_t st) {
+  using G = GemmTile<BM, BN, WM, WN, ST>;
+  auto k = k_gemm_nt_f64<BM, BN, WM, WN, ST>;
+  static const bool attr_once = (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM), true);
+  (void)attr_once;
+  const dim3 grid((Mst + BM - 1) / BM, (Nst + BN - 1) / BN, split);
+  k<<<grid, G::NT, G::SMEM, st>>>(A, lda, B, ldb, out, ldo, K, Mst, Nst, kchunk, stride);
+}
+
+GemmPlan plan_gemm_nt_f64(int ldo, int K, int Mst, int Nst, int want_split, size_t work_elems) {
+  const size_t fit = work_elems / ((size_t)Nst * ldo);
+  const int max_split = (int)std::max<size_t>(1, std::min<size_t>(std::min(128, K / GBK), fit));
+  GemmPlan p;
+  double best_us = 1e300;
+  for (int i = 0; i < (int)(sizeof kGemmShapes / sizeof kGemmShapes[0]); i++)
+    for (int sp = 1; sp <= max_split; sp++) {
+      if (want_split > 0 && sp != std::min(want_split, max_split)) continue;
+      const double us = gemm_cost(kGemmShapes[i], Mst, Nst, K, sp);
+      if (us < best_us - 1e-9) { best_us = us; p.tile = i; p.split = sp; }
+    }
+  p.kchunk = (K / GBK + p.split - 1) / p.split * GBK;
+  p.split = (K + p.kchunk - 1) / p.kchunk;
+  return p;
+}
+
+int launch_gemm_nt_f64(const GemmPlan &p, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
+                       int K, int Mst, int Nst, double *work, cudaStream_t st) {
+  const size_t stride = (size_t)Nst * ldo;
+  double *dst = p.split > 1 ? work : out;
+#define SDFT_G(...) launch_gemm_tile<__VA_ARGS__>(A, lda, B, ldb, dst, ldo, K, Mst, Nst, p.kchunk, p.split, stride, st)
+  switch (p.tile) {
+    case 0: SDFT_G(64, 64, 32, 32, 3); break;
+    case 1: SDFT_G(64, 32, 16, 16, 4); break;
+    case 2: SDFT_G(32, 16, 16, 8, 4); break;
+    case 3: SDFT_G(128, 16, 16, 16, 4); break;
+    case 4: SDFT_G(128, 8, 16, 8, 4); break;
+    default: SDFT_G(32, 8, 8, 8, 4); break;
   }
-  if (split == 1) {
-    k_gemm_nt_f64<<<grid, 256, sm, st>>>(A, lda, B, ldb, out, ldo, K, Mst, Nst, kchunk, 0);
-  } else {
-    const size_t stride = (size_t)N * ldo;
-    k_gemm_nt_f64<<<grid, 256, sm, st>>>(A, lda, B, ldb, work, ldo, K, Mst, Nst, kchunk, stride);
-    k_split_reduce<<<grid1d((size_t)Mst * Nst, 256), 256, 0, st>>>(work, split, stride, ldo, Mst, Nst, out);
-  }
+#undef SDFT_G
+  if (p.split > 1)
+    k_split_reduce<<<dim3((Mst + 31) / 32, Nst), dim3(32, kRedZ), 0, st>>>(work, p.split, stride, ldo, Mst, out);
+  return p.split > 1 ? 2 : 1;
 }
 
 void launch_dots_reduce(const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st) {

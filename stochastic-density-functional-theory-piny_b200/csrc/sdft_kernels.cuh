@@ -12,6 +12,8 @@ constexpr int kCPB = 8;          // column pairs per CTA (16 columns), generic p
 // thousand points, so that a transform pass has one or two units per thread of
 // 128 and the item phase one or two points, at every edge
 constexpr int col_cpb(int n3) { return n3 >= 72 ? 8 : (n3 >= 36 ? 16 : 32); }
+// and of the contexts whose orbitals would not fill the SMs with such CTAs
+constexpr int kCPBSmall = 8;
 constexpr int kColThreads = 256; // threads of the column stages
 
 // Device view of the G sphere and FFT grid.
@@ -22,6 +24,7 @@ struct DevGeom {
   int ngp;              // pitch of one re (or im) block of an orbital
   int ncols, ncols_pad, ncp, kamax;
   int nbatch;           // column-stage CTAs per orbital pair: ceil(ncp / pairs per CTA)
+  int cpb;              // column pairs per column-stage CTA
   const int *item_start; // [nbatch + 1] first item of each column-stage CTA (compile-time-edge path)
   const int2 *items;    // the CTAs' sphere points (ColItem, sdft_cols.cuh)
   const int2 *kc_rng;   // [ncols] signed kc range of each column, or the whole line (kc_contig = 0)
@@ -127,13 +130,17 @@ template <typename T>
 void launch_stage_b_noise(const DevGeom &g, const unsigned char *neg, int nstate, int pair0,
                           int npairs, void *X, cudaStream_t st);
 
-// FP64 NT GEMM on DMMA: out[n*ldo + m] = sum_p A[m*lda + p] * B[n*ldb + p]
-// (beta = 0).  M, N, K must be multiples of 128, 64, 16 (padded buffers);
-// only m < Mst, n < Nst are stored.  split > 1 writes partials to
-// work[split][N][ldo] and reduces in fixed order.
-void launch_gemm_nt_f64(const double *A, int lda, const double *B, int ldb, double *out, int ldo,
-                        int M, int N, int K, int Mst, int Nst, int split, double *work,
-                        cudaStream_t st);
+// FP64 NT GEMM on DMMA: out[n*ldo + m] = sum_p A[m*lda + p] * B[n*ldb + p] for
+// m < Mst, n < Nst (beta = 0); the rows of A and B are padded to multiples of
+// 128 and 64, K is a multiple of 16.  The plan picks the tile shape and the
+// split of K for a shape (want_split > 0: that split, as far as the workspace
+// and K allow; work_elems 0: no split); split partials go to
+// work[split][Nst][ldo] and are reduced in fixed order.  The launch returns the
+// number of kernels.
+struct GemmPlan { int tile = 0, split = 1, kchunk = 0; };
+GemmPlan plan_gemm_nt_f64(int ldo, int K, int Mst, int Nst, int want_split, size_t work_elems);
+int launch_gemm_nt_f64(const GemmPlan &p, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
+                       int K, int Mst, int Nst, double *work, cudaStream_t st);
 
 // sum over nparts CTA partials (3 doubles each) -> out[0, ndots); blk: kDotBlocks*3
 // doubles of scratch (two launches, fixed order)
