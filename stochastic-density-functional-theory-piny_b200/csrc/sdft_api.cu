@@ -292,6 +292,17 @@ static int default_plane_threads(const sdft_ctx *c) {
   return (!c->fft64 && c->fast && c->n1 <= 72 && c->n2 <= 72 && c->n1 * c->n2 >= 48 * 48) ? 128 : 256;
 }
 
+// Whether the kernels of an H application on nstate orbitals start early
+// (sdft_pdl.cuh).  It hides the start of every kernel, which is what short
+// applications spend (per filter step: 64 atoms x 128 orbitals 116 -> 100 us, 8 x
+// 16 FP64 27 -> 21); at 512 atoms x 512 orbitals, 24576 planes, the waiting CTAs
+// cost 1 to 2 % instead, and in a graph of several systems they hold SMs that
+// another system's kernel could use (six uneven systems 2 % slower).
+constexpr long long kEarlyPlanes = 8192;
+static bool early_ok(const sdft_ctx *ctx, int nstate) {
+  return !ctx->in_batch && (long long)((nstate + 1) / 2) * ctx->n3 <= kEarlyPlanes;
+}
+
 // Nonlocal projection Z = Pj C and back projection FNL = Bk Z for `nstate`
 // orbitals held in `vec`, mixed precision: INT8 Ozaki GEMMs on the digit
 // form of the orbitals; Z = Pj C is split over K with FP64 partial sums, the
@@ -301,6 +312,7 @@ static int default_plane_threads(const sdft_ctx *c) {
 static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
                      const double *gk = nullptr, const unsigned long long *gk_max = nullptr) {
   const int K1 = 2 * ctx->ngp, S = ctx->s_oz, Ppad = ctx->Ppad;
+  const bool early = early_ok(ctx, nstate);
   // tile width of both GEMMs: the set one, else 64 where it pads the orbitals less
   const int bn = ctx->gemm_bn ? ctx->gemm_bn : ((nstate + 63) / 64 * 64 < (nstate + 127) / 128 * 128 ? 64 : 128);
   const int N = (nstate + bn - 1) / bn * bn;
@@ -317,11 +329,12 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
         ctx->launches++;
       }
       launch_oz_slice(vec, K1, nstate, K1, ctx->d_rowmax, ctx->d_c_dig, ctx->kp_oz, (size_t)S * ctx->kp_oz,
-                      ctx->d_c_sc, ctx->st);
+                      ctx->d_c_sc, ctx->st, OZ_7x4, early);
       ctx->launches++;
     }
   }
   OzGemm g1 = ctx->om1, g2 = ctx->om2;
+  g1.early = g2.early = early;
   g1.N = N; g1.Nst = nstate;
   g2.N = N; g2.Nst = nstate;
   g1.bn = g2.bn = bn;
@@ -344,7 +357,7 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
     // also zeroes d_rowmax[0, nstate) for the next stage C (the slice above
     // has consumed it)
     launch_oz_reduce_slice(ctx->d_oz_part, used, stride, Ppad, ctx->P, nstate, ctx->d_z, ctx->d_z_dig,
-                           (size_t)S * Ppad, ctx->d_z_sc, ctx->d_rowmax, ctx->st, ctx->om2.fmt);
+                           (size_t)S * Ppad, ctx->d_z_sc, ctx->d_rowmax, ctx->st, ctx->om2.fmt, early);
     ctx->launches += 2;
     ctx->rowmax_zero_n = nstate;
     ctx->omax_vec = nullptr;
@@ -368,6 +381,7 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
   if (ctx->P == 0) return SDFT_OK;
   if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back);
   const int K1 = 2 * ctx->ngp;
+  const bool early = early_ok(ctx, nstate);
   // K of the back projection: the projector rows up to a multiple of 16 (the
   // padding columns of Bk and Z are zero)
   const int K2 = (int)rup(ctx->P, 16);
@@ -379,7 +393,7 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
   }
   {
     TScope ts(ctx, 3);
-    ctx->launches += launch_gemm_nt_f64(ctx->plan1, ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, K1, ctx->P, nstate,
+    ctx->launches += launch_gemm_nt_f64(ctx->plan1, early, ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, K1, ctx->P, nstate,
                                         ctx->d_zwork, ctx->st);
   }
   if (want_enl) {
@@ -389,7 +403,7 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
   if (!back) return SDFT_OK;
   {
     TScope ts(ctx, 4);
-    ctx->launches += launch_gemm_nt_f64(ctx->plan2, ctx->d_bk, ctx->Ppad, ctx->d_z, ctx->Ppad, ctx->d_fnl, K1, K2, K1,
+    ctx->launches += launch_gemm_nt_f64(ctx->plan2, early, ctx->d_bk, ctx->Ppad, ctx->d_z, ctx->Ppad, ctx->d_fnl, K1, K2, K1,
                                         nstate, nullptr, ctx->st);
   }
   return SDFT_OK;
@@ -400,6 +414,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   int r = run_kb(ctx, cur, nstate, want_enl);
   if (r) return r;
   const int npairs = (nstate + 1) / 2;
+  ctx->g.early = early_ok(ctx, nstate);
   if ((r = ensure_x(ctx, npairs))) return r;
   e.nstate = nstate;
   e.pair0 = 0;
@@ -523,7 +538,7 @@ static int filter_cheby_core(sdft_ctx *ctx, int nstate, int L, int nmu, double s
     }
     if ((r = apply_h(ctx, cur, nstate, e, false))) return r;
     if (store_moments) {
-      launch_dots_reduce(ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
+      launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
                          ctx->st);
       ctx->launches += 2;
     }
@@ -586,7 +601,7 @@ static int moments_core(sdft_ctx *ctx, int nstate, int L, double scale, double e
       e.PREV = prev;
     }
     if ((r = apply_h(ctx, cur, nstate, e, false))) return r;
-    launch_dots_reduce(ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
+    launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
                        ctx->st);
     ctx->launches += 2;
     prev = cur;
@@ -1633,8 +1648,11 @@ extern "C" int sdft_batch_create(int n, sdft_ctx *const *ctxs, const int *nstate
   for (int i = 0; i < n && rc == SDFT_OK; i++) {
     sdft_ctx *c = ctxs[i];
     if ((rc = ck(cudaStreamWaitEvent(c->st, b->evs[0], 0)))) break;
-    if ((rc = filter_cheby_core(c, nstate[i], L[i], 1, scale[i], emean[i], false))) break;
-    if ((rc = density_core(c, c->d_acc, nstate[i], occ_over_nsto[i]))) break;
+    c->in_batch = n > 1;
+    rc = filter_cheby_core(c, nstate[i], L[i], 1, scale[i], emean[i], false);
+    if (!rc) rc = density_core(c, c->d_acc, nstate[i], occ_over_nsto[i]);
+    c->in_batch = false;
+    if (rc) break;
     if ((rc = ck(cudaEventRecord(b->evs[i + 1], c->st)))) break;
     if ((rc = ck(cudaStreamWaitEvent(b->st, b->evs[i + 1], 0)))) break;
   }

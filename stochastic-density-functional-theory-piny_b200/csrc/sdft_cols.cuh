@@ -23,6 +23,7 @@
 #include <type_traits>
 #include "sdft_fft2.cuh"
 #include "sdft_kernels.cuh"
+#include "sdft_pdl.cuh"
 #include "sdft_tw_edges.cuh"
 
 namespace sdft {
@@ -112,6 +113,7 @@ kf_stage_a(DevGeom g, const double *__restrict__ C, int nstate, int pair0, typen
   constexpr int P3 = G::P3, NL = G::NL, NT = G::NT;
   __shared__ __align__(16) C2 buf[NL * P3];
   __shared__ int2 rng[NL];
+  pdl_trigger();
   const int tid = threadIdx.x;
   const int col0 = NL * blockIdx.x;
   const int ncl = min(NL, g.ncols - col0);
@@ -122,6 +124,7 @@ kf_stage_a(DevGeom g, const double *__restrict__ C, int nstate, int pair0, typen
     for (int i = tid; i < ncl * P3; i += NT) buf[i] = cmk<C2>(0.0, 0.0);
     __syncthreads();
   }
+  pdl_wait();
   const double *c1 = C + (size_t)(2 * p) * 2 * g.ngp, *c2 = c1 + 2 * (size_t)g.ngp;
   const int it1 = g.item_start[blockIdx.x + 1];
   for (int it = g.item_start[blockIdx.x] + tid; it < it1; it += NT) {
@@ -266,6 +269,7 @@ kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
   __shared__ __align__(16) C2 buf[NL * P3];
   __shared__ int2 rng[NL];
   __shared__ double red[KIND == COL_DOTS ? NW : 1][3], mred[NW][2];
+  pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int col0 = NL * blockIdx.x;
   const int ncl = min(NL, g.ncols - col0);
@@ -273,6 +277,9 @@ kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
   const bool has2 = s1 + 1 < e.nstate;
   const size_t xoff = (size_t)blockIdx.y * N3 * g.ncols_pad + col0;
   const TwC<N3, C2> tw{};
+  if (e.Xnext)
+    for (int i = tid; i < ncl; i += NT) rng[i] = g.kc_rng[col0 + i];
+  pdl_wait();
   {
     const C2 *Xp = X + xoff;
 #pragma unroll 1
@@ -290,8 +297,6 @@ kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
       for (int j2 = 1; j2 < R2; j2++) p[j2] = cmul(v[j2], tw(j2 * k1));
     }
   }
-  if (e.Xnext)
-    for (int i = tid; i < ncl; i += NT) rng[i] = g.kc_rng[col0 + i];
   __syncthreads();
 #pragma unroll 1
   for (int u = tid; u < NL * R2; u += NT) {  // phase 2
@@ -365,8 +370,8 @@ kf_stage_c(DevGeom g, const typename CT<T>::type *X, EpiArgs e) {
 
 template <typename T, int N3, int CPB>
 void cols_launch_a_n(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
-  kf_stage_a<T, N3, CPB><<<dim3(g.nbatch, npairs), ColCfg<T, N3, CPB>::NT, 0, st>>>(g, C, nstate, pair0,
-                                                                                   (typename CT<T>::type *)X);
+  launch_pdl(g.early, kf_stage_a<T, N3, CPB>, dim3(g.nbatch, npairs), ColCfg<T, N3, CPB>::NT, 0, st, g, C, nstate, pair0,
+             (typename CT<T>::type *)X);
 }
 
 template <typename T, int N3, int CPB>
@@ -374,9 +379,9 @@ void cols_launch_c_n(const DevGeom &g, const void *X, const EpiArgs &e, int npai
   using C2 = typename CT<T>::type;
   const dim3 grid(g.nbatch, npairs);
   constexpr int NT = ColCfg<T, N3, CPB>::NT;
-  if (e.mode == EPI_HPSI || e.mode == EPI_NOISE) kf_stage_c<T, N3, CPB, COL_RAW><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
-  else if (e.dots) kf_stage_c<T, N3, CPB, COL_DOTS><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
-  else kf_stage_c<T, N3, CPB, COL_STEP><<<grid, NT, 0, st>>>(g, (const C2 *)X, e);
+  if (e.mode == EPI_HPSI || e.mode == EPI_NOISE) launch_pdl(g.early, kf_stage_c<T, N3, CPB, COL_RAW>, grid, NT, 0, st, g, (const C2 *)X, e);
+  else if (e.dots) launch_pdl(g.early, kf_stage_c<T, N3, CPB, COL_DOTS>, grid, NT, 0, st, g, (const C2 *)X, e);
+  else launch_pdl(g.early, kf_stage_c<T, N3, CPB, COL_STEP>, grid, NT, 0, st, g, (const C2 *)X, e);
 }
 
 // the CPB instance that the context's item table was made for

@@ -73,6 +73,7 @@ struct sdft_ctx {
   long long dev_bytes = 0;
   long long kb_bytes = 0;  // the part of dev_bytes held by the KB buffers (released by a rebuild)
   double gcut = 0.0;
+  bool in_batch = false;  // being captured into a graph with other contexts
   bool fast = false;  // compile-time-edge FFT kernels available
   bool fft64 = true;  // FFT scratch / V_KS in FP64 (plain form)
   // mixed precision KB GEMMs (Ozaki scheme on INT8 tensor cores)

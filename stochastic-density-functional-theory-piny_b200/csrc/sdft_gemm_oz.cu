@@ -29,6 +29,7 @@
 #include "sdft_internal.h"
 #include "sdft_tc_common.cuh"
 #include "sdft_gemm_oz.cuh"
+#include "sdft_pdl.cuh"
 
 namespace sdft {
 
@@ -92,6 +93,7 @@ k_gemm_oz8(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * OZ_BM;
   const int kt0 = blockIdx.z * ktiles_per_split;
   const int nkt = max(0, min(ktiles_total, kt0 + ktiles_per_split) - kt0);
+  pdl_trigger();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < OZ_STAGES; s++) {
@@ -111,17 +113,28 @@ k_gemm_oz8(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // the first stages' projector digits (A) do not depend on the kernels before
+  // this one; the orbital digits (B) do
+  const int pre = min(nkt, OZ_STAGES);
+  if (threadIdx.x == 0)
+    for (int it = 0; it < pre; it++) {
+      mbar_expect_tx(bar_full + 8 * it, S::STAGE_BYTES);
+      tma_load_3d(sbase + it * S::STAGE_BYTES, &tA, (kt0 + it) * OZ_BK, m0, 0, bar_full + 8 * it);
+    }
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {  // TMA producer
       for (int it = 0; it < nkt; it++) {
         const int s = it % OZ_STAGES;
         const uint32_t par = ((it / OZ_STAGES) & 1) ^ 1;
-        if (!mbar_wait(bar_empty + 8 * s, par, err)) break;
         const uint32_t st = sbase + s * S::STAGE_BYTES;
-        mbar_expect_tx(bar_full + 8 * s, S::STAGE_BYTES);
         const int kx = (kt0 + it) * OZ_BK;
-        tma_load_3d(st, &tA, kx, m0, 0, bar_full + 8 * s);
+        if (it >= pre) {
+          if (!mbar_wait(bar_empty + 8 * s, par, err)) break;
+          mbar_expect_tx(bar_full + 8 * s, S::STAGE_BYTES);
+          tma_load_3d(st, &tA, kx, m0, 0, bar_full + 8 * s);
+        }
         tma_load_3d(st + S::A_BYTES, &tB, kx, n0, 0, bar_full + 8 * s);
       }
     }
@@ -225,6 +238,7 @@ k_gemm_oz8p(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUte
   const uint32_t bar_tempty = bar_tfull + 8;
   uint32_t *tmem_slot = (uint32_t *)(smem + S::BAR_OFF + 8 * (2 * OZ_STAGES + 2));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_trigger();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < OZ_STAGES; s++) {
@@ -245,6 +259,14 @@ k_gemm_oz8p(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUte
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // projector digits of the first tile's first stages, as in k_gemm_oz8
+  const int pre = min(nkt, OZ_STAGES);
+  if (threadIdx.x == 0)
+    for (int it = 0; it < pre; it++) {
+      mbar_expect_tx(bar_full + 8 * it, S::STAGE_BYTES);
+      tma_load_3d(sbase + it * S::STAGE_BYTES, &tA, it * OZ_BK, (blockIdx.x / ntn) * OZ_BM, 0, bar_full + 8 * it);
+    }
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {  // TMA producer, continuous over the CTA's tiles
@@ -253,10 +275,12 @@ k_gemm_oz8p(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUte
         const int n0 = (tile % ntn) * BN, m0 = (tile / ntn) * OZ_BM;
         for (int it = 0; it < nkt; it++) {
           const int g = ti * nkt + it, s = g % OZ_STAGES;
-          if (!mbar_wait(bar_empty + 8 * s, ((g / OZ_STAGES) & 1) ^ 1, err)) { go = false; break; }
           const uint32_t st = sbase + s * S::STAGE_BYTES;
-          mbar_expect_tx(bar_full + 8 * s, S::STAGE_BYTES);
-          tma_load_3d(st, &tA, it * OZ_BK, m0, 0, bar_full + 8 * s);
+          if (g >= pre) {
+            if (!mbar_wait(bar_empty + 8 * s, ((g / OZ_STAGES) & 1) ^ 1, err)) { go = false; break; }
+            mbar_expect_tx(bar_full + 8 * s, S::STAGE_BYTES);
+            tma_load_3d(st, &tA, it * OZ_BK, m0, 0, bar_full + 8 * s);
+          }
           tma_load_3d(st + S::A_BYTES, &tB, it * OZ_BK, n0, 0, bar_full + 8 * s);
         }
       }
@@ -428,6 +452,8 @@ template <int FMT, typename SRC>
 __global__ void k_slice_rows(SRC src, int rows, int cols, const unsigned long long *__restrict__ rowmax,
                              int8_t *__restrict__ dig, int ld, size_t sstride, double *__restrict__ scale) {
   constexpr int NS = OzF<FMT>::NS;
+  pdl_trigger();
+  pdl_wait();
   const int g4 = ld >> 2;
   const size_t tot = (size_t)rows * g4;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
@@ -457,6 +483,8 @@ __global__ void k_reduce_slice(const double *__restrict__ part, int split, size_
                                double *__restrict__ out, int8_t *__restrict__ dig, size_t dig_stride,
                                double *__restrict__ scale, unsigned long long *__restrict__ zero_rowmax) {
   constexpr int NS = OzF<FMT>::NS;
+  pdl_trigger();
+  pdl_wait();
   const int n = blockIdx.x;
   if (zero_rowmax && threadIdx.x == 0) zero_rowmax[n] = 0ull;
   double mx = 0.0;
@@ -579,16 +607,16 @@ static int run_gemm_oz_t(const OzGemm &g, int split, OutT *out, size_t split_str
     (void)attr_p;
     const int ntn = g.N / BN, ntiles = ntn * (g.M / OZ_BM);
     const int grid = ntiles < 148 ? ntiles : 148;
-    k_gemm_oz8p<OutT, FMT, BN><<<grid, OZP_THREADS, S::TOTAL, st>>>(g.tA, g.tB, ktiles, ntn, ntiles, g.sa, g.sb, out, g.ldo,
-                                                               g.Mst, g.Nst, err);
+    launch_pdl(g.early, k_gemm_oz8p<OutT, FMT, BN>, dim3(grid), OZP_THREADS, S::TOTAL, st, g.tA, g.tB, ktiles, ntn, ntiles, g.sa,
+               g.sb, out, g.ldo, g.Mst, g.Nst, err);
     return SDFT_OK;
   }
   static const bool attr_once =
       (cudaFuncSetAttribute(k_gemm_oz8<OutT, FMT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL), true);
   (void)attr_once;
   dim3 grid(g.N / BN, g.M / OZ_BM, split);
-  k_gemm_oz8<OutT, FMT, BN><<<grid, OZ_THREADS, S::TOTAL, st>>>(g.tA, g.tB, ktiles, kps, g.sa, g.sb, out, split_stride,
-                                                            g.ldo, g.Mst, g.Nst, err);
+  launch_pdl(g.early, k_gemm_oz8<OutT, FMT, BN>, grid, OZ_THREADS, S::TOTAL, st, g.tA, g.tB, ktiles, kps, g.sa, g.sb, out,
+             split_stride, g.ldo, g.Mst, g.Nst, err);
   return SDFT_OK;
 }
 
@@ -621,15 +649,15 @@ static void rowmax_of(SRC src, int rows, int cols, unsigned long long *rowmax, c
 }
 
 template <typename SRC>
-static void slice_of(SRC src, int rows, int cols, const unsigned long long *rowmax, int8_t *dig, int ld,
+static void slice_of(bool early, SRC src, int rows, int cols, const unsigned long long *rowmax, int8_t *dig, int ld,
                      size_t slice_stride, double *scale, cudaStream_t st, int fmt) {
   const size_t tot = (size_t)rows * (ld / 4);
   int blocks = (int)((tot + 255) / 256);
   if (blocks > 148 * 32) blocks = 148 * 32;
   if (fmt == OZ_8x3)
-    k_slice_rows<OZ_8x3, SRC><<<blocks, 256, 0, st>>>(src, rows, cols, rowmax, dig, ld, slice_stride, scale);
+    launch_pdl(early, k_slice_rows<OZ_8x3, SRC>, dim3(blocks), 256, 0, st, src, rows, cols, rowmax, dig, ld, slice_stride, scale);
   else
-    k_slice_rows<OZ_7x4, SRC><<<blocks, 256, 0, st>>>(src, rows, cols, rowmax, dig, ld, slice_stride, scale);
+    launch_pdl(early, k_slice_rows<OZ_7x4, SRC>, dim3(blocks), 256, 0, st, src, rows, cols, rowmax, dig, ld, slice_stride, scale);
 }
 
 void launch_oz_rowmax(const double *x, int ldx, int rows, int cols, unsigned long long *rowmax, cudaStream_t st) {
@@ -676,12 +704,12 @@ void launch_oz_rowmax_igc3(const double *v, const double *gk, int ngp, int ncoef
 void launch_oz_slice_igc(const double *v, const double *gk, int ngp, int ncoef, int rows,
                          const unsigned long long *rowmax, int8_t *dig, int ld, size_t slice_stride, double *scale,
                          cudaStream_t st) {
-  slice_of(SrcIGc{v, gk, ngp, ncoef}, rows, 2 * ngp, rowmax, dig, ld, slice_stride, scale, st, OZ_7x4);
+  slice_of(false, SrcIGc{v, gk, ngp, ncoef}, rows, 2 * ngp, rowmax, dig, ld, slice_stride, scale, st, OZ_7x4);
 }
 
 void launch_oz_slice(const double *x, int ldx, int rows, int cols, const unsigned long long *rowmax, int8_t *dig,
-                     int ld, size_t slice_stride, double *scale, cudaStream_t st, int fmt) {
-  slice_of(SrcRows{x, ldx}, rows, cols, rowmax, dig, ld, slice_stride, scale, st, fmt);
+                     int ld, size_t slice_stride, double *scale, cudaStream_t st, int fmt, bool early) {
+  slice_of(early, SrcRows{x, ldx}, rows, cols, rowmax, dig, ld, slice_stride, scale, st, fmt);
 }
 
 void launch_oz_slice_rows(const double *x, int ldx, int rows, int cols, unsigned long long *rowmax, int8_t *dig,
@@ -692,13 +720,13 @@ void launch_oz_slice_rows(const double *x, int ldx, int rows, int cols, unsigned
 
 void launch_oz_reduce_slice(const double *part, int split, size_t stride, int ldo, int Mst, int Nst, double *out,
                             int8_t *dig, size_t dig_stride, double *scale, unsigned long long *zero_rowmax,
-                            cudaStream_t st, int fmt) {
+                            cudaStream_t st, int fmt, bool early) {
   if (fmt == OZ_8x3)
-    k_reduce_slice<OZ_8x3><<<Nst, 256, 0, st>>>(part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
-                                                 zero_rowmax);
+    launch_pdl(early, k_reduce_slice<OZ_8x3>, dim3(Nst), 256, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
+               zero_rowmax);
   else
-    k_reduce_slice<OZ_7x4><<<Nst, 256, 0, st>>>(part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
-                                                 zero_rowmax);
+    launch_pdl(early, k_reduce_slice<OZ_7x4>, dim3(Nst), 256, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
+               zero_rowmax);
 }
 
 // The bounded wait of the GEMM pipeline, made to run out on purpose: an

@@ -42,6 +42,7 @@ struct OzGemm {
   const double *sa, *sb;  // row scales 2^E of A (M) and B (N)
   int fmt = OZ_7x4;       // digit format of both operands
   int bn = 128;           // output columns per tile (128 or 64; tB's box height, N a multiple of it)
+  bool early = false;     // start before the kernel ahead is complete (sdft_pdl.cuh)
 };
 
 bool gemm_oz_available();
@@ -72,7 +73,7 @@ void launch_oz_rowmax(const double *x, int ldx, int rows, int cols, unsigned lon
 // digits (row pitch ld, slice pitch slice_stride bytes) + scales of rows x
 // cols doubles under the row maxima in rowmax
 void launch_oz_slice(const double *x, int ldx, int rows, int cols, const unsigned long long *rowmax, int8_t *dig,
-                     int ld, size_t slice_stride, double *scale, cudaStream_t st, int fmt = OZ_7x4);
+                     int ld, size_t slice_stride, double *scale, cudaStream_t st, int fmt = OZ_7x4, bool early = false);
 // the same two passes for the rows of i G_d c formed from c on the fly
 // (v: rows of 2 ngp, re then im; gk: G_d per coefficient; 28-bit digits of
 // 2 ngp columns), the vector whose projection is dZ/dR_d
@@ -90,6 +91,6 @@ void launch_oz_slice_rows(const double *x, int ldx, int rows, int cols, unsigned
 // dig_stride bytes).  zero_rowmax (nullable): words [0, Nst) set to 0.
 void launch_oz_reduce_slice(const double *part, int split, size_t stride, int ldo, int Mst, int Nst, double *out,
                             int8_t *dig, size_t dig_stride, double *scale, unsigned long long *zero_rowmax,
-                            cudaStream_t st, int fmt = OZ_7x4);
+                            cudaStream_t st, int fmt = OZ_7x4, bool early = false);
 
 }  // namespace sdft

@@ -21,6 +21,7 @@
 #include "sdft_fft.cuh"
 #include "sdft_internal.h"
 #include "sdft_kernels.cuh"
+#include "sdft_pdl.cuh"
 
 namespace sdft {
 
@@ -440,28 +441,40 @@ k_gemm_nt_f64(const double *__restrict__ A, int lda, const double *__restrict__ 
 #pragma unroll
     for (int j = 0; j < FN; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  auto load_tile = [&](int kt) {  // rows of 8 chunks of 16 B
+  auto load_a = [&](int kt) {  // rows of 8 chunks of 16 B
     const int st = kt % ST, k0 = kbeg + kt * GBK;
 #pragma unroll
     for (int c = tid; c < BM * 8; c += NT) {
       const int r = c >> 3, q = c & 7;
       cp_async16(As + (st * BM + r) * GPITCH + q * 2, A + (size_t)(m0 + r) * lda + k0 + q * 2);
     }
+  };
+  auto load_b = [&](int kt) {
+    const int st = kt % ST, k0 = kbeg + kt * GBK;
 #pragma unroll
     for (int c = tid; c < BN * 8; c += NT) {
       const int r = c >> 3, q = c & 7;
       cp_async16(Bs + (st * BN + r) * GPITCH + q * 2, B + (size_t)(n0 + r) * ldb + k0 + q * 2);
     }
   };
+  // the projectors (A) do not depend on the kernels before this one
+  pdl_trigger();
+#pragma unroll
+  for (int kt = 0; kt < ST - 1; kt++)
+    if (kt < nk) load_a(kt);
+  pdl_wait();
 #pragma unroll
   for (int kt = 0; kt < ST - 1; kt++) {  // (an empty group where K is shorter: the counts stay in step)
-    if (kt < nk) load_tile(kt);
+    if (kt < nk) load_b(kt);
     cp_async_commit();
   }
   for (int kt = 0; kt < nk; kt++) {
     cp_async_wait<ST - 2>();
     __syncthreads();  // stage kt is in, and every warp is done with stage kt - 1
-    if (kt + ST - 1 < nk) load_tile(kt + ST - 1);
+    if (kt + ST - 1 < nk) {
+      load_a(kt + ST - 1);
+      load_b(kt + ST - 1);
+    }
     cp_async_commit();
     const double *a = As + ((kt % ST) * BM + wm * WM + (lane >> 2)) * GPITCH + (lane & 3);
     const double *b = Bs + ((kt % ST) * BN + wn * WN + (lane >> 2)) * GPITCH + (lane & 3);
@@ -502,6 +515,8 @@ k_split_reduce(const double *__restrict__ work, int split, size_t stride, int ld
   const size_t idx = (size_t)blockIdx.y * ldo + m;
   const int z0 = split * z / kRedZ, z1 = split * (z + 1) / kRedZ;
   __shared__ double sh[kRedZ][32];
+  pdl_trigger();
+  pdl_wait();
   double s = 0.0;
   if (m < Mst) {
 #pragma unroll 4
@@ -524,6 +539,8 @@ k_split_reduce(const double *__restrict__ work, int split, size_t stride, int ld
 __global__ void __launch_bounds__(256) k_dots_reduce(const double *__restrict__ part, int nparts,
                                                      double *__restrict__ blk) {
   __shared__ double sh[256][3];
+  pdl_trigger();
+  pdl_wait();
   const int i0 = (int)((long long)nparts * blockIdx.x / kDotBlocks);
   const int i1 = (int)((long long)nparts * (blockIdx.x + 1) / kDotBlocks);
   double a[3] = {0.0, 0.0, 0.0};
@@ -541,6 +558,8 @@ __global__ void __launch_bounds__(256) k_dots_reduce(const double *__restrict__ 
 }
 
 __global__ void k_dots_sum(const double *__restrict__ blk, int ndots, double *__restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x < ndots) {
     double a = 0.0;
     for (int b = 0; b < kDotBlocks; b++) a += blk[b * 3 + threadIdx.x];
@@ -730,14 +749,14 @@ static double gemm_cost(GemmShape t, int M, int N, int K, int split) {
 }
 
 template <int BM, int BN, int WM, int WN, int ST>
-static void launch_gemm_tile(const double *A, int lda, const double *B, int ldb, double *out, int ldo, int K, int Mst,
+static void launch_gemm_tile(bool early, const double *A, int lda, const double *B, int ldb, double *out, int ldo, int K, int Mst,
                              int Nst, int kchunk, int split, size_t stride, cudaStream_t st) {
   using G = GemmTile<BM, BN, WM, WN, ST>;
   auto k = k_gemm_nt_f64<BM, BN, WM, WN, ST>;
   static const bool attr_once = (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM), true);
   (void)attr_once;
   const dim3 grid((Mst + BM - 1) / BM, (Nst + BN - 1) / BN, split);
-  k<<<grid, G::NT, G::SMEM, st>>>(A, lda, B, ldb, out, ldo, K, Mst, Nst, kchunk, stride);
+  launch_pdl(early, k, grid, G::NT, G::SMEM, st, A, lda, B, ldb, out, ldo, K, Mst, Nst, kchunk, stride);
 }
 
 GemmPlan plan_gemm_nt_f64(int ldo, int K, int Mst, int Nst, int want_split, size_t work_elems) {
@@ -753,14 +772,19 @@ GemmPlan plan_gemm_nt_f64(int ldo, int K, int Mst, int Nst, int want_split, size
     }
   p.kchunk = (K / GBK + p.split - 1) / p.split * GBK;
   p.split = (K + p.kchunk - 1) / p.kchunk;
+  // CTAs started early go to the SMs that empty first, several to an SM, and
+  // leave the others idle: 216 atoms, 64 orbitals (two CTAs an SM) lost 12 % of
+  // a filter step that way, so only CTAs of under 2 us of arithmetic start early
+  p.light = p.kchunk / GBK * (double)kGemmShapes[p.tile].bm * kGemmShapes[p.tile].bn * GBK / (62.0 * 1900.0) < 2.0;
   return p;
 }
 
-int launch_gemm_nt_f64(const GemmPlan &p, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
+int launch_gemm_nt_f64(const GemmPlan &p, bool early, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
                        int K, int Mst, int Nst, double *work, cudaStream_t st) {
   const size_t stride = (size_t)Nst * ldo;
   double *dst = p.split > 1 ? work : out;
-#define SDFT_G(...) launch_gemm_tile<__VA_ARGS__>(A, lda, B, ldb, dst, ldo, K, Mst, Nst, p.kchunk, p.split, stride, st)
+#define SDFT_G(...) \
+  launch_gemm_tile<__VA_ARGS__>(early && p.light, A, lda, B, ldb, dst, ldo, K, Mst, Nst, p.kchunk, p.split, stride, st)
   switch (p.tile) {
     case 0: SDFT_G(64, 64, 32, 32, 3); break;
     case 1: SDFT_G(64, 32, 16, 16, 4); break;
@@ -771,13 +795,14 @@ int launch_gemm_nt_f64(const GemmPlan &p, const double *A, int lda, const double
   }
 #undef SDFT_G
   if (p.split > 1)
-    k_split_reduce<<<dim3((Mst + 31) / 32, Nst), dim3(32, kRedZ), 0, st>>>(work, p.split, stride, ldo, Mst, out);
+    launch_pdl(early, k_split_reduce, dim3((Mst + 31) / 32, Nst), dim3(32, kRedZ), 0, st, (const double *)work, p.split, stride,
+               ldo, Mst, out);
   return p.split > 1 ? 2 : 1;
 }
 
-void launch_dots_reduce(const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st) {
-  k_dots_reduce<<<kDotBlocks, 256, 0, st>>>(part, nparts, blk);
-  k_dots_sum<<<1, 32, 0, st>>>(blk, ndots, out);
+void launch_dots_reduce(bool early, const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st) {
+  launch_pdl(early, k_dots_reduce, dim3(kDotBlocks), 256, 0, st, part, nparts, blk);
+  launch_pdl(early, k_dots_sum, dim3(1), 32, 0, st, (const double *)blk, ndots, out);
 }
 
 void launch_enl(const double *Z, int ldz, const double *w, int P, int nstate, double *out, cudaStream_t st) {

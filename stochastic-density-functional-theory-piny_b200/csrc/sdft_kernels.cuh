@@ -24,6 +24,7 @@ struct DevGeom {
   int ngp;              // pitch of one re (or im) block of an orbital
   int ncols, ncols_pad, ncp, kamax;
   int nbatch;           // column-stage CTAs per orbital pair: ceil(ncp / pairs per CTA)
+  bool early;           // launch the stage kernels before their predecessor is complete (sdft_pdl.cuh)
   int cpb;              // column pairs per column-stage CTA
   const int *item_start; // [nbatch + 1] first item of each column-stage CTA (compile-time-edge path)
   const int2 *items;    // the CTAs' sphere points (ColItem, sdft_cols.cuh)
@@ -137,15 +138,18 @@ void launch_stage_b_noise(const DevGeom &g, const unsigned char *neg, int nstate
 // and K allow; work_elems 0: no split); split partials go to
 // work[split][Nst][ldo] and are reduced in fixed order.  The launch returns the
 // number of kernels.
-struct GemmPlan { int tile = 0, split = 1, kchunk = 0; };
+struct GemmPlan {
+  int tile = 0, split = 1, kchunk = 0;
+  bool light = false;  // a CTA's arithmetic is short beside its latencies: an early start cannot hurt
+};
 GemmPlan plan_gemm_nt_f64(int ldo, int K, int Mst, int Nst, int want_split, size_t work_elems);
-int launch_gemm_nt_f64(const GemmPlan &p, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
+int launch_gemm_nt_f64(const GemmPlan &p, bool early, const double *A, int lda, const double *B, int ldb, double *out, int ldo,
                        int K, int Mst, int Nst, double *work, cudaStream_t st);
 
 // sum over nparts CTA partials (3 doubles each) -> out[0, ndots); blk: kDotBlocks*3
 // doubles of scratch (two launches, fixed order)
 constexpr int kDotBlocks = 128;
-void launch_dots_reduce(const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st);
+void launch_dots_reduce(bool early, const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st);
 // E_NL = sum_u w[u] sum_{s<nstate} Z[s*ldz + u]^2 -> out[0]; out[1 .. kEnlBlocks]
 // hold the partials (two launches)
 constexpr int kEnlBlocks = 128;

@@ -44,10 +44,12 @@ kf_stage_b(DevGeom g, typename CT<T>::type *__restrict__ X, const T *__restrict_
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int2 *rng = reinterpret_cast<int2 *>(smem_raw);
   C2 *pl = plane_of<C2>(smem_raw, N1);
+  pdl_trigger();
   const int tid = threadIdx.x;
   const int r = blockIdx.x;
   const int ka = g.kamax;
   plane_ranges<NT>(g, rng, pl, P2, tid);
+  pdl_wait();
   __syncthreads();
   C2 *Xrow = X + ((size_t)blockIdx.y * g.n3 + r) * g.ncols_pad;
   plane_scatter<NT>(g, Xrow, pl, P2, tid);
@@ -102,7 +104,7 @@ static void launch_plane_b(const DevGeom &g, dim3 grid, void *X, const T *Vp, cu
   auto k = kf_stage_b<T, A, B, NT, MINB, PM>;
   static const bool attr_once = (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), true);
   (void)attr_once;
-  k<<<grid, NT, sm, st>>>(g, (typename CT<T>::type *)X, Vp);
+  launch_pdl(g.early, k, grid, NT, sm, st, g, (typename CT<T>::type *)X, Vp);
 }
 
 template <typename T>

@@ -22,8 +22,10 @@ kf_stage_b_any(DevGeom g, typename CT<T>::type *__restrict__ X, const T *__restr
   const int n1 = g.n1, n2 = g.n2, P2 = plane_pitch(n2), ka = g.kamax;
   int2 *rng = reinterpret_cast<int2 *>(smem_raw);
   C2 *pl = plane_of<C2>(smem_raw, n1);
+  pdl_trigger();
   const int tid = threadIdx.x, r = blockIdx.x;
   plane_ranges<NT>(g, rng, pl, P2, tid);
+  pdl_wait();
   __syncthreads();
   C2 *Xrow = X + ((size_t)blockIdx.y * g.n3 + r) * g.ncols_pad;
   plane_scatter<NT>(g, Xrow, pl, P2, tid);
@@ -225,7 +227,7 @@ static void launch_any_b(const DevGeom &g, void *X, const T *Vp, int npairs, cud
   auto k = kf_stage_b_any<T, NT, MINB>;
   static const bool attr_once = (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), true);
   (void)attr_once;
-  k<<<dim3(g.n3, npairs), NT, plane_bytes<T>(g.n1, g.n2), st>>>(g, (typename CT<T>::type *)X, Vp);
+  launch_pdl(g.early, k, dim3(g.n3, npairs), NT, plane_bytes<T>(g.n1, g.n2), st, g, (typename CT<T>::type *)X, Vp);
 }
 
 template <> void any_stage_b<float>(const DevGeom &g, void *X, const float *Vp, int npairs, cudaStream_t st) {

@@ -3,6 +3,7 @@
 #pragma once
 #include "sdft_fft2.cuh"
 #include "sdft_kernels.cuh"
+#include "sdft_pdl.cuh"
 #include "sdft_tw_edges.cuh"
 
 namespace sdft {

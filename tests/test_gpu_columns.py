@@ -13,6 +13,9 @@ from conftest import rel_l2
 pytestmark = pytest.mark.gpu
 
 
+ECUT = {(12, 12, 12): 5.0, (24, 24, 32): 18.0}  # others 10 Ha
+
+
 def _system(wl, grid, reps, holes, ecut=10.0):
     s = wl.make_system(reps, grid, strain=(0.01, -0.015, 0.005), disp_sigma=0.05, seed=3, ecut=ecut)
     if holes:  # drop interior points of some columns (the list stays grouped by column)
@@ -45,17 +48,21 @@ def _results(pkg, s, prec, ns):
     return out
 
 
-# every edge with a compile-time plan on every axis
+# every edge with a compile-time plan on every axis, the plane pairs with stage-B
+# instances of their own, and spheres narrower and wider than 3/8 of the planes
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("grid,reps,ns,holes", [
-    ((12, 12, 12), 1, 3, False), ((24, 24, 24), 1, 1, False), ((24, 24, 24), 1, 5, True),
+    ((12, 12, 12), 1, 3, False), ((24, 24, 32), 1, 3, False), ((32, 32, 24), 1, 5, True),
+    ((64, 64, 24), (2, 2, 1), 3, False), ((96, 64, 32), (3, 2, 1), 2, False), ((32, 96, 24), (1, 3, 1), 3, False),
+    ((64, 32, 48), (2, 1, 2), 3, True), ((72, 48, 24), (3, 2, 1), 3, False), ((64, 96, 24), (2, 3, 1), 2, False),
+    ((96, 32, 24), (3, 1, 1), 3, False), ((24, 24, 24), 1, 1, False), ((24, 24, 24), 1, 5, True),
     ((48, 24, 72), (2, 1, 3), 4, False), ((72, 72, 24), (3, 3, 1), 2, False), ((24, 72, 48), (1, 3, 2), 3, True),
     ((96, 96, 96), 2, 2, False), ((16, 18, 27), 1, 3, False), ((27, 16, 18), 1, 4, True), ((18, 27, 16), 1, 2, False),
     ((32, 36, 54), (1, 1, 2), 3, False), ((54, 32, 36), (2, 1, 1), 3, True), ((36, 64, 32), (1, 2, 1), 1, False),
     ((64, 54, 81), (2, 2, 3), 2, False), ((81, 64, 108), (2, 2, 3), 3, False), ((108, 81, 64), (3, 2, 2), 2, False),
     ((64, 108, 128), (2, 3, 3), 2, False), ((128, 48, 96), (3, 2, 3), 3, False), ((96, 128, 64), (3, 3, 2), 2, True)])
 def test_compile_time_edges_match_run_time_sizes(pkg, wl, monkeypatch, prec, grid, reps, ns, holes):
-    s = _system(wl, grid, reps, holes, 5.0 if min(grid) == 12 else 10.0)
+    s = _system(wl, grid, reps, holes, ECUT.get(grid, 10.0))
     fast = _results(pkg, s, prec, ns)
     monkeypatch.setenv("SDFT_GENERIC_FFT", "1")
     slow = _results(pkg, s, prec, ns)
