@@ -422,7 +422,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   if (ctx->P && ctx->oz) e.FNLf = reinterpret_cast<const float *>(ctx->d_fnl);
   else e.FNL = ctx->P ? ctx->d_fnl : nullptr;
   e.invN = 1.0 / (double)ctx->N;
-  if (ctx->oz && ctx->track_omax && e.OUT) {  // (row maxima exist only for the digit GEMMs)
+  if (ctx->oz && ctx->track_omax && e.OUT && !e.keep_omax) {  // (row maxima exist only for the digit GEMMs)
     if (ctx->rowmax_zero_n < nstate) CK(cudaMemsetAsync(ctx->d_rowmax, 0, (size_t)nstate * 8, ctx->st));
     e.omax = ctx->d_rowmax;
   }
@@ -1356,15 +1356,19 @@ static int ensure_red(sdft_ctx *ctx) {
   return SDFT_OK;
 }
 
-// Lanczos with device-resident vectors: c in row 0 of d_chi, H c in d_b1,
-// the previous vector in d_b2; alpha_k, beta_k read back per step.
+// Lanczos with device-resident vectors: c in row 0 of d_chi, H c in d_b1, the
+// previous vector in d_b2.  Stage C writes H c itself (the Chebyshev epilogue
+// with scale 1 and shift 0) with the partials of alpha = <c|H c>; alpha and beta
+// stay on the device, so the steps follow one another without the host, and are
+// read back once.  A step after a vanishing beta divides by it: what it leaves
+// is cut off below.
 extern "C" int sdft_lanczos_bounds(sdft_ctx *ctx, int nstep, const double *v0re, const double *v0im, double margin,
                                    double *alpha, double *beta, int *nsteps, double *emin, double *emax) {
   int r = check_ready(ctx, 1);
   if (r) return r;
   if (nstep < 1 || !v0re || !v0im || !emin || !emax) return set_error(SDFT_ERR_ARG, "lanczos_bounds: bad argument");
   cudaSetDevice(ctx->device);
-  if ((r = ensure_red(ctx))) return r;
+  if ((r = ensure_red(ctx)) || (r = ensure_mom(ctx, (size_t)2 * nstep))) return r;
   const int nc = ctx->ncoef, ngp = ctx->ngp;
   double *c = ctx->d_chi, *f = ctx->d_b1, *p = ctx->d_b2;
   double *part = ctx->d_red, *sc = ctx->d_red + kRedBlocks;
@@ -1373,30 +1377,41 @@ extern "C" int sdft_lanczos_bounds(sdft_ctx *ctx, int nstep, const double *v0re,
   launch_half_dot(c, c, nc, ngp, part, sc, ctx->st);
   launch_lz_div(c, sc, nc, ngp, ctx->st);
   ctx->launches += 3;
-  std::vector<double> al, be;
-  double b = 0.0;
-  for (int k = 0; k < nstep; k++) {
-    EpiArgs e = base_epi(ctx);
-    e.mode = EPI_HPSI;
-    e.OUT = f;
-    if ((r = apply_h(ctx, c, 1, e, false))) return r;
-    launch_lz_hc(f, nc, ngp, ctx->st);
-    launch_half_dot(c, f, nc, ngp, part, sc, ctx->st);                 // alpha
-    launch_lz_w(f, c, k > 0 ? p : nullptr, sc, b, nc, ngp, ctx->st);  // w = H c - alpha c - beta p
-    launch_half_dot(f, f, nc, ngp, part, sc + 1, ctx->st);             // |w|^2
-    ctx->launches += 6;
-    double h2[2];
-    CK(cudaMemcpyAsync(h2, sc, sizeof h2, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    al.push_back(h2[0]);
-    b = std::sqrt(std::max(h2[1], 0.0));
-    be.push_back(b);
-    if (b < 1e-12) break;
-    launch_lz_next(f, c, p, b, nc, ngp, ctx->st);
-    ctx->launches++;
+  std::vector<double> h((size_t)2 * nstep);
+  double *d_al = ctx->d_mom, *d_be = ctx->d_mom + nstep;
+  {
+    OmaxScope om(ctx);
+    for (int k = 0; k < nstep; k++) {
+      EpiArgs e = base_epi(ctx);
+      e.mode = EPI_CHEB1;
+      e.OUT = f;
+      e.s1 = -0.25; e.s2 = -0.5; e.pre = 0.0;
+      e.CHI = c;
+      e.dots = ctx->d_dots;
+      e.ndots = 1;
+      e.keep_omax = true;
+      if ((r = apply_h(ctx, c, 1, e, false))) return r;
+      launch_lz_w(f, c, k > 0 ? p : nullptr, ctx->d_dots, ctx->g.nbatch, k > 0 ? d_be + k - 1 : nullptr, d_al + k, nc,
+                  ngp, part, ctx->st);
+      unsigned long long *omax = ctx->oz ? ctx->d_rowmax : nullptr;  // cleared by the projection's reduction
+      launch_lz_next(f, c, p, part, d_be + k, nc, ngp, omax, ctx->st);
+      ctx->launches += 2;
+      if (omax) {
+        ctx->omax_vec = c;
+        ctx->omax_n = 1;
+        ctx->rowmax_zero_n = 0;
+      }
+    }
   }
   CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(h.data(), ctx->d_mom, h.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
+  std::vector<double> al, be;
+  for (int i = 0; i < nstep; i++) {
+    al.push_back(h[i]);
+    be.push_back(h[nstep + i]);
+    if (be.back() < 1e-12) break;
+  }
   const int k = (int)al.size();
   for (int i = 0; i < k; i++) {
     if (alpha) alpha[i] = al[i];

@@ -79,6 +79,7 @@ struct EpiArgs {
   void *Xnext;           // column scratch to receive the packed, c-transformed OUT
                          // (stage A of the next H application; fast path), or nullptr
   bool pack_next;        // set by the loops: a next application follows this step
+  bool keep_omax;            // set by the caller: OUT is not the next vector, leave the row maxima alone
   unsigned long long *omax;  // per orbital: atomicMax of max|OUT| (bits of a
                              // non-negative double; +inf if not finite), or nullptr
 };

@@ -7,7 +7,9 @@
 // summed in block order by one thread.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include "sdft_kernels.cuh"
 #include "sdft_lanczos.h"
+#include "sdft_pdl.cuh"
 
 namespace sdft {
 
@@ -43,40 +45,71 @@ __global__ void k_sum_fixed(const double *__restrict__ part, int n, double *__re
   }
 }
 
-// H c from the raw PINY force f (-4 H c at G != 0, -2 H c at G0), in place;
-// Im H c (G0) = 0
-__global__ void k_lz_hc(double *__restrict__ f, int ncoef, int ngp) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ncoef; g += gridDim.x * blockDim.x) {
-    const bool g0 = g == ncoef - 1;
-    f[g] = (g0 ? -0.5 : -0.25) * f[g];
-    f[ngp + g] = g0 ? 0.0 : -0.25 * f[ngp + g];
+// Sum of n values spaced `stride` apart, the same in every block: per thread in
+// order, then a fixed tree (blockDim.x = kRedThreads; every thread returns it).
+__device__ __forceinline__ double block_sum_all(const double *__restrict__ v, int n, int stride) {
+  __shared__ double sh[kRedThreads];
+  double a = 0.0;
+  for (int i = threadIdx.x; i < n; i += kRedThreads) a += v[(size_t)i * stride];
+  sh[threadIdx.x] = a;
+  __syncthreads();
+  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+    __syncthreads();
   }
+  a = sh[0];
+  __syncthreads();
+  return a;
 }
 
-// w = h - alpha c - beta p (in place in h); p may be null when beta == 0
-__global__ void k_lz_w(double *__restrict__ h, const double *__restrict__ c, const double *__restrict__ p,
-                       const double *__restrict__ alpha, double beta, int ncoef, int ngp) {
-  const double a = *alpha;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ncoef; g += gridDim.x * blockDim.x) {
-    for (int part = 0; part < 2; part++) {
-      const int i = part * ngp + g;
-      double w = h[i] - a * c[i];
-      if (p) w -= beta * p[i];
-      h[i] = w;
+// w = h - alpha c - beta p in place in h (p null: no p term), alpha = sum of the
+// stage-C dot partials (first of every three); part: block partials of |w|^2
+__global__ void __launch_bounds__(kRedThreads)
+k_lz_w(double *__restrict__ h, const double *__restrict__ c, const double *__restrict__ p,
+       const double *__restrict__ dots, int nparts, const double *__restrict__ beta, double *__restrict__ alpha,
+       int ncoef, int ngp, double *__restrict__ part) {
+  pdl_trigger();
+  pdl_wait();
+  const double a = block_sum_all(dots, nparts, 3);
+  const double b = p ? *beta : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *alpha = a;
+  double s = 0.0;
+  for (int g = blockIdx.x * kRedThreads + threadIdx.x; g < ncoef; g += kRedBlocks * kRedThreads) {
+    double re = h[g] - a * c[g], im = h[ngp + g] - a * c[ngp + g];
+    if (p) {
+      re -= b * p[g];
+      im -= b * p[ngp + g];
     }
+    h[g] = re;
+    h[ngp + g] = im;
+    s += (g == ncoef - 1) ? re * re + 2.0 * im * im : 2.0 * (re * re + im * im);
   }
+  block_sum_to(s, part + blockIdx.x);
 }
 
-// p = c, c = w / beta
-__global__ void k_lz_next(const double *__restrict__ w, double *__restrict__ c, double *__restrict__ p, double beta,
-                          int ncoef, int ngp) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ncoef; g += gridDim.x * blockDim.x) {
-    for (int part = 0; part < 2; part++) {
-      const int i = part * ngp + g;
+// beta = |w| from the block partials; p = c, c = w / beta; omax (nullable):
+// atomicMax of max |c|, as stage C records it for the digit pass
+__global__ void __launch_bounds__(kRedThreads)
+k_lz_next(const double *__restrict__ w, double *__restrict__ c, double *__restrict__ p,
+          const double *__restrict__ part, double *__restrict__ beta, int ncoef, int ngp, unsigned long long *omax) {
+  pdl_trigger();
+  pdl_wait();
+  const double b = sqrt(fmax(block_sum_all(part, kRedBlocks, 1), 0.0));
+  if (blockIdx.x == 0 && threadIdx.x == 0) *beta = b;
+  double m = 0.0;
+  for (int g = blockIdx.x * kRedThreads + threadIdx.x; g < ncoef; g += kRedBlocks * kRedThreads) {
+    for (int q = 0; q < 2; q++) {
+      const int i = q * ngp + g;
+      const double x = w[i] / b;
       p[i] = c[i];
-      c[i] = w[i] / beta;
+      c[i] = x;
+      m = fmax(m, absmax_key_d(x));
     }
   }
+  if (!omax) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(omax, (unsigned long long)__double_as_longlong(m));
 }
 
 // c /= d (normalisation of the start vector)
@@ -164,17 +197,14 @@ void launch_half_dot(const double *a, const double *b, int ncoef, int ngp, doubl
   k_sum_fixed<<<1, 32, 0, st>>>(part, kRedBlocks, out);
 }
 
-void launch_lz_hc(double *f, int ncoef, int ngp, cudaStream_t st) {
-  k_lz_hc<<<grid_for(ncoef), 256, 0, st>>>(f, ncoef, ngp);
+void launch_lz_w(double *h, const double *c, const double *p, const double *dots, int nparts, const double *beta,
+                 double *alpha, int ncoef, int ngp, double *part, cudaStream_t st) {
+  launch_pdl(true, k_lz_w, dim3(kRedBlocks), dim3(kRedThreads), 0, st, h, c, p, dots, nparts, beta, alpha, ncoef, ngp, part);
 }
 
-void launch_lz_w(double *h, const double *c, const double *p, const double *alpha, double beta, int ncoef, int ngp,
-                 cudaStream_t st) {
-  k_lz_w<<<grid_for(ncoef), 256, 0, st>>>(h, c, p, alpha, beta, ncoef, ngp);
-}
-
-void launch_lz_next(const double *w, double *c, double *p, double beta, int ncoef, int ngp, cudaStream_t st) {
-  k_lz_next<<<grid_for(ncoef), 256, 0, st>>>(w, c, p, beta, ncoef, ngp);
+void launch_lz_next(const double *w, double *c, double *p, const double *part, double *beta, int ncoef, int ngp,
+                    unsigned long long *omax, cudaStream_t st) {
+  launch_pdl(true, k_lz_next, dim3(kRedBlocks), dim3(kRedThreads), 0, st, w, c, p, part, beta, ncoef, ngp, omax);
 }
 
 void launch_lz_div(double *c, const double *nrm2, int ncoef, int ngp, cudaStream_t st) {

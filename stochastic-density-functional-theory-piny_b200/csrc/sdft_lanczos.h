@@ -11,13 +11,14 @@ constexpr int kRedBlocks = 128, kRedThreads = 256;  // partials of a determinist
 // part: kRedBlocks doubles of scratch
 void launch_half_dot(const double *a, const double *b, int ncoef, int ngp, double *part, double *out,
                      cudaStream_t st);
-// raw force -> H c in place (-f/4, -f/2 and Im = 0 at G0)
-void launch_lz_hc(double *f, int ncoef, int ngp, cudaStream_t st);
-// h <- h - (*alpha) c - beta p  (p null: no p term)
-void launch_lz_w(double *h, const double *c, const double *p, const double *alpha, double beta, int ncoef, int ngp,
-                 cudaStream_t st);
-// p <- c, c <- w / beta
-void launch_lz_next(const double *w, double *c, double *p, double beta, int ncoef, int ngp, cudaStream_t st);
+// *alpha = sum of nparts dot partials (the first of every three doubles),
+// h <- w = h - (*alpha) c - (*beta) p (p null: no p term); part: kRedBlocks
+// partials of |w|^2
+void launch_lz_w(double *h, const double *c, const double *p, const double *dots, int nparts, const double *beta,
+                 double *alpha, int ncoef, int ngp, double *part, cudaStream_t st);
+// *beta = |w| from part, p <- c, c <- w / *beta; omax (nullable): atomicMax of max |c|
+void launch_lz_next(const double *w, double *c, double *p, const double *part, double *beta, int ncoef, int ngp,
+                    unsigned long long *omax, cudaStream_t st);
 // c <- c / sqrt(*nrm2)
 void launch_lz_div(double *c, const double *nrm2, int ncoef, int ngp, cudaStream_t st);
 // *out = sum over nstate rows, G != G0 of 2 ak2 (re^2 + im^2)
