@@ -308,27 +308,32 @@ static bool early_ok(const sdft_ctx *ctx, int nstate) {
 // form of the orbitals; Z = Pj C is split over K with FP64 partial sums, the
 // reduction also produces the digit form of Z for FNL = Bk Z.
 // gk (nullable): project i G_d vec instead of vec, formed inside the digit
-// pass (gk = G_d per coefficient) under the row maxima gk_max
+// pass (gk = G_d per coefficient).  max_of (nullable without gk): the row maxima
+// of what is projected.
 static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
-                     const double *gk = nullptr, const unsigned long long *gk_max = nullptr) {
+                     const double *gk = nullptr, const unsigned long long *max_of = nullptr) {
   const int K1 = 2 * ctx->ngp, S = ctx->s_oz, Ppad = ctx->Ppad;
   const bool early = early_ok(ctx, nstate);
-  // tile width of both GEMMs: the set one, else 64 where it pads the orbitals less
+  // tile width: the set one, else 64 where it pads the orbitals less; for the
+  // projection also where 128-wide tiles with the longest split (32) leave SMs
+  // idle (64 atoms, 128 orbitals: 16.4 us at 128, 13.2 at 64; the back projection
+  // 13.6 and 15.0)
   const int bn = ctx->gemm_bn ? ctx->gemm_bn : ((nstate + 63) / 64 * 64 < (nstate + 127) / 128 * 128 ? 64 : 128);
-  const int N = (nstate + bn - 1) / bn * bn;
+  const int bn1 = ctx->gemm_bn ? bn : (32 * (Ppad / 128) * ((nstate + 127) / 128) < 148 ? 64 : bn);
+  const int N = (nstate + bn1 - 1) / bn1 * bn1, N2 = (nstate + bn - 1) / bn * bn;
   {
     TScope ts(ctx, 7);
     if (gk) {
-      launch_oz_slice_igc(vec, gk, ctx->ngp, ctx->ncoef, nstate, gk_max, ctx->d_c_dig, ctx->kp_oz,
+      launch_oz_slice_igc(vec, gk, ctx->ngp, ctx->ncoef, nstate, max_of, ctx->d_c_dig, ctx->kp_oz,
                           (size_t)S * ctx->kp_oz, ctx->d_c_sc, ctx->st);
       ctx->launches++;
     } else {
       // row maxima: from the stage C that wrote `vec`, else one pass over it
-      if (!(ctx->track_omax && ctx->omax_vec == vec && ctx->omax_n == nstate)) {  // (set only when oz)
+      if (!max_of && !(ctx->track_omax && ctx->omax_vec == vec && ctx->omax_n == nstate)) {  // (set only when oz)
         launch_oz_rowmax(vec, K1, nstate, K1, ctx->d_rowmax, ctx->st);  // clears the rows first
         ctx->launches++;
       }
-      launch_oz_slice(vec, K1, nstate, K1, ctx->d_rowmax, ctx->d_c_dig, ctx->kp_oz, (size_t)S * ctx->kp_oz,
+      launch_oz_slice(vec, K1, nstate, K1, max_of ? max_of : ctx->d_rowmax, ctx->d_c_dig, ctx->kp_oz, (size_t)S * ctx->kp_oz,
                       ctx->d_c_sc, ctx->st, OZ_7x4, early);
       ctx->launches++;
     }
@@ -336,18 +341,17 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
   OzGemm g1 = ctx->om1, g2 = ctx->om2;
   g1.early = g2.early = early;
   g1.N = N; g1.Nst = nstate;
-  g2.N = N; g2.Nst = nstate;
-  g1.bn = g2.bn = bn;
-  if (bn == 64) {
-    g1.tB = ctx->om1_tb64;
-    g2.tB = ctx->om2_tb64;
-  }
+  g2.N = N2; g2.Nst = nstate;
+  g1.bn = bn1;
+  g2.bn = bn;
+  if (bn1 == 64) g1.tB = ctx->om1_tb64;
+  if (bn == 64) g2.tB = ctx->om2_tb64;
   const size_t stride = (size_t)N * Ppad;
   const int max_split = (int)std::min<size_t>(32, ctx->oz_part_elems / stride);
   const int min_split = oz_min_split(ctx->kp_oz, OZ_7x4);
   if (min_split > max_split) return set_error(SDFT_ERR_NOMEM, "oz gemm: partial buffer too small for K");
   const int split = ctx->gemm_split > 0 ? std::max(min_split, std::min(ctx->gemm_split, std::max(1, max_split)))
-                                        : oz_choose_split((Ppad / 128) * (N / bn), ctx->kp_oz / 64, max_split);
+                                        : oz_choose_split((Ppad / 128) * (N / bn1), ctx->kp_oz / 64, max_split);
   int r;
   {
     TScope ts(ctx, 3);
@@ -1352,7 +1356,7 @@ extern "C" int sdft_noise_real(sdft_ctx *ctx, int nstate, double seed, int np_st
 // ---- spectral bounds and energies --------------------------------------------
 static int ensure_red(sdft_ctx *ctx) {
   if (ctx->d_red) return SDFT_OK;
-  DM(ctx->d_red, (kRedBlocks + 8) * sizeof(double));
+  DM(ctx->d_red, (kRedPart + 8) * sizeof(double));
   return SDFT_OK;
 }
 
@@ -1371,7 +1375,7 @@ extern "C" int sdft_lanczos_bounds(sdft_ctx *ctx, int nstep, const double *v0re,
   if ((r = ensure_red(ctx)) || (r = ensure_mom(ctx, (size_t)2 * nstep))) return r;
   const int nc = ctx->ncoef, ngp = ctx->ngp;
   double *c = ctx->d_chi, *f = ctx->d_b1, *p = ctx->d_b2;
-  double *part = ctx->d_red, *sc = ctx->d_red + kRedBlocks;
+  double *part = ctx->d_red, *sc = ctx->d_red + kRedPart;
   ctx->resident = 0;
   if ((r = upload_block(ctx, c, 1, v0re, v0im))) return r;
   launch_half_dot(c, c, nc, ngp, part, sc, ctx->st);
@@ -1435,7 +1439,7 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   int r = ensure_red(ctx);
   if (r) return r;
   const double *v = ctx->d_acc + (size_t)imu * ctx->vec_elems;
-  double *sc = ctx->d_red + kRedBlocks;
+  double *sc = ctx->d_red + kRedPart;
   launch_ekin(v, nstate, ctx->ncoef, ctx->ngp, ctx->d_ak2, ctx->d_red, sc + 2, ctx->st);
   ctx->launches += 2;
   double ek = 0.0, en = 0.0;
@@ -1490,13 +1494,15 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
   do {                                  \
     if ((e = (call)) != cudaSuccess) goto out; \
   } while (0)
-  if ((r = run_kb(ctx, v, nstate, true, false))) goto out;
+  if (ctx->oz) {  // row maxima of c and of the three i G_d c in one pass over c
+    launch_oz_rowmax_igc3(v, ctx->d_gk, ctx->ngp, ctx->ncoef, nstate, ctx->d_rowmax, ctx->d_rowmax3, ctx->st);
+    ctx->launches++;
+    if ((r = run_kb_oz(ctx, v, nstate, true, false, nullptr, ctx->d_rowmax))) goto out;
+  } else if ((r = run_kb(ctx, v, nstate, true, false))) {
+    goto out;
+  }
   CKG(cudaMemcpyAsync(ctx->d_zsave, ctx->d_z, (size_t)nstate * ctx->Ppad * sizeof(double), cudaMemcpyDeviceToDevice,
                       ctx->st));
-  if (ctx->oz) {  // row maxima of the three i G_d c in one pass over c
-    launch_oz_rowmax_igc3(v, ctx->d_gk, ctx->ngp, ctx->ncoef, nstate, ctx->d_rowmax3, ctx->st);
-    ctx->launches++;
-  }
   for (int d = 0; d < 3; d++) {
     const double *gk = ctx->d_gk + (size_t)d * ctx->ngp;
     if (ctx->oz) {  // the digit pass forms i G_d c from c itself

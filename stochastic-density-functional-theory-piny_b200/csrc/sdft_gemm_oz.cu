@@ -24,6 +24,7 @@
 // All mbarrier waits are bounded (sdft_tc_common.cuh).  No TMA multicast.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <cmath>
 #include "sdft_internal.h"
@@ -385,38 +386,50 @@ __device__ __forceinline__ double absmax_key(double a) { return isfinite(a) ? fa
 // Element sources of the digit passes: a stored row, or the row of i G_d c
 // formed on the fly from c (Re = -G_d Im c, Im = G_d Re c; G = 0 and the
 // padding give 0), the vector whose projection is dZ/dR_d.
+// load4: elements c .. c+3 (c a multiple of 4) of a row.
 struct SrcRows {
   const double *x;
   int ldx;
-  __device__ __forceinline__ double operator()(int row, int c) const { return x[(size_t)row * ldx + c]; }
+  __device__ __forceinline__ void load4(int row, int c, double *v) const {
+    const double2 *q = reinterpret_cast<const double2 *>(x + (size_t)row * ldx + c);
+    const double2 a = q[0], b = q[1];
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
 };
 struct SrcIGc {
   const double *v;  // rows of 2 ngp: re[0, ngp), im[ngp, 2 ngp)
   const double *gk; // G_d per coefficient
   int ngp, ncoef;
-  __device__ __forceinline__ double operator()(int row, int c) const {
+  __device__ __forceinline__ void load4(int row, int c, double *o) const {
     const double *r = v + (size_t)row * 2 * ngp;
-    const bool im = c >= ngp;
+    const bool im = c >= ngp;  // (ngp is a multiple of 16: the four share a block)
     const int g = im ? c - ngp : c;
-    if (g >= ncoef - 1) return 0.0;
-    return im ? gk[g] * r[g] : -gk[g] * r[ngp + g];
+    const double2 *q = reinterpret_cast<const double2 *>(im ? r + g : r + ngp + g);
+    const double2 *k = reinterpret_cast<const double2 *>(gk + g);
+    const double2 a = q[0], b = q[1], ka = k[0], kb = k[1];
+    const double sg = im ? 1.0 : -1.0;
+    o[0] = g + 0 < ncoef - 1 ? sg * ka.x * a.x : 0.0;
+    o[1] = g + 1 < ncoef - 1 ? sg * ka.y * a.y : 0.0;
+    o[2] = g + 2 < ncoef - 1 ? sg * kb.x * b.x : 0.0;
+    o[3] = g + 3 < ncoef - 1 ? sg * kb.y * b.y : 0.0;
   }
 };
 
+// grid (rows, column chunks); four columns a thread and step (cols is a multiple
+// of 4, rows 16-byte aligned)
 template <typename SRC>
 __global__ void k_row_absmax(SRC src, int cols, unsigned long long *rowmax) {
   const int row = blockIdx.x;
   double m = 0.0;
-  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < cols; c += gridDim.y * blockDim.x)
-    m = fmax(m, absmax_key(src(row, c)));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmax(m, red[w]);
-    atomicMax(rowmax + row, (unsigned long long)__double_as_longlong(m));
+#pragma unroll 2
+  for (int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x); c < cols; c += 4 * gridDim.y * blockDim.x) {
+    double v[4];
+    src.load4(row, c, v);
+#pragma unroll
+    for (int e = 0; e < 4; e++) m = fmax(m, absmax_key(v[e]));
   }
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(rowmax + row, (unsigned long long)__double_as_longlong(m));
 }
 
 // Exponent E with max < 2^E (E = 0 for an all-zero row, clamped below so
@@ -446,40 +459,41 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
          ((uint32_t)(d & 0xff) << 24);
 }
 
-// digits of rows x cols doubles; 4 consecutive columns per thread, zero
-// digits for cols <= k < ld.
+// digits of rows x cols doubles (cols a multiple of 4), zero digits for
+// cols <= k < ld; grid (rows, column chunks), four consecutive columns a thread
+// and step.  Bound by memory: 8 bytes read and 4 written per value.
 template <int FMT, typename SRC>
-__global__ void k_slice_rows(SRC src, int rows, int cols, const unsigned long long *__restrict__ rowmax,
-                             int8_t *__restrict__ dig, int ld, size_t sstride, double *__restrict__ scale) {
+__global__ void __launch_bounds__(256)
+k_slice_rows(SRC src, int cols, const unsigned long long *__restrict__ rowmax,
+             int8_t *__restrict__ dig, int ld, size_t sstride, double *__restrict__ scale) {
   constexpr int NS = OzF<FMT>::NS;
+  const int row = blockIdx.x;
   pdl_trigger();
   pdl_wait();
-  const int g4 = ld >> 2;
-  const size_t tot = (size_t)rows * g4;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x) {
-    const int row = (int)(i / g4), c4 = (int)(i - (size_t)row * g4) * 4;
-    const unsigned long long mb = rowmax[row];
-    const bool bad = mb >= 0x7ff0000000000000ull;
-    const int E = bad ? 0 : row_exponent(mb);
-    const double p = ldexp(1.0, kTopShift<FMT> - E);
+  const unsigned long long mb = rowmax[row];
+  const bool bad = mb >= 0x7ff0000000000000ull;
+  const int E = bad ? 0 : row_exponent(mb);
+  const double p = ldexp(1.0, kTopShift<FMT> - E);
+  int8_t *o = dig + (size_t)row * ld;
+#pragma unroll 2
+  for (int c4 = 4 * (blockIdx.y * 256 + threadIdx.x); c4 < ld; c4 += 4 * 256 * gridDim.y) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (c4 < cols && !bad) src.load4(row, c4, v);
     int d[4][NS];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int c = c4 + e;
-      const double v = (c < cols && !bad) ? src(row, c) : 0.0;
-      digits_of<FMT>(v * p, d[e]);
-    }
+    for (int e = 0; e < 4; e++) digits_of<FMT>(v[e] * p, d[e]);
 #pragma unroll
     for (int s = 0; s < NS; s++)
-      *(uint32_t *)(dig + s * sstride + (size_t)row * ld + c4) = pack4(d[0][s], d[1][s], d[2][s], d[3][s]);
-    if (c4 == 0) scale[row] = bad ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, E);
+      *(uint32_t *)(o + s * sstride + c4) = pack4(d[0][s], d[1][s], d[2][s], d[3][s]);
   }
+  if (blockIdx.y == 0 && threadIdx.x == 0) scale[row] = bad ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, E);
 }
 
 // Sum of split-K partials for one row per CTA, then the digit form of the
 // row (second sweep over the just-written row, which is L2 resident).
 template <int FMT>
-__global__ void k_reduce_slice(const double *__restrict__ part, int split, size_t stride, int ldo, int Mst,
+__global__ void __launch_bounds__(1024)
+k_reduce_slice(const double *__restrict__ part, int split, size_t stride, int ldo, int Mst,
                                double *__restrict__ out, int8_t *__restrict__ dig, size_t dig_stride,
                                double *__restrict__ scale, unsigned long long *__restrict__ zero_rowmax) {
   constexpr int NS = OzF<FMT>::NS;
@@ -639,66 +653,65 @@ int run_gemm_oz(const OzGemm &g, int split, float *out, size_t split_stride, int
   return run_gemm_oz_any(g, split, out, split_stride, err, st, split_used);
 }
 
+// column chunks of a rows x cols pass: CTAs of at least 256 x 4 values, about
+// sixteen per SM in all
+static int pass_chunks(int rows, int cols) {
+  const int most = (cols + 1023) / 1024, want = (148 * 16 + rows - 1) / rows;
+  return std::max(1, std::min(most, want));
+}
+
 template <typename SRC>
 static void rowmax_of(SRC src, int rows, int cols, unsigned long long *rowmax, cudaStream_t st) {
   cudaMemsetAsync(rowmax, 0, (size_t)rows * sizeof(unsigned long long), st);
-  int chunks = (cols + 255) / 256;  // grid = rows x chunks (rows on x: up to 2^31 - 1)
-  if (chunks > 64) chunks = 64;
-  if (chunks < 1) chunks = 1;
-  k_row_absmax<SRC><<<dim3(rows, chunks), 256, 0, st>>>(src, cols, rowmax);
+  k_row_absmax<SRC><<<dim3(rows, pass_chunks(rows, cols)), 256, 0, st>>>(src, cols, rowmax);
 }
 
 template <typename SRC>
 static void slice_of(bool early, SRC src, int rows, int cols, const unsigned long long *rowmax, int8_t *dig, int ld,
                      size_t slice_stride, double *scale, cudaStream_t st, int fmt) {
-  const size_t tot = (size_t)rows * (ld / 4);
-  int blocks = (int)((tot + 255) / 256);
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  if (fmt == OZ_8x3)
-    launch_pdl(early, k_slice_rows<OZ_8x3, SRC>, dim3(blocks), 256, 0, st, src, rows, cols, rowmax, dig, ld, slice_stride, scale);
-  else
-    launch_pdl(early, k_slice_rows<OZ_7x4, SRC>, dim3(blocks), 256, 0, st, src, rows, cols, rowmax, dig, ld, slice_stride, scale);
+  const dim3 grid(rows, pass_chunks(rows, ld));
+  if (fmt == OZ_8x3) launch_pdl(early, k_slice_rows<OZ_8x3, SRC>, grid, 256, 0, st, src, cols, rowmax, dig, ld, slice_stride, scale);
+  else launch_pdl(early, k_slice_rows<OZ_7x4, SRC>, grid, 256, 0, st, src, cols, rowmax, dig, ld, slice_stride, scale);
 }
 
 void launch_oz_rowmax(const double *x, int ldx, int rows, int cols, unsigned long long *rowmax, cudaStream_t st) {
   rowmax_of(SrcRows{x, ldx}, rows, cols, rowmax, st);
 }
 
-// Row maxima of i G_d c for d = x, y, z in one pass over c: |Re| = |G_d| |Im c|
-// and |Im| = |G_d| |Re c|, so each coefficient contributes |G_d| max(|Re c|,
-// |Im c|) (G = 0 and the padding contribute 0).  rowmax3: 3 rows-long words.
+// Row maxima of c and of i G_d c for d = x, y, z in one pass over c: |Re| =
+// |G_d| |Im c| and |Im| = |G_d| |Re c|, so each coefficient contributes |G_d|
+// max(|Re c|, |Im c|) (G = 0 and the padding contribute 0).  rowmax: rows words,
+// rowmax3: 3 rows-long words.  Two coefficients a thread and step.
 __global__ void k_row_absmax_igc3(const double *__restrict__ v, const double *__restrict__ gk, int ngp, int ncoef,
-                                  int rows, unsigned long long *rowmax3) {
+                                  int rows, unsigned long long *rowmax, unsigned long long *rowmax3) {
   const int row = blockIdx.x;
   const double *r = v + (size_t)row * 2 * ngp;
-  double m[3] = {0.0, 0.0, 0.0};
-  for (int g = blockIdx.y * blockDim.x + threadIdx.x; g < ncoef - 1; g += gridDim.y * blockDim.x) {
-    const double a = fmax(absmax_key(r[g]), absmax_key(r[ngp + g]));
+  double m[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int g = 2 * (blockIdx.y * blockDim.x + threadIdx.x); g < ncoef; g += 2 * gridDim.y * blockDim.x) {
+    const double2 re = *reinterpret_cast<const double2 *>(r + g), im = *reinterpret_cast<const double2 *>(r + ngp + g);
+    const double a0 = fmax(absmax_key(re.x), absmax_key(im.x)), a1 = fmax(absmax_key(re.y), absmax_key(im.y));
+    m[3] = fmax(m[3], g + 1 < ncoef ? fmax(a0, a1) : a0);
 #pragma unroll
-    for (int d = 0; d < 3; d++) m[d] = fmax(m[d], absmax_key(gk[(size_t)d * ngp + g] * a));
+    for (int d = 0; d < 3; d++) {
+      const double2 k = *reinterpret_cast<const double2 *>(gk + (size_t)d * ngp + g);
+      if (g < ncoef - 1) m[d] = fmax(m[d], absmax_key(k.x * a0));
+      if (g + 1 < ncoef - 1) m[d] = fmax(m[d], absmax_key(k.y * a1));
+    }
   }
-  __shared__ double red[3][32];
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
+  for (int d = 0; d < 4; d++) {
     for (int o = 16; o > 0; o >>= 1) m[d] = fmax(m[d], __shfl_xor_sync(0xffffffffu, m[d], o));
-    if ((threadIdx.x & 31) == 0) red[d][threadIdx.x >> 5] = m[d];
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    const int d = threadIdx.x;
-    double x = red[d][0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) x = fmax(x, red[d][w]);
-    atomicMax(rowmax3 + (size_t)d * rows + row, (unsigned long long)__double_as_longlong(x));
+    if ((threadIdx.x & 31) == 0)
+      atomicMax(d < 3 ? rowmax3 + (size_t)d * rows + row : rowmax + row, (unsigned long long)__double_as_longlong(m[d]));
   }
 }
 
-void launch_oz_rowmax_igc3(const double *v, const double *gk, int ngp, int ncoef, int rows,
+void launch_oz_rowmax_igc3(const double *v, const double *gk, int ngp, int ncoef, int rows, unsigned long long *rowmax,
                            unsigned long long *rowmax3, cudaStream_t st) {
+  cudaMemsetAsync(rowmax, 0, (size_t)rows * sizeof(unsigned long long), st);
   cudaMemsetAsync(rowmax3, 0, (size_t)3 * rows * sizeof(unsigned long long), st);
-  int chunks = (ncoef + 255) / 256;
-  if (chunks > 64) chunks = 64;
-  if (chunks < 1) chunks = 1;
-  k_row_absmax_igc3<<<dim3(rows, chunks), 256, 0, st>>>(v, gk, ngp, ncoef, rows, rowmax3);
+  k_row_absmax_igc3<<<dim3(rows, pass_chunks(rows, 2 * ngp)), 256, 0, st>>>(v, gk, ngp, ncoef, rows, rowmax, rowmax3);
 }
 
 void launch_oz_slice_igc(const double *v, const double *gk, int ngp, int ncoef, int rows,
@@ -721,11 +734,12 @@ void launch_oz_slice_rows(const double *x, int ldx, int rows, int cols, unsigned
 void launch_oz_reduce_slice(const double *part, int split, size_t stride, int ldo, int Mst, int Nst, double *out,
                             int8_t *dig, size_t dig_stride, double *scale, unsigned long long *zero_rowmax,
                             cudaStream_t st, int fmt, bool early) {
+  const int nt = Nst < 148 && ldo > 512 ? 1024 : 256;  // (few rows: one CTA's walk along its row is the time)
   if (fmt == OZ_8x3)
-    launch_pdl(early, k_reduce_slice<OZ_8x3>, dim3(Nst), 256, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
+    launch_pdl(early, k_reduce_slice<OZ_8x3>, dim3(Nst), nt, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
                zero_rowmax);
   else
-    launch_pdl(early, k_reduce_slice<OZ_7x4>, dim3(Nst), 256, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
+    launch_pdl(early, k_reduce_slice<OZ_7x4>, dim3(Nst), nt, 0, st, part, split, stride, ldo, Mst, out, dig, dig_stride, scale,
                zero_rowmax);
 }
 

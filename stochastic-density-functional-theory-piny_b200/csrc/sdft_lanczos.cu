@@ -121,24 +121,32 @@ __global__ void k_lz_div(double *__restrict__ c, const double *__restrict__ nrm2
   }
 }
 
-// sum over nstate rows and G != G0 of 2 ak2(G) (re^2 + im^2); block b takes
-// the rows [nstate b / kRedBlocks, nstate (b+1) / kRedBlocks), threads the G
-// vectors of each row (a fixed order, no index division)
+// sum over nstate rows and G != G0 of 2 ak2(G) (re^2 + im^2); blocks
+// (row group, chunk of G): a thread's G stay the same over the group's rows, so
+// ak2 is read once per thread and the rows stream (a fixed order)
 __global__ void __launch_bounds__(kRedThreads) k_ekin_part(const double *__restrict__ v, int nstate, int ncoef,
                                                            int ngp, const double *__restrict__ ak2,
                                                            double *__restrict__ part) {
   double s = 0.0;
-  const int ng = ncoef - 1;
-  const int r0 = (int)((long long)nstate * blockIdx.x / kRedBlocks);
-  const int r1 = (int)((long long)nstate * (blockIdx.x + 1) / kRedBlocks);
-  for (int st = r0; st < r1; st++) {
-    const double *row = v + (size_t)st * 2 * ngp;
-    for (int g = threadIdx.x; g < ng; g += kRedThreads) {
-      const double re = row[g], im = row[ngp + g];
-      s += 2.0 * ak2[g] * (re * re + im * im);
+  const int r0 = (int)((long long)nstate * blockIdx.y / kEkRows);
+  const int r1 = (int)((long long)nstate * (blockIdx.y + 1) / kEkRows);
+  for (int g = 2 * (blockIdx.x * kRedThreads + threadIdx.x); g < ncoef - 1; g += 2 * kEkChunks * kRedThreads) {
+    const double k0 = 2.0 * ak2[g], k1 = g + 1 < ncoef - 1 ? 2.0 * ak2[g + 1] : 0.0;
+    const double *row = v + (size_t)r0 * 2 * ngp + g;  // (16-byte aligned: ngp is a multiple of 16)
+#pragma unroll 4
+    for (int st = r0; st < r1; st++, row += 2 * (size_t)ngp) {
+      const double2 re = *reinterpret_cast<const double2 *>(row), im = *reinterpret_cast<const double2 *>(row + ngp);
+      const double e0 = k0 * (re.x * re.x + im.x * im.x);
+      s += k1 == 0.0 ? e0 : e0 + k1 * (re.y * re.y + im.y * im.y);
     }
   }
-  block_sum_to(s, part + blockIdx.x);
+  block_sum_to(s, part + blockIdx.y * kEkChunks + blockIdx.x);
+}
+
+__global__ void __launch_bounds__(kRedThreads) k_sum_tree(const double *__restrict__ part, int n,
+                                                          double *__restrict__ out) {
+  const double a = block_sum_all(part, n, 1);
+  if (threadIdx.x == 0) *out = a;
 }
 
 // i G_d c: the orbital whose KB projection is dZ/dR_d (get_nlmat,
@@ -213,8 +221,8 @@ void launch_lz_div(double *c, const double *nrm2, int ncoef, int ngp, cudaStream
 
 void launch_ekin(const double *v, int nstate, int ncoef, int ngp, const double *ak2, double *part, double *out,
                  cudaStream_t st) {
-  k_ekin_part<<<kRedBlocks, kRedThreads, 0, st>>>(v, nstate, ncoef, ngp, ak2, part);
-  k_sum_fixed<<<1, 32, 0, st>>>(part, kRedBlocks, out);
+  k_ekin_part<<<dim3(kEkChunks, kEkRows), kRedThreads, 0, st>>>(v, nstate, ncoef, ngp, ak2, part);
+  k_sum_tree<<<1, kRedThreads, 0, st>>>(part, kEkChunks * kEkRows, out);
 }
 
 void launch_dcoef(const double *v, int nstate, int ncoef, int ngp, const double *gk, double *out, cudaStream_t st) {

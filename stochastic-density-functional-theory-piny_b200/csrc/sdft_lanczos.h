@@ -6,6 +6,10 @@
 namespace sdft {
 
 constexpr int kRedBlocks = 128, kRedThreads = 256;  // partials of a deterministic reduction
+// row groups and G chunks of the kinetic energy's partials (kRedPart CTAs, each
+// keeping its |G|^2 over the rows of a group; 512 atoms, 256 orbitals, 214 MB:
+// 50 us, 128 CTAs of whole rows 148)
+constexpr int kEkRows = 32, kEkChunks = 32, kRedPart = kEkRows * kEkChunks;
 
 // *out = <a|b> over the half sphere (2 sum(re re + im im) - re(G0) re(G0));
 // part: kRedBlocks doubles of scratch
