@@ -28,11 +28,14 @@
 #include <cstdio>
 #include <vector>
 #include "sdft_internal.h"
-#include "sdft_fft.cuh"
+#include "sdft_fft2.cuh"
+#include "sdft_tw_edges.cuh"
+#include "sdft_xc.h"
 
 struct sdft_vks {
   int device = 0;
-  cudaStream_t st = nullptr;
+  cudaStream_t st = nullptr, st_copy = nullptr;  // st_copy: rho(G) to the host beside the second transform
+  cudaEvent_t ev_rhog = nullptr;
   int n1 = 0, n2 = 0, n3 = 0;
   long long N = 0;
   int ncoef = 0;  // half sphere + G0 (last)
@@ -57,7 +60,7 @@ struct sdft_vks {
 namespace sdft {
 namespace {
 
-constexpr int kLines = 16, kFftThreads = 256, kGBlocks = 128, kGThreads = 256;
+constexpr int kLines = 16, kFftThreads = 256, kGBlocks = 512, kGThreads = 256;
 
 // One axis of the three-axis FFT: every CTA transforms kLines lines of
 // length n held in shared memory (line pitch n + 1), in place, natural order
@@ -124,9 +127,102 @@ k_fft3_axis(double2 *__restrict__ z, int n1, int n2, int n3, int axis, const dou
   }
 }
 
-__global__ void k_pack_real(const double *__restrict__ r, double2 *__restrict__ z, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+// The same for an axis with a compile-time plan (n = R1 R2, sdft_fft2.cuh): two
+// register passes with one exchange through shared memory.  Pass 1 loads its R1
+// points straight from the grid, pass 2 stores its R2 outputs straight to it, at
+// their natural places k1 + R1 k2.  Consecutive threads take consecutive lines
+// (axes 1 and 2) or consecutive points of a line (axis 0), so a warp's accesses
+// are whole 128 B lines.  128^3: 20 us an axis (67 MB, L2 resident); the
+// radix-by-radix form above 33.
+// REAL_IN (axis 0): the grid is read from a real array, which is multiplied by
+// rscale in place; REAL_OUT (axis 2): only the real part is written, to out.
+template <int N, int DIR>
+__device__ __forceinline__ void fft_axis(double2 *z, double *rin, double rscale, double *rout,
+                                         double2 *buf, long long base0, int lstride, long long estride, int nl,
+                                         bool contig, double scale, int tid) {
+  constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2, PL = kLines + 1;
+  const TwC<N, double2> tw{};
+#pragma unroll 1
+  for (int u = tid; u < kLines * R2; u += kFftThreads) {
+    const int l = contig ? u / R2 : u % kLines, j2 = contig ? u % R2 : u / kLines;
+    if (l >= nl) continue;
+    const long long b = base0 + (long long)l * lstride + (long long)j2 * estride;
+    double2 v[R1];
+#pragma unroll
+    for (int j1 = 0; j1 < R1; j1++) {
+      const long long i = b + (long long)(R2 * j1) * estride;
+      if (rin) {
+        const double r = rin[i];
+        rin[i] = r * rscale;
+        v[j1] = make_double2(r, 0.0);
+      } else {
+        v[j1] = z[i];
+      }
+    }
+    dftr<R1, DIR>(v);
+    buf[j2 * PL + l] = v[0];
+#pragma unroll
+    for (int k1 = 1; k1 < R1; k1++) {
+      double2 w = tw(j2 * k1);
+      if (DIR > 0) w.y = -w.y;
+      buf[(j2 + R2 * k1) * PL + l] = cmul(v[k1], w);
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int u = tid; u < kLines * R1; u += kFftThreads) {
+    const int l = contig ? u / R1 : u % kLines, k1 = contig ? u % R1 : u / kLines;
+    if (l >= nl) continue;
+    double2 v[R2];
+#pragma unroll
+    for (int j = 0; j < R2; j++) v[j] = buf[(R2 * k1 + j) * PL + l];
+    dftr<R2, DIR>(v);
+    const long long b = base0 + (long long)l * lstride + (long long)k1 * estride;
+#pragma unroll
+    for (int k2 = 0; k2 < R2; k2++) {
+      const long long i = b + (long long)(R1 * k2) * estride;
+      if (rout) rout[i] = v[k2].x * scale;
+      else z[i] = make_double2(v[k2].x * scale, v[k2].y * scale);
+    }
+  }
+}
+
+template <int DIR>
+__global__ void __launch_bounds__(kFftThreads, 2)
+k_fft3_plan(double2 *__restrict__ z, int n1, int n2, int n3, int axis, double scale, double *__restrict__ rin,
+            double rscale, double *__restrict__ rout) {
+  extern __shared__ __align__(16) double2 sm[];
+  const int n = axis == 0 ? n1 : (axis == 1 ? n2 : n3);
+  long long base0 = 0, estride = 1;
+  int nl = kLines, lstride = 1;
+  if (axis == 0) {
+    const long long l0 = (long long)blockIdx.x * kLines;
+    nl = (int)min((long long)kLines, (long long)n2 * n3 - l0);
+    base0 = l0 * n1;
+    lstride = n1;
+  } else {
+    const int na = (n1 + kLines - 1) / kLines;
+    const int a0 = (blockIdx.x % na) * kLines, o = blockIdx.x / na;
+    nl = min(kLines, n1 - a0);
+    if (axis == 1) { base0 = a0 + (long long)n1 * n2 * o; estride = n1; }
+    else { base0 = a0 + (long long)n1 * o; estride = (long long)n1 * n2; }
+  }
+  switch (n) {
+#define SDFT_F(N)                                                                                             \
+  case N:                                                                                                     \
+    fft_axis<N, DIR>(z, rin, rscale, rout, sm, base0, lstride, estride, nl, axis == 0, scale, threadIdx.x); \
+    break;
+    SDFT_EDGES(SDFT_F)
+#undef SDFT_F
+  }
+}
+
+// z = rho + 0 i, rho *= rscale (grids whose first axis has no compile-time plan)
+__global__ void k_pack_real(double *__restrict__ r, double2 *__restrict__ z, double rscale, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     z[i] = make_double2(r[i], 0.0);
+    r[i] *= rscale;
+  }
 }
 
 // rho(G) from the transformed grid, the energies' block partials and V(G):
@@ -169,13 +265,23 @@ k_vks_gspace(const double2 *__restrict__ z, const int *__restrict__ map, const d
   }
 }
 
-// E_H = 2 sum, E_ext = 2 sum + vext(0) rho(0), in block order (one thread)
+// Sum of n partials by one warp: each lane its own in order, then a fixed tree.
+__device__ __forceinline__ double warp_sum_of(const double *__restrict__ part, int n) {
+  double a = 0.0;
+  for (int b = threadIdx.x & 31; b < n; b += 32) a += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
+// E_H = 2 sum, E_ext = 2 sum + vext(0) rho(0) (one warp)
 __global__ void k_vks_energies(const double *__restrict__ part, const double2 *__restrict__ vext,
                                const double *__restrict__ rhog, int ncoef, double *__restrict__ out) {
-  double eh = 0.0, ee = 0.0;
-  for (int b = 0; b < kGBlocks; b++) { eh += part[b]; ee += part[kGBlocks + b]; }
-  out[0] = 2.0 * eh;
-  out[1] = 2.0 * ee + vext[ncoef - 1].x * rhog[ncoef - 1];
+  const double eh = warp_sum_of(part, kGBlocks), ee = warp_sum_of(part + kGBlocks, kGBlocks);
+  if (threadIdx.x == 0) {
+    out[0] = 2.0 * eh;
+    out[1] = 2.0 * ee + vext[ncoef - 1].x * rhog[ncoef - 1];
+  }
 }
 
 __global__ void k_vks_scatter(const double2 *__restrict__ vg, const int *__restrict__ map,
@@ -188,24 +294,24 @@ __global__ void k_vks_scatter(const double2 *__restrict__ vg, const int *__restr
   }
 }
 
-// V(r) = Re z (package layout) and rho_in / vol for the xc step
-__global__ void k_vks_real(const double2 *__restrict__ z, const double *__restrict__ rho_in, double rvol,
-                           double *__restrict__ v, double *__restrict__ nr, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+// V(r) = Re z (grids whose last axis has no compile-time plan)
+__global__ void k_vks_real(const double2 *__restrict__ z, double *__restrict__ v, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     v[i] = z[i].x;
-    nr[i] = rho_in[i] * rvol;
-  }
 }
 
-// package layout (a fastest) -> filter layout (c fastest)
-__global__ void k_pkg_to_filter(const double *__restrict__ v, double *__restrict__ out, int n1, int n2, int n3) {
-  const long long N = (long long)n1 * n2 * n3;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    const int ic = (int)(i % n3);
-    const long long ab = i / n3;
-    const int ib = (int)(ab % n2), ia = (int)(ab / n2);
-    out[i] = v[ia + (long long)n1 * (ib + (long long)n2 * ic)];
-  }
+// package layout (a fastest) -> filter layout (c fastest), 32 x 32 tiles of (a, c)
+// at one b through shared memory
+constexpr int kTile = 32, kTileRows = 8;
+__global__ void __launch_bounds__(kTile * kTileRows)
+k_pkg_to_filter(const double *__restrict__ v, double *__restrict__ out, int n1, int n2, int n3) {
+  __shared__ double t[kTile][kTile + 1];
+  const int a0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile, b = blockIdx.z;
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+    if (c0 + j < n3 && a0 + threadIdx.x < n1) t[j][threadIdx.x] = v[a0 + threadIdx.x + (long long)n1 * (b + (long long)n2 * (c0 + j))];
+  __syncthreads();
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+    if (a0 + j < n1 && c0 + threadIdx.x < n3) out[((long long)(a0 + j) * n2 + b) * n3 + c0 + threadIdx.x] = t[threadIdx.x][j];
 }
 
 // vext(G) = (1/vol) sum_a v_t(a)(|G|) (cos, -sin)(2 pi k . s_a) for G != 0 and
@@ -332,10 +438,9 @@ __global__ void k_loc_force_sum(const double *__restrict__ fpart, int natm, cons
     for (int j = 0; j < kFChunks; j++) acc += fpart[((size_t)a * kFChunks + j) * 3 + d];
     out[e] = acc;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    double v = 0.0;
-    for (int b = 0; b < kGBlocks; b++) v += part[b];
-    out[3 * natm] = v;
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    const double v = warp_sum_of(part, kGBlocks);
+    if (threadIdx.x == 0) out[3 * natm] = v;
   }
 }
 
@@ -355,17 +460,30 @@ bool edge_ok(int n) {
   return n == 1;
 }
 
-int fft3(sdft_vks *v, int dir, double scale) {
+// Three-axis transform of d_z.  dir -1 starts from the real array rho (scaled by
+// rscale in place); dir +1 ends in the real array vout.
+int fft3(sdft_vks *v, int dir, double scale, double *rho, double rscale, double *vout) {
   const int ns[3] = {v->n1, v->n2, v->n3};
   const double2 *tw[3] = {v->d_tw, v->d_tw + v->n1, v->d_tw + v->n1 + v->n2};
+  const int blocks = (int)std::min<long long>((v->N + 255) / 256, 148 * 8);
   for (int axis = 0; axis < 3; axis++) {
     const int n = ns[axis];
-    const long long nblk = axis == 0 ? ((long long)v->n2 * v->n3 + kLines - 1) / kLines
-                                     : (long long)((v->n1 + kLines - 1) / kLines) * (axis == 1 ? v->n3 : v->n2);
-    const size_t smem = sizeof(double2) * (size_t)(n + kLines * (n + 1));
+    const unsigned nblk = axis == 0 ? (unsigned)(((long long)v->n2 * v->n3 + kLines - 1) / kLines)
+                                    : (unsigned)((v->n1 + kLines - 1) / kLines) * (axis == 1 ? v->n3 : v->n2);
     const double sc = axis == 2 ? scale : 1.0;
-    if (dir > 0) k_fft3_axis<+1><<<(unsigned)nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, tw[axis], sc);
-    else k_fft3_axis<-1><<<(unsigned)nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, tw[axis], sc);
+    const bool first = axis == 0 && dir < 0, last = axis == 2 && dir > 0;
+    if (plan_rt(n).r1) {
+      const size_t smem = sizeof(double2) * (size_t)n * (kLines + 1);
+      double *rin = first ? rho : nullptr, *rout = last ? vout : nullptr;
+      if (dir > 0) k_fft3_plan<+1><<<nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, sc, rin, rscale, rout);
+      else k_fft3_plan<-1><<<nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, sc, rin, rscale, rout);
+      continue;
+    }
+    if (first) k_pack_real<<<blocks, 256, 0, v->st>>>(rho, v->d_z, rscale, v->N);
+    const size_t smem = sizeof(double2) * (size_t)(n + kLines * (n + 1));
+    if (dir > 0) k_fft3_axis<+1><<<nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, tw[axis], sc);
+    else k_fft3_axis<-1><<<nblk, kFftThreads, smem, v->st>>>(v->d_z, v->n1, v->n2, v->n3, axis, tw[axis], sc);
+    if (last) k_vks_real<<<blocks, 256, 0, v->st>>>(v->d_z, vout, v->N);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SDFT_OK : set_error(SDFT_ERR_CUDA, cudaGetErrorString(e));
@@ -392,6 +510,8 @@ extern "C" int sdft_vks_destroy(sdft_vks *v) {
     cudaStreamSynchronize(v->st);
     cudaStreamDestroy(v->st);
   }
+  if (v->st_copy) cudaStreamDestroy(v->st_copy);
+  if (v->ev_rhog) cudaEventDestroy(v->ev_rhog);
   delete v;
   return SDFT_OK;
 }
@@ -425,7 +545,9 @@ extern "C" int sdft_vks_create(int n1, int n2, int n3, const double *hmat, int n
   v->vol = std::fabs(v->vol);
   v->ka.assign(ka, ka + ncoef); v->kb.assign(kb, kb + ncoef); v->kc.assign(kc, kc + ncoef);
   if (cudaSetDevice(device) != cudaSuccess) return fail(set_error(SDFT_ERR_CUDA, "cudaSetDevice failed"));
-  if (cudaStreamCreateWithFlags(&v->st, cudaStreamNonBlocking) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&v->st, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&v->st_copy, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&v->ev_rhog, cudaEventDisableTiming) != cudaSuccess)
     return fail(set_error(SDFT_ERR_CUDA, "stream create failed"));
   // grid positions (package layout, a fastest) of G and -G; |G|^2 (hmat
   // columns are the cell vectors, column-major: G = 2 pi k h^-1)
@@ -465,7 +587,7 @@ extern "C" int sdft_vks_create(int n1, int n2, int n3, const double *hmat, int n
   DMV(v->d_vpkg, v->N * sizeof(double));
   DMV(v->d_nr, v->N * sizeof(double));
   DMV(v->d_tw, tw.size() * sizeof(double2));
-  DMV(v->d_part, (2 * kGBlocks + 8) * sizeof(double));
+  DMV(v->d_part, (2 * kGBlocks + 8 + kXcScratch) * sizeof(double));
   DMV(v->d_rhog, 2 * (size_t)ncoef * sizeof(double));
 #undef DMV
   auto ck = [&](cudaError_t e) { return e == cudaSuccess ? SDFT_OK : set_error(SDFT_ERR_CUDA, cudaGetErrorString(e)); };
@@ -477,8 +599,10 @@ extern "C" int sdft_vks_create(int n1, int n2, int n3, const double *hmat, int n
       (r = ck(cudaStreamSynchronize(v->st))))
     return fail(r);
   {
-    const size_t smax = sizeof(double2) * (size_t)(128 + kLines * 129);
-    if ((r = ck(cudaFuncSetAttribute(k_fft3_axis<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax))) ||
+    const size_t smax = sizeof(double2) * (size_t)(128 + kLines * 129), smax2 = sizeof(double2) * (size_t)128 * (kLines + 1);
+    if ((r = ck(cudaFuncSetAttribute(k_fft3_plan<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax2))) ||
+        (r = ck(cudaFuncSetAttribute(k_fft3_plan<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax2))) ||
+        (r = ck(cudaFuncSetAttribute(k_fft3_axis<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax))) ||
         (r = ck(cudaFuncSetAttribute(k_fft3_axis<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax))))
       return fail(r);
   }
@@ -611,26 +735,21 @@ extern "C" int sdft_vks_from_rho(sdft_vks *v, const double *rho, int xc_kind, do
   if (!v->have_local) return set_error(SDFT_ERR_STATE, "vks_from_rho: local potential not set (sdft_vks_set_local)");
   cudaSetDevice(v->device);
   const long long N = v->N;
-  const int blocks = (int)std::min<long long>((N + 255) / 256, 148 * 8);
   // rho may be host or device memory: stage it in the real-space buffer
   CKV(cudaMemcpyAsync(v->d_nr, rho, N * sizeof(double), cudaMemcpyDefault, v->st));
-  k_pack_real<<<blocks, 256, 0, v->st>>>(v->d_nr, v->d_z, N);
   int r;
-  if ((r = fft3(v, -1, 1.0 / (double)N))) return r;
+  // (leaves rho_in / vol in d_nr for the xc step)
+  if ((r = fft3(v, -1, 1.0 / (double)N, v->d_nr, 1.0 / v->vol, nullptr))) return r;
+  double *d_e = v->d_part + 2 * kGBlocks;  // E_H, E_ext, then the xc sums
   k_vks_gspace<<<kGBlocks, kGThreads, 0, v->st>>>(v->d_z, v->d_map, v->d_ak2, v->d_vext, v->ncoef, v->vol, v->d_vg,
                                                  v->d_rhog, v->d_part);
-  k_vks_energies<<<1, 1, 0, v->st>>>(v->d_part, v->d_vext, v->d_rhog, v->ncoef, v->d_part + 2 * kGBlocks);
+  if (rho_g) CKV(cudaEventRecord(v->ev_rhog, v->st));
+  k_vks_energies<<<1, 32, 0, v->st>>>(v->d_part, v->d_vext, v->d_rhog, v->ncoef, d_e);
   CKV(cudaMemsetAsync(v->d_z, 0, N * sizeof(double2), v->st));
   k_vks_scatter<<<(int)std::min(((long long)v->ncoef + 255) / 256, 148LL * 8), 256, 0, v->st>>>(
       v->d_vg, v->d_map, v->d_mapc, v->ncoef, v->d_z);
-  if ((r = fft3(v, +1, 1.0))) return r;
-  // d_nr held rho_in; V(r) into d_vpkg, rho_in / vol back into d_nr
-  k_vks_real<<<blocks, 256, 0, v->st>>>(v->d_z, v->d_nr, 1.0 / v->vol, v->d_vpkg, v->d_nr, N);
-  CKV(cudaGetLastError());
-  double e[4] = {0.0, 0.0, 0.0, 0.0};
-  if (xc_kind) {
-    if ((r = sdft_xc_lda_dev(xc_kind, N, v->d_nr, v->d_vpkg, v->vol, &e[2], &e[3], v->st))) return r;
-  }
+  if ((r = fft3(v, +1, 1.0, nullptr, 0.0, v->d_vpkg))) return r;
+  if (xc_kind) launch_xc_lda(xc_kind, N, v->d_nr, v->d_vpkg, d_e + 8, d_e + 2, v->st);
   // into the filter layout: the caller's buffer directly when it is device
   // memory, else through the work grid (free again at this point)
   cudaPointerAttributes at{};
@@ -638,12 +757,22 @@ extern "C" int sdft_vks_from_rho(sdft_vks *v, const double *rho, int xc_kind, do
                        (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged);
   cudaGetLastError();
   double *dst = dev_out ? vks_filter : reinterpret_cast<double *>(v->d_z);
-  k_pkg_to_filter<<<blocks, 256, 0, v->st>>>(v->d_vpkg, dst, v->n1, v->n2, v->n3);
+  k_pkg_to_filter<<<dim3((v->n1 + kTile - 1) / kTile, (v->n3 + kTile - 1) / kTile, v->n2), dim3(kTile, kTileRows), 0,
+                    v->st>>>(v->d_vpkg, dst, v->n1, v->n2, v->n3);
   CKV(cudaGetLastError());
+  // rho(G) leaves on the copy stream while the kernels queued above run
+  if (rho_g) {
+    CKV(cudaStreamWaitEvent(v->st_copy, v->ev_rhog, 0));
+    CKV(cudaMemcpyAsync(rho_g, v->d_rhog, 2 * (size_t)v->ncoef * sizeof(double), cudaMemcpyDefault, v->st_copy));
+    CKV(cudaStreamSynchronize(v->st_copy));
+  }
   if (!dev_out) CKV(cudaMemcpyAsync(vks_filter, dst, N * sizeof(double), cudaMemcpyDeviceToHost, v->st));
-  if (rho_g) CKV(cudaMemcpyAsync(rho_g, v->d_rhog, 2 * (size_t)v->ncoef * sizeof(double), cudaMemcpyDefault, v->st));
-  CKV(cudaMemcpyAsync(e, v->d_part + 2 * kGBlocks, 2 * sizeof(double), cudaMemcpyDeviceToHost, v->st));
+  double h[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, e[4] = {0.0, 0.0, 0.0, 0.0};
+  CKV(cudaMemcpyAsync(h, d_e, (xc_kind ? 5 : 2) * sizeof(double), cudaMemcpyDeviceToHost, v->st));
   CKV(cudaStreamSynchronize(v->st));
+  e[0] = h[0];
+  e[1] = h[1];
+  if (xc_kind) xc_energies(h + 2, v->vol / (double)N, &e[2], &e[3]);
   v->have_rho = true;
   if (energies) for (int i = 0; i < 4; i++) energies[i] = e[i];
   return SDFT_OK;
