@@ -268,20 +268,19 @@ k_vks_gspace(const double2 *__restrict__ z, const int *__restrict__ map, const d
 // Sum of n partials by one warp: each lane its own in order, then a fixed tree.
 __device__ __forceinline__ double warp_sum_of(const double *__restrict__ part, int n) {
   double a = 0.0;
+#pragma unroll 8
   for (int b = threadIdx.x & 31; b < n; b += 32) a += part[b];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
   return a;
 }
 
-// E_H = 2 sum, E_ext = 2 sum + vext(0) rho(0) (one warp)
+// E_H = 2 sum, E_ext = 2 sum + vext(0) rho(0) (a warp each)
 __global__ void k_vks_energies(const double *__restrict__ part, const double2 *__restrict__ vext,
                                const double *__restrict__ rhog, int ncoef, double *__restrict__ out) {
-  const double eh = warp_sum_of(part, kGBlocks), ee = warp_sum_of(part + kGBlocks, kGBlocks);
-  if (threadIdx.x == 0) {
-    out[0] = 2.0 * eh;
-    out[1] = 2.0 * ee + vext[ncoef - 1].x * rhog[ncoef - 1];
-  }
+  const double s = warp_sum_of(part + (threadIdx.x >> 5) * kGBlocks, kGBlocks);
+  if (threadIdx.x == 0) out[0] = 2.0 * s;
+  if (threadIdx.x == 32) out[1] = 2.0 * s + vext[ncoef - 1].x * rhog[ncoef - 1];
 }
 
 __global__ void k_vks_scatter(const double2 *__restrict__ vg, const int *__restrict__ map,
@@ -744,7 +743,7 @@ extern "C" int sdft_vks_from_rho(sdft_vks *v, const double *rho, int xc_kind, do
   k_vks_gspace<<<kGBlocks, kGThreads, 0, v->st>>>(v->d_z, v->d_map, v->d_ak2, v->d_vext, v->ncoef, v->vol, v->d_vg,
                                                  v->d_rhog, v->d_part);
   if (rho_g) CKV(cudaEventRecord(v->ev_rhog, v->st));
-  k_vks_energies<<<1, 32, 0, v->st>>>(v->d_part, v->d_vext, v->d_rhog, v->ncoef, d_e);
+  k_vks_energies<<<1, 64, 0, v->st>>>(v->d_part, v->d_vext, v->d_rhog, v->ncoef, d_e);
   CKV(cudaMemsetAsync(v->d_z, 0, N * sizeof(double2), v->st));
   k_vks_scatter<<<(int)std::min(((long long)v->ncoef + 255) / 256, 148LL * 8), 256, 0, v->st>>>(
       v->d_vg, v->d_map, v->d_mapc, v->ncoef, v->d_z);

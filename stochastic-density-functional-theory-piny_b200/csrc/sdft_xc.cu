@@ -84,14 +84,18 @@ __global__ void __launch_bounds__(kXcThreads) k_xc_lda(const double *__restrict_
   if (threadIdx.x < 3) part[(size_t)threadIdx.x * kXcBlocks + blockIdx.x] = sh[threadIdx.x][0];
 }
 
-// one warp per sum: each lane its blocks in order, then a fixed tree
-__global__ void __launch_bounds__(96) k_xc_sum(const double *__restrict__ part, double *__restrict__ out) {
-  const int d = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// one CTA per sum: each thread its blocks in order, then a fixed tree
+__global__ void __launch_bounds__(kXcThreads) k_xc_sum(const double *__restrict__ part, double *__restrict__ out) {
+  __shared__ double sh[kXcThreads];
   double s = 0.0;
-  for (int b = lane; b < kXcBlocks; b += 32) s += part[(size_t)d * kXcBlocks + b];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[d] = s;
+  for (int b = threadIdx.x; b < kXcBlocks; b += kXcThreads) s += part[(size_t)blockIdx.x * kXcBlocks + b];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int h = kXcThreads / 2; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
 }  // namespace
@@ -100,7 +104,7 @@ void launch_xc_lda(int kind, long long n, const double *rho, double *vks, double
                    cudaStream_t st) {
   if (kind == SDFT_XC_PZ_LDA) k_xc_lda<SDFT_XC_PZ_LDA><<<kXcBlocks, kXcThreads, 0, st>>>(rho, vks, n, scratch);
   else k_xc_lda<SDFT_XC_PW_LDA><<<kXcBlocks, kXcThreads, 0, st>>>(rho, vks, n, scratch);
-  k_xc_sum<<<1, 96, 0, st>>>(scratch, sums);
+  k_xc_sum<<<3, kXcThreads, 0, st>>>(scratch, sums);
 }
 }  // namespace sdft
 
