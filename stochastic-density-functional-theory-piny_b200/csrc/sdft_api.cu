@@ -295,7 +295,7 @@ static int default_plane_threads(const sdft_ctx *c) {
 // Whether the kernels of an H application on nstate orbitals start early
 // (sdft_pdl.cuh).  It hides the start of every kernel, which is what short
 // applications spend (per filter step: 64 atoms x 128 orbitals 116 -> 100 us, 8 x
-// 16 FP64 27 -> 21); at 512 atoms x 512 orbitals, 24576 planes, the waiting CTAs
+// 16 FP64 26.8 -> 17.4); at 512 atoms x 512 orbitals, 24576 planes, the waiting CTAs
 // cost 1 to 2 % instead, and in a graph of several systems they hold SMs that
 // another system's kernel could use (six uneven systems 2 % slower).
 constexpr long long kEarlyPlanes = 8192;
@@ -723,11 +723,20 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   g.plane_nt = default_plane_threads(ctx);
   g.ncoef = ncoef; g.ngp = ctx->ngp;
   g.ncols = ctx->cols.ncols; g.ncols_pad = ctx->cols.ncols_pad; g.ncp = ctx->cols.ncp; g.kamax = ctx->cols.kamax;
-  // fewer columns per CTA where the context's orbitals make fewer than two
-  // CTAs per SM of the default size: 8 atoms, 16 orbitals, FP64, 24 CTAs of 32
-  // column pairs took 7.6 us per stage C, 88 of 8 pairs 3.9
+  // columns per CTA: the size whose rounds of resident CTAs (8 per SM in FP32, 5
+  // in FP64) take the shorter time for the context's orbitals.  A small CTA fills
+  // its threads less well: 1.25 times the time per column from edge 36 on, about
+  // twice below (its passes then have fewer units than threads).  8 atoms, 16
+  // orbitals, FP64: 24 CTAs of 32 column pairs 7.6 us per stage C, 88 of 8 pairs
+  // 3.9; 48^3, 64 pairs: 1408 CTAs of 16 (1.2 rounds) 28.7 us, 2752 of 8 26.8.
   int cpb = ctx->fast ? col_cpb(n3) : kCPB;
-  if (ctx->fast && (long long)ctx->npairs_max * ((g.ncp + cpb - 1) / cpb) < 2 * 148) cpb = kCPBSmall;
+  if (ctx->fast && cpb > kCPBSmall) {
+    const long long slots = 148 * (is_fp64(ctx) ? 5 : 8);
+    auto time = [&](int c) {
+      return (double)c * (double)(((long long)ctx->npairs_max * ((g.ncp + c - 1) / c) + slots - 1) / slots);
+    };
+    if (time(kCPBSmall) * (n3 >= 36 ? 1.25 : 2.0) < time(cpb)) cpb = kCPBSmall;
+  }
   g.cpb = cpb;
   g.nbatch = (g.ncp + cpb - 1) / cpb;
   g.cp_gstart = ctx->d_cp_gstart; g.cp_gcount = ctx->d_cp_gcount; g.col_ab = ctx->d_col_ab;

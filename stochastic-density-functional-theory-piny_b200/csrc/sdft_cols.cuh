@@ -31,10 +31,10 @@ namespace sdft {
 // Threads and resident CTAs of the column kernels.  Small CTAs: the phases
 // are separated by barriers and each waits for its own loads, so what hides
 // one CTA's wait is another CTA, not more threads of the same.  Stage C at
-// 96^3, 256 pairs, FP32, per launch: 128 threads x 8 CTAs/SM (64 registers,
-// no spills) 0.697 ms; x 7 and 6 0.743 and 0.758; 96 x 10 0.707; 64 x 16 with
+// 96^3, 256 pairs, FP32, per launch: 128 threads x 8 CTAs/SM (64 registers, 104
+// bytes of spill loads a thread) 0.697 ms; x 7 and 6 0.743 and 0.758; 96 x 10 0.707; 64 x 16 with
 // half the columns 0.709; 160 x 8 0.714; 192 x 8 0.791; 256 x 5 0.788;
-// 256 x 6 (40 registers, spills) 0.822.  The earlier form -- 256 x 6, two
+// 256 x 6 (40 registers) 0.822.  The earlier form -- 256 x 6, two
 // buffers, columns copied through shared memory before and after the
 // transforms -- took 0.965 ms, 42.4 us at 48^3 and 64 pairs (28.7 now) and
 // 65.7 us at N3 = 24 with moment dots (19.3 now).  Bound: 2.98 GB at 96^3,
