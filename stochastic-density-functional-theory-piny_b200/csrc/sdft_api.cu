@@ -542,9 +542,8 @@ static int filter_cheby_core(sdft_ctx *ctx, int nstate, int L, int nmu, double s
     }
     if ((r = apply_h(ctx, cur, nstate, e, false))) return r;
     if (store_moments) {
-      launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
-                         ctx->st);
-      ctx->launches += 2;
+      ctx->launches += launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3,
+                                          ctx->d_mom + (size_t)k * 3, ctx->st);
     }
     prev = cur;
     cur = out;
@@ -605,9 +604,8 @@ static int moments_core(sdft_ctx *ctx, int nstate, int L, double scale, double e
       e.PREV = prev;
     }
     if ((r = apply_h(ctx, cur, nstate, e, false))) return r;
-    launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3, ctx->d_mom + (size_t)k * 3,
-                       ctx->st);
-    ctx->launches += 2;
+    ctx->launches += launch_dots_reduce(ctx->g.early, ctx->d_dots, nparts, 3, ctx->d_dots + ctx->dots_cap * 3,
+                                        ctx->d_mom + (size_t)k * 3, ctx->st);
     prev = cur;
     cur = out;
   }

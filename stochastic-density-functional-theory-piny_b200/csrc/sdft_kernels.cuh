@@ -148,9 +148,9 @@ int launch_gemm_nt_f64(const GemmPlan &p, bool early, const double *A, int lda, 
                        int K, int Mst, int Nst, double *work, cudaStream_t st);
 
 // sum over nparts CTA partials (3 doubles each) -> out[0, ndots); blk: kDotBlocks*3
-// doubles of scratch (two launches, fixed order)
+// doubles of scratch (fixed order; returns the launches made, one or two)
 constexpr int kDotBlocks = 128;
-void launch_dots_reduce(bool early, const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st);
+int launch_dots_reduce(bool early, const double *part, int nparts, int ndots, double *blk, double *out, cudaStream_t st);
 // E_NL = sum_u w[u] sum_{s<nstate} Z[s*ldz + u]^2 -> out[0]; out[1 .. kEnlBlocks]
 // hold the partials (two launches)
 constexpr int kEnlBlocks = 128;
