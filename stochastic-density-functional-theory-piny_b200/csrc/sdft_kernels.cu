@@ -751,6 +751,11 @@ void launch_density_reduce(const double *rho_part, int nsplit, int N, double sca
 // 207, 188 us.  8 atoms, 16 orbitals: 32 x 16 2.1 us against 15.5 of 128 x 64;
 // 512 atoms, one orbital: 128 x 8 284 us (6.0 TB/s of projector) against 1650.
 struct GemmShape { int bm, bn; double eff; };
+// the share of that rate reached with one, two, three CTAs on an SM (a CTA's
+// warps wait for their own stages and barriers): with it the projection of 216
+// atoms x 64 orbitals splits K 31 ways, three CTAs an SM, instead of 21, two an
+// SM; the FP64 filter takes 7.85 ms instead of 8.20
+constexpr double kGemmFill[] = {0.75, 0.9, 1.0};
 constexpr GemmShape kGemmShapes[] = {{64, 64, 1.0}, {64, 32, 0.92}, {32, 16, 0.85},
                                      {128, 16, 0.9}, {128, 8, 0.85}, {32, 8, 0.8}};
 
@@ -762,7 +767,8 @@ static double gemm_cost(GemmShape t, int M, int N, int K, int split) {
   const int it = (K / GBK + split - 1) / split;
   const long long ctas = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * split;
   const double per_sm = (double)((ctas + 147) / 148);
-  const double mma = (double)t.bm * t.bn * GBK / (62.0 * 1900.0 * t.eff);
+  const double fill = t.bm * t.bn >= 2048 ? kGemmFill[(int)std::min(per_sm, 3.0) - 1] : 1.0;
+  const double mma = (double)t.bm * t.bn * GBK / (62.0 * 1900.0 * t.eff * fill);
   const double mem = (double)(t.bm + t.bn) * GBK * 8.0 / 44000.0;
   const double chain = 1.0 + it * std::max(0.18, mma);
   double us = std::max(chain, 1.0 + per_sm * it * std::max(mma, mem));
