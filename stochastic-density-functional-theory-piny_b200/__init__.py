@@ -191,6 +191,17 @@ def _f64(a):
     return np.ascontiguousarray(a, dtype=np.float64)
 
 
+def _out(like, n):
+    """An array like `like` whose first n values the call will write: not
+    cleared first, since on a large result that costs as much as the copy that
+    fills it (V_KS at 128^3, 16.8 MB: 1.13 ms a call with cleared arrays, 0.60
+    without; six filters of 48 to 216 atoms 6.3 and 5.8)."""
+    a = np.empty_like(like)
+    if a.size > n:
+        a.reshape(-1)[n:] = 0.0
+    return a
+
+
 def _i32(a):
     return np.ascontiguousarray(a, dtype=np.int32)
 
@@ -436,21 +447,21 @@ class Context:
     # -- hot path (host buffers)
     def calc_coef_force(self, cre, cim, want_enl=False):
         cre, cim = _f64(cre), _f64(cim)
-        fr, fi = np.zeros_like(cre), np.zeros_like(cim)
+        fr, fi = _out(cre, cre.size), _out(cim, cre.size)
         e = C.c_double(0.0)
         _chk(lib.sdft_hpsi(self._p, self._ns(cre), _d(cre), _d(cim), _d(fr), _d(fi), C.byref(e) if want_enl else None))
         return (fr, fi, e.value) if want_enl else (fr, fi)
 
     def normHCheby(self, cre, cim, wf1re, wf1im, ipoly, scale, energy_mean, cpy_flag=1):
         """In place like normHCheby: returns (fcre, fcim); with cpy_flag cre/cim/wf1 rotate."""
-        fr, fi = np.zeros_like(cre), np.zeros_like(cim)
+        fr, fi = _out(cre, cre.size), _out(cim, cre.size)
         _chk(lib.sdft_normh_cheby(self._p, self._ns(cre), ipoly, cpy_flag, scale, energy_mean, _d(cre), _d(cim),
                                   _d(wf1re) if wf1re is not None else None, _d(wf1im) if wf1im is not None else None,
                                   _d(fr), _d(fi)))
         return fr, fi
 
     def normHNewtonHerm(self, cre, cim, scale, energy_mean, zn):
-        fr, fi = np.zeros_like(cre), np.zeros_like(cim)
+        fr, fi = _out(cre, cre.size), _out(cim, cre.size)
         _chk(lib.sdft_normh_newton(self._p, self._ns(cre), scale, energy_mean, zn, _d(cre), _d(cim), _d(fr), _d(fi)))
         return fr, fi
 
@@ -459,8 +470,8 @@ class Context:
         ec = _f64(expan_coeff)
         L = ec.size // num_chem_pot
         ns = self._ns(cre)
-        sre = [np.zeros_like(cre) for _ in range(num_chem_pot)]
-        sim = [np.zeros_like(cim) for _ in range(num_chem_pot)]
+        sre = [_out(cre, cre.size) for _ in range(num_chem_pot)]
+        sim = [_out(cim, cre.size) for _ in range(num_chem_pot)]
         pr = (_dp * num_chem_pot)(*[_d(a) for a in sre])
         pi = (_dp * num_chem_pot)(*[_d(a) for a in sim])
         mom = np.zeros(L + 1) if store_moments else None
@@ -473,8 +484,8 @@ class Context:
         ec, sp = _f64(expan_coeff), _f64(samp_point)
         L = ec.size // num_chem_pot
         ns = self._ns(cre)
-        sre = [np.zeros_like(cre) for _ in range(num_chem_pot)]
-        sim = [np.zeros_like(cim) for _ in range(num_chem_pot)]
+        sre = [_out(cre, cre.size) for _ in range(num_chem_pot)]
+        sim = [_out(cim, cre.size) for _ in range(num_chem_pot)]
         pr = (_dp * num_chem_pot)(*[_d(a) for a in sre])
         pi = (_dp * num_chem_pot)(*[_d(a) for a in sim])
         _chk(lib.sdft_filter_newton(self._p, ns, _d(cre), _d(cim), L, num_chem_pot, _d(ec), _d(sp), scale,
@@ -490,13 +501,13 @@ class Context:
     def rhoCalcRealStoHybrid(self, cre, cim):
         """sum_s |psi_s(r)|^2 in package layout (a fastest), unscaled."""
         cre, cim = _f64(cre), _f64(cim)
-        rho = np.zeros(self.n[0] * self.n[1] * self.n[2])
+        rho = np.empty(self.n[0] * self.n[1] * self.n[2])
         _chk(lib.sdft_density(self._p, self._ns(cre), _d(cre), _d(cim), _d(rho)))
         return rho
 
     def genNoiseOrbitalReal(self, nstate, seed=10.0, np_states=1, myid=0):
-        cre = np.zeros(nstate * self.ncoef)
-        cim = np.zeros(nstate * self.ncoef)
+        cre = np.empty(nstate * self.ncoef)
+        cim = np.empty(nstate * self.ncoef)
         _chk(lib.sdft_noise_real(self._p, nstate, seed, np_states, myid, _d(cre), _d(cim)))
         return cre, cim
 
@@ -530,13 +541,13 @@ class Context:
         if out_ptr is not None:
             _chk(lib.sdft_density_dev(self._p, nstate, imu, scale, C.cast(C.c_void_p(out_ptr), _dp)))
             return None
-        rho = np.zeros(self.n[0] * self.n[1] * self.n[2]) if want else None
+        rho = np.empty(self.n[0] * self.n[1] * self.n[2]) if want else None
         _chk(lib.sdft_density_dev(self._p, nstate, imu, scale, _d(rho) if want else None))
         return rho
 
     def download_density(self):
         """The last density computed on this context (no recomputation)."""
-        rho = np.zeros(self.n[0] * self.n[1] * self.n[2])
+        rho = np.empty(self.n[0] * self.n[1] * self.n[2])
         _chk(lib.sdft_download_density(self._p, _d(rho)))
         return rho
 
@@ -603,8 +614,8 @@ class Context:
         return int(lib.sdft_ctx_stream(self._p) or 0)
 
     def download_filtered(self, nstate, imu=0):
-        re = np.zeros(nstate * self.ncoef)
-        im = np.zeros(nstate * self.ncoef)
+        re = np.empty(nstate * self.ncoef)
+        im = np.empty(nstate * self.ncoef)
         _chk(lib.sdft_download_filtered(self._p, nstate, imu, _d(re), _d(im)))
         return re, im
 
@@ -669,11 +680,11 @@ class DensityGrid:
             rp = C.c_void_p(rho.ctypes.data)
         v = None
         if out_ptr is None:
-            v = np.zeros(N)
+            v = np.empty(N)
             vp = C.c_void_p(v.ctypes.data)
         else:
             vp = C.c_void_p(int(out_ptr))
-        rg = np.zeros(2 * self.ncoef)
+        rg = np.empty(2 * self.ncoef)
         e = np.zeros(4)
         _chk(lib.sdft_vks_from_rho(self._p, rp, int(xc_kind), vp, _d(rg), _d(e)))
         return v, rg[:self.ncoef], rg[self.ncoef:], e
