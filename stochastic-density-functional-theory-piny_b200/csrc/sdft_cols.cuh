@@ -37,8 +37,9 @@ namespace sdft {
 // 256 x 6 (40 registers) 0.822.  The earlier form -- 256 x 6, two
 // buffers, columns copied through shared memory before and after the
 // transforms -- took 0.965 ms, 42.4 us at 48^3 and 64 pairs (28.7 now) and
-// 65.7 us at N3 = 24 with moment dots (19.3 now).  Bound: 2.98 GB at 96^3,
-// 0.65 of the copy bandwidth.
+// 65.7 us at N3 = 24 with moment dots (19.3 now).  (All before the order of the
+// epilogue's loads, 682 -> 611 us, see epilogue_pair.)  Bound: 2.98 GB at 96^3,
+// 4.9 TB/s, 0.73 of a copy; the waits for those loads.
 // FP64: 128 x 5 46.5 us at 72^3 and 32 pairs, 256 x 3 53.3, 192 x 4 49.0.
 template <typename T, int N3, int CPB> struct ColCfg {
   static constexpr int NL = 2 * CPB;
@@ -154,18 +155,12 @@ __device__ __forceinline__ void epilogue_pair(const DevGeom &g, const EpiArgs &e
   } else {
     const bool rec = KIND != COL_RAW && (e.mode == EPI_CHEBK || e.mode == EPI_MOMK);
     const bool acc1 = KIND != COL_RAW && e.ACC && e.nmu == 1 && !e.acoef0;
+    const double w = g.ak2[gi];
     double c1r = e.C[o1], c1i = e.C[o1 + n], c2r = 0.0, c2i = 0.0;
     double x1r = 0.0, x1i = 0.0, x2r = 0.0, x2i = 0.0;
     double p1r = 0.0, p1i = 0.0, p2r = 0.0, p2i = 0.0;
     double q1r = 0.0, q1i = 0.0, q2r = 0.0, q2i = 0.0;
     if (has2) { c2r = e.C[o2]; c2i = e.C[o2 + n]; }
-    if (e.FNLf) {
-      x1r = e.FNLf[o1]; x1i = e.FNLf[o1 + n];
-      if (has2) { x2r = e.FNLf[o2]; x2i = e.FNLf[o2 + n]; }
-    } else if (e.FNL) {
-      x1r = e.FNL[o1]; x1i = e.FNL[o1 + n];
-      if (has2) { x2r = e.FNL[o2]; x2i = e.FNL[o2 + n]; }
-    }
     if (rec) {
       p1r = e.PREV[o1]; p1i = e.PREV[o1 + n];
       if (has2) { p2r = e.PREV[o2]; p2i = e.PREV[o2 + n]; }
@@ -179,7 +174,17 @@ __device__ __forceinline__ void epilogue_pair(const DevGeom &g, const EpiArgs &e
       h1r = e.CHI[o1]; h1i = e.CHI[o1 + n];
       if (has2) { h2r = e.CHI[o2]; h2i = e.CHI[o2 + n]; }
     }
-    const double k2 = g0 ? 0.0 : 2.0 * g.ak2[gi];
+    // last: the FP32 values are widened inside the branch, which waits for them,
+    // and no load after that wait is in flight with these (96^3, 256 pairs, this
+    // block right after c: 682 us, here 611)
+    if (e.FNLf) {
+      x1r = e.FNLf[o1]; x1i = e.FNLf[o1 + n];
+      if (has2) { x2r = e.FNLf[o2]; x2i = e.FNLf[o2 + n]; }
+    } else if (e.FNL) {
+      x1r = e.FNL[o1]; x1i = e.FNL[o1 + n];
+      if (has2) { x2r = e.FNL[o2]; x2i = e.FNL[o2 + n]; }
+    }
+    const double k2 = g0 ? 0.0 : 2.0 * w;
     ar = f1r + x1r - k2 * c1r;
     br = f2r + x2r - k2 * c2r;
     ai = g0 ? 0.0 : f1i + x1i - k2 * c1i;
