@@ -97,7 +97,10 @@ def _bytes(grid, ncoef, cols, natm, nsto):
     ppad = (P + 127) // 128 * 128
     kp = (2 * ncoef + 63) // 64 * 64
     mpad = (2 * ncoef + 127) // 128 * 128
-    return int(5 * vec + npairs * n3 * cols * 8 + npairs * n1 * n2 * n3 * 8 + 4 * (ppad * kp + mpad * ppad)
+    # projector bytes per value: four digits, or FP64 where the projections are
+    # small (csrc/sdft_kb.cu kOzMinWork, 9e7; with room for padding)
+    pv = 8 if P * kp * nsto < 1.0e8 else 4
+    return int(5 * vec + npairs * n3 * cols * 8 + npairs * n1 * n2 * n3 * 8 + pv * (ppad * kp + mpad * ppad)
                + 4 * spad * (kp + ppad) + 32 * spad * ppad * 8 + 64 * 2 ** 20)
 
 

@@ -65,3 +65,16 @@ def test_mixed_on_both_sides_of_the_digit_limit(pkg, sys1, nmax):
         assert rel_l2(np.concatenate([fr, fi]), np.concatenate(ref[:2])) < tol
         assert abs(e - ref[2]) < 1e-6 * abs(ref[2])
         ctx.close()
+
+
+@pytest.mark.parametrize("cells,grid,ns", [((2, 2, 2), (48, 48, 48), 2), ((3, 3, 3), (72, 72, 72), 2),
+                                           ((3, 3, 3), (72, 72, 72), 4)])  # FP64, FP64 and digit projectors
+def test_estimate_covers_either_form(pkg, wl, cells, grid, ns):
+    serve = __import__(pkg.__name__ + ".serve", fromlist=["estimate_bytes"])
+    s = wl.make_system(cells, grid)
+    ctx = _ctx(pkg, s, pkg.SDFT_PREC_MIXED, ns)
+    ctx.noise_dev(ns)
+    ctx.filter_cheby_dev(ns, np.ones(3), 1, 0.1, 2.0)
+    ctx.density_dev(ns, want=False)
+    assert ctx.device_bytes <= serve.estimate_bytes(s, ns)
+    ctx.close()
