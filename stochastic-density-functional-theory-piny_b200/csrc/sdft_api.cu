@@ -309,11 +309,13 @@ static bool early_ok(const sdft_ctx *ctx, int nstate) {
 // reduction also produces the digit form of Z for FNL = Bk Z.
 // gk (nullable): project i G_d vec instead of vec, formed inside the digit
 // pass (gk = G_d per coefficient).  max_of (nullable without gk): the row maxima
-// of what is projected.
+// of what is projected.  side (nullable): the stream to run on instead of ctx->st.
 static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
-                     const double *gk = nullptr, const unsigned long long *max_of = nullptr) {
+                     const double *gk = nullptr, const unsigned long long *max_of = nullptr,
+                     cudaStream_t side = nullptr) {
   const int K1 = 2 * ctx->ngp, S = ctx->s_oz, Ppad = ctx->Ppad;
-  const bool early = early_ok(ctx, nstate);
+  const cudaStream_t st = side ? side : ctx->st;
+  const bool early = early_ok(ctx, nstate), first = early && !side;
   // tile width: the set one, else 64 where it pads the orbitals less; for the
   // projection also where 128-wide tiles with the longest split (32) leave SMs
   // idle (64 atoms, 128 orbitals: 16.4 us at 128, 13.2 at 64; the back projection
@@ -325,16 +327,16 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
     TScope ts(ctx, 7);
     if (gk) {
       launch_oz_slice_igc(vec, gk, ctx->ngp, ctx->ncoef, nstate, max_of, ctx->d_c_dig, ctx->kp_oz,
-                          (size_t)S * ctx->kp_oz, ctx->d_c_sc, ctx->st);
+                          (size_t)S * ctx->kp_oz, ctx->d_c_sc, st);
       ctx->launches++;
     } else {
       // row maxima: from the stage C that wrote `vec`, else one pass over it
       if (!max_of && !(ctx->track_omax && ctx->omax_vec == vec && ctx->omax_n == nstate)) {  // (set only when oz)
-        launch_oz_rowmax(vec, K1, nstate, K1, ctx->d_rowmax, ctx->st);  // clears the rows first
+        launch_oz_rowmax(vec, K1, nstate, K1, ctx->d_rowmax, st);  // clears the rows first
         ctx->launches++;
       }
       launch_oz_slice(vec, K1, nstate, K1, max_of ? max_of : ctx->d_rowmax, ctx->d_c_dig, ctx->kp_oz, (size_t)S * ctx->kp_oz,
-                      ctx->d_c_sc, ctx->st, OZ_7x4, early);
+                      ctx->d_c_sc, st, OZ_7x4, first);
       ctx->launches++;
     }
   }
@@ -356,18 +358,18 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
   {
     TScope ts(ctx, 3);
     int used = split;  // the partials the launch writes (K tiles dealt out evenly)
-    r = run_gemm_oz(g1, split, ctx->d_oz_part, stride, ctx->d_err, ctx->st, &used);
+    r = run_gemm_oz(g1, split, ctx->d_oz_part, stride, ctx->d_err, st, &used);
     if (r) return r;
     // also zeroes d_rowmax[0, nstate) for the next stage C (the slice above
     // has consumed it)
     launch_oz_reduce_slice(ctx->d_oz_part, used, stride, Ppad, ctx->P, nstate, ctx->d_z, ctx->d_z_dig,
-                           (size_t)S * Ppad, ctx->d_z_sc, ctx->d_rowmax, ctx->st, ctx->om2.fmt, early);
+                           (size_t)S * Ppad, ctx->d_z_sc, ctx->d_rowmax, st, ctx->om2.fmt, early);
     ctx->launches += 2;
     ctx->rowmax_zero_n = nstate;
     ctx->omax_vec = nullptr;
   }
   if (want_enl) {
-    launch_enl(ctx->d_z, Ppad, ctx->d_w, ctx->P, nstate, ctx->d_enl, ctx->st);
+    launch_enl(ctx->d_z, Ppad, ctx->d_w, ctx->P, nstate, ctx->d_enl, st);
     ctx->launches += 2;
   }
   if (!back) return SDFT_OK;
@@ -375,16 +377,18 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
     TScope ts(ctx, 4);
     // FNL in FP32 (its rounding is below the FP32 transforms' error in the
     // same force); stage C reads it through EpiArgs::FNLf
-    r = run_gemm_oz(g2, 1, reinterpret_cast<float *>(ctx->d_fnl), 0, ctx->d_err, ctx->st);
+    r = run_gemm_oz(g2, 1, reinterpret_cast<float *>(ctx->d_fnl), 0, ctx->d_err, st);
     ctx->launches++;
   }
   return r;
 }
 
-static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true) {
+static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
+                  cudaStream_t side = nullptr) {
   if (ctx->P == 0) return SDFT_OK;
-  if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back);
+  if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back, nullptr, nullptr, side);
   const int K1 = 2 * ctx->ngp;
+  const cudaStream_t st = side ? side : ctx->st;
   const bool early = early_ok(ctx, nstate);
   // K of the back projection: the projector rows up to a multiple of 16 (the
   // padding columns of Bk and Z are zero)
@@ -397,29 +401,69 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
   }
   {
     TScope ts(ctx, 3);
-    ctx->launches += launch_gemm_nt_f64(ctx->plan1, early, ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, K1, ctx->P, nstate,
-                                        ctx->d_zwork, ctx->st);
+    ctx->launches += launch_gemm_nt_f64(ctx->plan1, early && !side, ctx->d_pj, K1, vec, K1, ctx->d_z, ctx->Ppad, K1, ctx->P, nstate,
+                                        ctx->d_zwork, st);
   }
   if (want_enl) {
-    launch_enl(ctx->d_z, ctx->Ppad, ctx->d_w, ctx->P, nstate, ctx->d_enl, ctx->st);
+    launch_enl(ctx->d_z, ctx->Ppad, ctx->d_w, ctx->P, nstate, ctx->d_enl, st);
     ctx->launches += 2;
   }
   if (!back) return SDFT_OK;
   {
     TScope ts(ctx, 4);
     ctx->launches += launch_gemm_nt_f64(ctx->plan2, early, ctx->d_bk, ctx->Ppad, ctx->d_z, ctx->Ppad, ctx->d_fnl, K1, K2, K1,
-                                        nstate, nullptr, ctx->st);
+                                        nstate, nullptr, st);
   }
+  return SDFT_OK;
+}
+
+// Whether an H application on nstate orbitals runs its nonlocal chain beside
+// the plane stage.  Neither needs the other: the chain's short kernels and the
+// tails of its GEMMs leave SMs idle that the planes' CTAs fill, and it has the
+// more urgent stream, since it is a chain (at equal priority moments and 216 atoms
+// FP64 were no faster than in turn).  In turn -> beside, per filter or call:
+// 64 atoms x 128 orbitals 5.81 -> 5.53 ms, one orbital of 512 atoms (Lanczos)
+// 7.28 -> 7.10, 512 orbitals equal; FP64 moments of 64 atoms 1.84 -> 1.53, 216
+// atoms 7.81 -> 7.18.  The lines, in grid points times orbital pairs: with the
+// digit GEMMs every size from 8.9e5 on gained 4 % or more (5.2e5 lost, the fork
+// and the join cost about 5 us); with the FP64 GEMM the two compete for the FP64
+// pipe and a displaced round of plane CTAs can cost more than it hides (48^3 x 10
+// pairs 53 -> 59 us a step, 72 x 48 x 48 x 28 pairs 167 -> 184), up to 5.3e6,
+// against gains of 7 to 24 % from 6e6 on (96^3 equal).  Not while kernels are
+// timed one by one, and not where other systems fill the SMs: in a graph of
+// several, and in a context whose stream was given a priority, one of several at
+// work.
+constexpr double kForkPoints = 8e5, kForkPointsF64 = 6e6;
+static bool fork_ok(const sdft_ctx *ctx, int nstate) {
+  return ctx->P && ctx->fast && !ctx->timing && !ctx->in_batch && !ctx->shares &&
+         (double)((nstate + 1) / 2) * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
+}
+
+// st goes on when the nonlocal chain is done; stage C then has two kernels to
+// wait for and starts ordinarily.
+static int join_kb(sdft_ctx *ctx) {
+  CK(cudaStreamWaitEvent(ctx->st, ctx->ev_kb, 0));
+  ctx->g.early = false;
   return SDFT_OK;
 }
 
 // One application of the fused H pipeline on `cur` with epilogue `e`.
 static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool want_enl) {
-  int r = run_kb(ctx, cur, nstate, want_enl);
-  if (r) return r;
+  int r;
   const int npairs = (nstate + 1) / 2;
+  if ((r = ensure_x(ctx, npairs))) return r;  // (on st, so before the fork)
+  const bool fork = fork_ok(ctx, nstate);
+  if (fork) {
+    CK(cudaEventRecord(ctx->ev_fork, ctx->st));
+    CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+  }
+  r = run_kb(ctx, cur, nstate, want_enl, true, fork ? ctx->st_kb : nullptr);
+  if (fork) CK(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
+  if (r) {
+    if (fork) cudaStreamWaitEvent(ctx->st, ctx->ev_kb, 0);
+    return r;
+  }
   ctx->g.early = early_ok(ctx, nstate);
-  if ((r = ensure_x(ctx, npairs))) return r;
   e.nstate = nstate;
   e.pair0 = 0;
   e.C = cur;
@@ -441,10 +485,12 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
     if (is_fp64(ctx)) {
       if (!have_x) { TScope ts(ctx, 0); fast_stage_a<double>(ctx->g, cur, nstate, 0, npairs, ctx->d_x, ctx->st); }
       { TScope ts(ctx, 1); fast_stage_b<double>(ctx->g, ctx->d_x, (const double *)ctx->d_vp, npairs, ctx->st); }
+      if (fork && (r = join_kb(ctx))) return r;
       { TScope ts(ctx, 2); fast_stage_c<double>(ctx->g, ctx->d_x, e, npairs, ctx->st); }
     } else {
       if (!have_x) { TScope ts(ctx, 0); fast_stage_a<float>(ctx->g, cur, nstate, 0, npairs, ctx->d_x, ctx->st); }
       { TScope ts(ctx, 1); fast_stage_b<float>(ctx->g, ctx->d_x, (const float *)ctx->d_vp, npairs, ctx->st); }
+      if (fork && (r = join_kb(ctx))) return r;
       { TScope ts(ctx, 2); fast_stage_c<float>(ctx->g, ctx->d_x, e, npairs, ctx->st); }
     }
     if (have_x) nl = 2;
@@ -457,6 +503,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
     { TScope ts(ctx, 1); launch_stage_b<float>(ctx->g, ctx->d_x, (const float *)ctx->d_vp, npairs, ctx->st); }
     { TScope ts(ctx, 2); launch_stage_c<float>(ctx->g, ctx->d_x, e, npairs, ctx->st); }
   }
+  ctx->g.early = early_ok(ctx, nstate);
   ctx->launches += nl;
   CK(cudaGetLastError());
   if (e.omax) {
@@ -668,7 +715,10 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   ctx->npairs_max = (max_states + 1) / 2;
   ctx->vec_elems = (size_t)ctx->s_pad * 2 * ctx->ngp;
   if (cudaSetDevice(device) != cudaSuccess) return fail(set_error(SDFT_ERR_CUDA, "cudaSetDevice failed"));
-  if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&ctx->st_kb, cudaStreamNonBlocking, -1) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->ev_kb, cudaEventDisableTiming) != cudaSuccess)
     return fail(set_error(SDFT_ERR_CUDA, "stream create failed"));
   std::vector<int> cpg, cpc, colab;
   int r = build_columns(ctx, cpg, cpc, colab);
@@ -854,6 +904,9 @@ extern "C" int sdft_ctx_destroy(sdft_ctx *ctx) {
   for (auto &t : ctx->tev_pending) { cudaEventDestroy(t.a); cudaEventDestroy(t.b); }
   for (auto e : ctx->tev_free) cudaEventDestroy(e);
   if (ctx->st) cudaStreamDestroy(ctx->st);
+  if (ctx->st_kb) cudaStreamDestroy(ctx->st_kb);
+  if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+  if (ctx->ev_kb) cudaEventDestroy(ctx->ev_kb);
   delete ctx;
   return SDFT_OK;
 }
@@ -1580,6 +1633,7 @@ static int replace_stream(cudaStream_t *st, int priority) {
 extern "C" int sdft_ctx_set_priority(sdft_ctx *ctx, int priority) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   cudaSetDevice(ctx->device);
+  ctx->shares = true;
   return replace_stream(&ctx->st, priority);
 }
 

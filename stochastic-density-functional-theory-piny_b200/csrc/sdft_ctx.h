@@ -73,6 +73,11 @@ struct sdft_ctx {
   long long dev_bytes = 0;
   long long kb_bytes = 0;  // the part of dev_bytes held by the KB buffers (released by a rebuild)
   double gcut = 0.0;
+  // the nonlocal chain of an H application runs here while the plane stage
+  // runs on st; between the two events of apply_h, so st alone orders the rest
+  cudaStream_t st_kb = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_kb = nullptr;
+  bool shares = false;    // stream priority set: one of several contexts at work
   bool in_batch = false;  // being captured into a graph with other contexts
   bool fast = false;  // compile-time-edge FFT kernels available
   bool fft64 = true;  // FFT scratch / V_KS in FP64 (plain form)

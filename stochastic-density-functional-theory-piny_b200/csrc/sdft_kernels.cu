@@ -751,10 +751,10 @@ void launch_density_reduce(const double *rho_part, int nsplit, int N, double sca
 // 207, 188 us.  8 atoms, 16 orbitals: 32 x 16 2.1 us against 15.5 of 128 x 64;
 // 512 atoms, one orbital: 128 x 8 284 us (6.0 TB/s of projector) against 1650.
 struct GemmShape { int bm, bn; double eff; };
-// the share of that rate reached with one, two, three CTAs on an SM (a CTA's
-// warps wait for their own stages and barriers): with it the projection of 216
-// atoms x 64 orbitals splits K 31 ways, three CTAs an SM, instead of 21, two an
-// SM; the FP64 filter takes 7.85 ms instead of 8.20
+// the share of that rate taken for one, two, three CTAs on an SM (a CTA's warps
+// wait for their own stages and barriers): estimates, judged by the plans they
+// lead to.  216 atoms x 64 orbitals, room for 16 splits: 64 x 32 tiles and 15
+// splits, 7.85 ms a filter; without them 64 x 64 and 10, 8.20
 constexpr double kGemmFill[] = {0.75, 0.9, 1.0};
 constexpr GemmShape kGemmShapes[] = {{64, 64, 1.0}, {64, 32, 0.92}, {32, 16, 0.85},
                                      {128, 16, 0.9}, {128, 8, 0.85}, {32, 8, 0.8}};
