@@ -303,19 +303,43 @@ static bool early_ok(const sdft_ctx *ctx, int nstate) {
   return !ctx->in_batch && (long long)((nstate + 1) / 2) * ctx->n3 <= kEarlyPlanes;
 }
 
-// Nonlocal projection Z = Pj C and back projection FNL = Bk Z for `nstate`
-// orbitals held in `vec`, mixed precision: INT8 Ozaki GEMMs on the digit
-// form of the orbitals; Z = Pj C is split over K with FP64 partial sums, the
-// reduction also produces the digit form of Z for FNL = Bk Z.
-// gk (nullable): project i G_d vec instead of vec, formed inside the digit
-// pass (gk = G_d per coefficient).  max_of (nullable without gk): the row maxima
-// of what is projected.  side (nullable): the stream to run on instead of ctx->st.
-static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
-                     const double *gk = nullptr, const unsigned long long *max_of = nullptr,
-                     cudaStream_t side = nullptr) {
-  const int K1 = 2 * ctx->ngp, S = ctx->s_oz, Ppad = ctx->Ppad;
-  const cudaStream_t st = side ? side : ctx->st;
-  const bool early = early_ok(ctx, nstate), first = early && !side;
+// A digit form of the orbitals that a projection reads: the context's own, or
+// one laid in other scratch (see nl_force_dev).
+struct OzDigits {
+  int8_t *dig;
+  double *sc;
+  const CUtensorMap *t128, *t64;  // its maps with 128- and 64-row boxes
+};
+static OzDigits own_digits(sdft_ctx *ctx) { return {ctx->d_c_dig, ctx->d_c_sc, &ctx->om1.tB, &ctx->om1_tb64}; }
+
+// The digit form of the orbitals in `vec`, or, with gk (G_d per coefficient), of
+// i G_d vec, formed inside the pass.  max_of (nullable without gk): the row maxima
+// of what is projected.
+static void oz_digits(sdft_ctx *ctx, const double *vec, int nstate, const double *gk, const unsigned long long *max_of,
+                      const OzDigits &d, cudaStream_t st, bool early) {
+  const int K1 = 2 * ctx->ngp;
+  const size_t stride = (size_t)ctx->s_oz * ctx->kp_oz;
+  TScope ts(ctx, 7);
+  if (gk) {
+    launch_oz_slice_igc(vec, gk, ctx->ngp, ctx->ncoef, nstate, max_of, d.dig, ctx->kp_oz, stride, d.sc, st);
+  } else {
+    // row maxima: from the stage C that wrote `vec`, else one pass over it
+    if (!max_of && !(ctx->track_omax && ctx->omax_vec == vec && ctx->omax_n == nstate)) {  // (set only when oz)
+      launch_oz_rowmax(vec, K1, nstate, K1, ctx->d_rowmax, st);  // clears the rows first
+      ctx->launches++;
+    }
+    launch_oz_slice(vec, K1, nstate, K1, max_of ? max_of : ctx->d_rowmax, d.dig, ctx->kp_oz, stride, d.sc, st, OZ_7x4,
+                    early);
+  }
+  ctx->launches++;
+}
+
+// Nonlocal projection Z = Pj C and back projection FNL = Bk Z for the `nstate`
+// orbitals of a digit form: INT8 Ozaki GEMMs; Z = Pj C is split over K with FP64
+// partial sums, the reduction also produces the digit form of Z for FNL = Bk Z.
+static int oz_project(sdft_ctx *ctx, int nstate, const OzDigits &d, bool want_enl, bool back, cudaStream_t st) {
+  const int S = ctx->s_oz, Ppad = ctx->Ppad;
+  const bool early = early_ok(ctx, nstate);
   // tile width: the set one, else 64 where it pads the orbitals less; for the
   // projection also where 128-wide tiles with the longest split (32) leave SMs
   // idle (64 atoms, 128 orbitals: 16.4 us at 128, 13.2 at 64; the back projection
@@ -323,30 +347,14 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
   const int bn = ctx->gemm_bn ? ctx->gemm_bn : ((nstate + 63) / 64 * 64 < (nstate + 127) / 128 * 128 ? 64 : 128);
   const int bn1 = ctx->gemm_bn ? bn : (32 * (Ppad / 128) * ((nstate + 127) / 128) < 148 ? 64 : bn);
   const int N = (nstate + bn1 - 1) / bn1 * bn1, N2 = (nstate + bn - 1) / bn * bn;
-  {
-    TScope ts(ctx, 7);
-    if (gk) {
-      launch_oz_slice_igc(vec, gk, ctx->ngp, ctx->ncoef, nstate, max_of, ctx->d_c_dig, ctx->kp_oz,
-                          (size_t)S * ctx->kp_oz, ctx->d_c_sc, st);
-      ctx->launches++;
-    } else {
-      // row maxima: from the stage C that wrote `vec`, else one pass over it
-      if (!max_of && !(ctx->track_omax && ctx->omax_vec == vec && ctx->omax_n == nstate)) {  // (set only when oz)
-        launch_oz_rowmax(vec, K1, nstate, K1, ctx->d_rowmax, st);  // clears the rows first
-        ctx->launches++;
-      }
-      launch_oz_slice(vec, K1, nstate, K1, max_of ? max_of : ctx->d_rowmax, ctx->d_c_dig, ctx->kp_oz, (size_t)S * ctx->kp_oz,
-                      ctx->d_c_sc, st, OZ_7x4, first);
-      ctx->launches++;
-    }
-  }
   OzGemm g1 = ctx->om1, g2 = ctx->om2;
   g1.early = g2.early = early;
   g1.N = N; g1.Nst = nstate;
   g2.N = N2; g2.Nst = nstate;
   g1.bn = bn1;
   g2.bn = bn;
-  if (bn1 == 64) g1.tB = ctx->om1_tb64;
+  g1.tB = bn1 == 64 ? *d.t64 : *d.t128;
+  g1.sb = d.sc;
   if (bn == 64) g2.tB = ctx->om2_tb64;
   const size_t stride = (size_t)N * Ppad;
   const int max_split = (int)std::min<size_t>(32, ctx->oz_part_elems / stride);
@@ -383,10 +391,20 @@ static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl
   return r;
 }
 
+// The two for orbitals held in `vec`, mixed precision.  side (nullable): the
+// stream to run on instead of ctx->st.
+static int run_kb_oz(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
+                     cudaStream_t side = nullptr) {
+  const OzDigits d = own_digits(ctx);
+  const cudaStream_t st = side ? side : ctx->st;
+  oz_digits(ctx, vec, nstate, nullptr, nullptr, d, st, early_ok(ctx, nstate) && !side);
+  return oz_project(ctx, nstate, d, want_enl, back, st);
+}
+
 static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, bool back = true,
                   cudaStream_t side = nullptr) {
   if (ctx->P == 0) return SDFT_OK;
-  if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back, nullptr, nullptr, side);
+  if (ctx->oz) return run_kb_oz(ctx, vec, nstate, want_enl, back, side);
   const int K1 = 2 * ctx->ngp;
   const cudaStream_t st = side ? side : ctx->st;
   const bool early = early_ok(ctx, nstate);
@@ -1489,6 +1507,11 @@ extern "C" int sdft_lanczos_bounds(sdft_ctx *ctx, int nstep, const double *v0re,
   return SDFT_OK;
 }
 
+// Values of c from which the energies and forces run passes beside projections.
+// In turn -> beside: 512 atoms x 256 orbitals, both calls 2.43 -> 2.35 ms; 64 atoms
+// x 512 energies 120 -> 110 us, forces 310 -> 277; x 128 (1.7e6) 81 -> 74, 171 ->
+// 157; 8 atoms x 512 (8e5) 62 -> 64, 110.
+constexpr double kForceBeside = 1e6;
 extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, double occ, int nsto_total,
                                        double *energy_ke, double *energy_pnl) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
@@ -1500,11 +1523,20 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   if (r) return r;
   const double *v = ctx->d_acc + (size_t)imu * ctx->vec_elems;
   double *sc = ctx->d_red + kRedPart;
+  const bool beside = ctx->P && !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside;
+  if (beside) {  // the projection's first pass and the kinetic sum each read c; the sum hides behind the GEMM
+    CK(cudaEventRecord(ctx->ev_fork, ctx->st));
+    CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+    r = run_kb(ctx, v, nstate, true, false, ctx->st_kb);
+    CK(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
+  }
   launch_ekin(v, nstate, ctx->ncoef, ctx->ngp, ctx->d_ak2, ctx->d_red, sc + 2, ctx->st);
   ctx->launches += 2;
   double ek = 0.0, en = 0.0;
   if (ctx->P) {
-    if ((r = run_kb(ctx, v, nstate, true, false))) return r;
+    if (beside) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_kb, 0));
+    else r = run_kb(ctx, v, nstate, true, false);
+    if (r) return r;
     CK(cudaMemcpyAsync(&en, ctx->d_enl, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   }
   CK(cudaMemcpyAsync(&ek, sc + 2, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
@@ -1554,28 +1586,65 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
   do {                                  \
     if ((e = (call)) != cudaSuccess) goto out; \
   } while (0)
-  if (ctx->oz) {  // row maxima of c and of the three i G_d c in one pass over c
+  // projections of c and of the three i G_d c
+  if (ctx->oz) {
+    // the digit passes of the next projection run beside the current one's GEMM
+    // where a second digit set fits the back-projection buffer, which this call
+    // does not otherwise use, and a pass is longer than the events (about 5 us)
+    const OzDigits own = own_digits(ctx);
+    OzDigits d[2] = {own, own};
+    CUtensorMap t2[2];
+    const size_t db = (size_t)kOzSlices * ctx->s_oz * ctx->kp_oz;
+    const bool beside = !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
+                        db + ctx->s_oz * sizeof(double) <= ctx->vec_elems * sizeof(double);
+    if (beside) {
+      int8_t *dig = reinterpret_cast<int8_t *>(ctx->d_fnl);
+      if ((r = make_tmap_oz(&t2[0], dig, ctx->s_oz, ctx->kp_oz)) ||
+          (r = make_tmap_oz(&t2[1], dig, ctx->s_oz, ctx->kp_oz, OZ_7x4, 64)))
+        goto out;
+      d[1] = {dig, reinterpret_cast<double *>(dig + db), &t2[0], &t2[1]};
+    }
     launch_oz_rowmax_igc3(v, ctx->d_gk, ctx->ngp, ctx->ncoef, nstate, ctx->d_rowmax, ctx->d_rowmax3, ctx->st);
     ctx->launches++;
-    if ((r = run_kb_oz(ctx, v, nstate, true, false, nullptr, ctx->d_rowmax))) goto out;
-  } else if ((r = run_kb(ctx, v, nstate, true, false))) {
-    goto out;
-  }
-  CKG(cudaMemcpyAsync(ctx->d_zsave, ctx->d_z, (size_t)nstate * ctx->Ppad * sizeof(double), cudaMemcpyDeviceToDevice,
-                      ctx->st));
-  for (int d = 0; d < 3; d++) {
-    const double *gk = ctx->d_gk + (size_t)d * ctx->ngp;
-    if (ctx->oz) {  // the digit pass forms i G_d c from c itself
-      if ((r = run_kb_oz(ctx, v, nstate, false, false, gk, ctx->d_rowmax3 + (size_t)d * nstate))) goto out;
-    } else {
+    auto digits = [&](int k, cudaStream_t st) {  // k = 0: c, else direction k - 1, formed from c as it is read
+      oz_digits(ctx, v, nstate, k ? ctx->d_gk + (size_t)(k - 1) * ctx->ngp : nullptr,
+                k ? ctx->d_rowmax3 + (size_t)(k - 1) * nstate : ctx->d_rowmax, d[k & 1], st, false);
+    };
+    digits(0, ctx->st);
+    for (int k = 0; k < 4; k++) {
+      if (beside && k < 3) {  // d[(k + 1) & 1] is free: st has the GEMM that read it behind it
+        CKG(cudaEventRecord(ctx->ev_fork, ctx->st));
+        CKG(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+        digits(k + 1, ctx->st_kb);
+        CKG(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
+      } else if (!beside && k) {
+        digits(k, ctx->st);
+      }
+      r = oz_project(ctx, nstate, d[k & 1], k == 0, false, ctx->st);
+      if (beside && k < 3) CKG(cudaStreamWaitEvent(ctx->st, ctx->ev_kb, 0));
+      if (r) goto out;
+      if (k == 0) {
+        CKG(cudaMemcpyAsync(ctx->d_zsave, ctx->d_z, (size_t)nstate * ctx->Ppad * sizeof(double),
+                            cudaMemcpyDeviceToDevice, ctx->st));
+      } else {
+        launch_nl_force_atoms(ctx->d_zsave, ctx->d_z, ctx->Ppad, ctx->d_w, ctx->d_kb_rs, ctx->d_kb_rc, ctx->kb_natm,
+                              nstate, scale, k - 1, d_f, ctx->st);
+        ctx->launches++;
+      }
+    }
+  } else {
+    if ((r = run_kb(ctx, v, nstate, true, false))) goto out;
+    CKG(cudaMemcpyAsync(ctx->d_zsave, ctx->d_z, (size_t)nstate * ctx->Ppad * sizeof(double), cudaMemcpyDeviceToDevice,
+                        ctx->st));
+    for (int k = 0; k < 3; k++) {
       // i G_d c into the back-projection buffer, which this call does not otherwise use
-      launch_dcoef(v, nstate, ctx->ncoef, ctx->ngp, gk, ctx->d_fnl, ctx->st);
+      launch_dcoef(v, nstate, ctx->ncoef, ctx->ngp, ctx->d_gk + (size_t)k * ctx->ngp, ctx->d_fnl, ctx->st);
       ctx->launches++;
       if ((r = run_kb(ctx, ctx->d_fnl, nstate, false, false))) goto out;
+      launch_nl_force_atoms(ctx->d_zsave, ctx->d_z, ctx->Ppad, ctx->d_w, ctx->d_kb_rs, ctx->d_kb_rc, ctx->kb_natm,
+                            nstate, scale, k, d_f, ctx->st);
+      ctx->launches++;
     }
-    launch_nl_force_atoms(ctx->d_zsave, ctx->d_z, ctx->Ppad, ctx->d_w, ctx->d_kb_rs, ctx->d_kb_rc, ctx->kb_natm,
-                          nstate, scale, d, d_f, ctx->st);
-    ctx->launches++;
   }
   // (the direction projections leave d_enl alone: it still holds E_NL of c)
   CKG(cudaMemcpyAsync(h.data(), d_f, h.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));

@@ -1,8 +1,8 @@
 """The nonlocal chain beside the plane stage, from 8e5 grid points times pairs
-on with the digit GEMMs and 6e6 with the FP64 one.  While kernels are timed one
-by one, and once the stream has a priority, they run in turn on one stream: the
-same kernels on the same data, so every result is equal bit for bit, also
-replayed from a graph."""
+on with the digit GEMMs and 6e6 with the FP64 one, and the digit passes and the kinetic sum beside the projections, from 1e6
+values on.  While kernels are timed one by one, and once the stream has a
+priority, they run in turn on one stream: the same kernels on the same data, so
+every result is equal bit for bit, also replayed from a graph."""
 import numpy as np
 import pytest
 
@@ -44,4 +44,28 @@ def test_results_do_not_depend_on_the_streams(pkg, sys2, prec, ns):
         b.sync()
         assert np.array_equal(ctx.download_density(), ref[-1])
     b.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("ns", [60, 96, 330])  # 0.8e6 values of c in turn, 1.3e6 and 4.3e6 beside
+def test_energies_and_forces_do_not_depend_on_the_streams(pkg, sys2, prec, ns):
+    ctx = pkg.Context(*sys2["grid"], sys2["ka"], sys2["kb"], sys2["kc"], sys2["hmat"], precision=prec, max_states=ns)
+    ctx.set_vks(sys2["vks"])
+    ctx.set_kb(sys2["kb_desc"])
+    ctx.noise_dev(ns, seed=5.0)
+    ctx.filter_cheby_dev(ns, np.array([1.0, 0.5, 0.25]), 1, 0.1, 2.0)
+
+    def results():
+        f, e = ctx.nl_force_dev(ns)
+        return [np.array(ctx.energy_chempot_dev(ns)), f, np.array(e)]
+
+    ctx.set_timing(True)
+    ref = results()
+    ctx.read_timing()
+    ctx.set_timing(False)
+    assert np.abs(ref[1]).max() > 0
+    for _ in range(3):
+        for a, b in zip(results(), ref):
+            assert np.array_equal(a, b)
     ctx.close()
