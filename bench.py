@@ -138,24 +138,25 @@ def algorithmic(kind, s, nsto, csz):
 
 
 # DRAM bytes from ncu captures (profiles/): kf_stage_b<float,96,96> and
-# kf_stage_c<float,96,1> per orbital pair (136.5 + 73.2 MB and 294.2 +
-# 301.1 MB for 64 pairs, scaled by pairs); the KB GEMMs
+# kf_stage_c<float,96,8,0> per orbital pair (136.5 + 73.6 MB, and the mean of
+# 509.0 + 303.1 and 401.4 + 196.0 MB with and without the filter sum, for 64
+# pairs, scaled by pairs); the KB GEMMs
 # per launch at 512 orbitals (full-size capture, mean of the projection
 # 1.14 GB + 63.8 MB and the back projection 865.8 + 398.0 MB)
-PROFILED_TRAFFIC = {("kf_stage_b", (96, 96, 96), True): (136.5e6 + 73.2e6) / 64,
-                    ("kf_stage_c", (96, 96, 96), True): (294.2e6 + 301.1e6) / 64}
+PROFILED_TRAFFIC = {("kf_stage_b", (96, 96, 96), True): (136.5e6 + 73.6e6) / 64,
+                    ("kf_stage_c", (96, 96, 96), True): (509.0e6 + 303.1e6 + 401.4e6 + 196.0e6) / 128}
 PROFILED_GEMM_TRAFFIC = {((96, 96, 96), True, 512): (1.14e9 + 63.8e6 + 865.8e6 + 398.0e6) / 2}
 
 # What bounds the HBM-class kernels that sit well below the copy bandwidth,
 # from their ncu captures (profiles/)
 PROFILED_LIMITER = {
-    "kf_stage_b": "shared-memory pipe (l1tex 70.7 % of peak, issue 68 %; ten plane-sized shared passes per plane)",
-    "kf_stage_c": "latency (long-scoreboard and barrier stalls lead; DRAM 35 % on a 64-pair capture)",
+    "kf_stage_b": "shared-memory pipe (l1tex 76.6 % of peak, issue 67 %; ten plane-sized shared passes per plane)",
+    "kf_stage_c": "latency (long-scoreboard stalls lead, then barriers; DRAM 48 to 51 % on a 64-pair capture)",
 }
 
 KERNEL_OF = {"stage_a_pack_cfft": "kf_stage_a", "stage_b_plane_fft_vks": "kf_stage_b",
              "stage_c_cfft_unpack_recur": "kf_stage_c", "kb_proj_gemm": "kb_gemm", "kb_back_gemm": "kb_gemm",
-             "density_planes": "kf_stage_b_density"}
+             "density_planes": "kf_density"}
 
 
 def fp64_gemm_peak(local):

@@ -1,6 +1,6 @@
 """The nonlocal chain beside the plane stage, from 8e5 grid points times pairs
-on with the digit GEMMs and 6e6 with the FP64 one, and the digit passes and the kinetic sum beside the projections, from 1e6
-values on.  While kernels are timed one by one, and once the stream has a
+on with the digit GEMMs and 6e6 with the FP64 one, and the digit passes and the
+kinetic sum beside the projections, from 1e6 values on.  While kernels are timed one by one, and once the stream has a
 priority, they run in turn on one stream: the same kernels on the same data, so
 every result is equal bit for bit, also replayed from a graph."""
 import numpy as np
