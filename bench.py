@@ -139,19 +139,19 @@ def algorithmic(kind, s, nsto, csz):
 
 # DRAM bytes from ncu captures (profiles/): kf_stage_b<float,96,96> and
 # kf_stage_c<float,96,8,0> per orbital pair (136.5 + 73.6 MB, and the mean of
-# 509.0 + 303.1 and 401.4 + 196.0 MB with and without the filter sum, for 64
+# 509.1 + 303.9 and 401.9 + 203.6 MB with and without the filter sum, for 64
 # pairs, scaled by pairs); the KB GEMMs
 # per launch at 512 orbitals (full-size capture, mean of the projection
 # 1.14 GB + 63.8 MB and the back projection 865.8 + 398.0 MB)
 PROFILED_TRAFFIC = {("kf_stage_b", (96, 96, 96), True): (136.5e6 + 73.6e6) / 64,
-                    ("kf_stage_c", (96, 96, 96), True): (509.0e6 + 303.1e6 + 401.4e6 + 196.0e6) / 128}
+                    ("kf_stage_c", (96, 96, 96), True): (509.1e6 + 303.9e6 + 401.9e6 + 203.6e6) / 128}
 PROFILED_GEMM_TRAFFIC = {((96, 96, 96), True, 512): (1.14e9 + 63.8e6 + 865.8e6 + 398.0e6) / 2}
 
 # What bounds the HBM-class kernels that sit well below the copy bandwidth,
 # from their ncu captures (profiles/)
 PROFILED_LIMITER = {
     "kf_stage_b": "shared-memory pipe (l1tex 76.6 % of peak, issue 67 %; ten plane-sized shared passes per plane)",
-    "kf_stage_c": "latency (long-scoreboard stalls lead, then barriers; DRAM 48 to 51 % on a 64-pair capture)",
+    "kf_stage_c": "latency (long-scoreboard stalls lead, then barriers; DRAM 54 to 60 % on a 64-pair capture)",
 }
 
 KERNEL_OF = {"stage_a_pack_cfft": "kf_stage_a", "stage_b_plane_fft_vks": "kf_stage_b",

@@ -447,7 +447,7 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
 // and the join cost about 5 us); with the FP64 GEMM the two compete for the FP64
 // pipe and a displaced round of plane CTAs can cost more than it hides (48^3 x 10
 // pairs 53 -> 59 us a step, 72 x 48 x 48 x 28 pairs 167 -> 184), up to 5.3e6,
-// against gains of 7 to 24 % from 6e6 on (96^3 equal).  Not while kernels are
+// against gains of 1 to 24 % from 6e6 on (cells of 8 to 512 atoms).  Not while kernels are
 // timed one by one, and not where other systems fill the SMs: in a graph of
 // several, and in a context whose stream was given a priority, one of several at
 // work.
