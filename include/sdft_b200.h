@@ -404,6 +404,15 @@ int sdft_ctx_set_gemm_bn(sdft_ctx *ctx, int bn);
  * accepted by mixed-precision contexts on the fast FFT path only; chosen
  * per system by the autotuner (tuner.py).  No counterpart in the reference. */
 int sdft_ctx_set_plane_threads(sdft_ctx *ctx, int nt);
+/* Which of its alternative routes a context takes, for the autotuner's cache
+ * keys and for tests (-1: null context or unknown `what`).  No counterpart in
+ * the reference. */
+enum {
+  SDFT_INFO_DIGIT_GEMMS = 0,  /* 1: the projections are INT8 digit GEMMs, 0: FP64 */
+  SDFT_INFO_COLUMN_PAIRS = 1, /* column pairs per CTA of the column stages */
+  SDFT_INFO_SIDE_RUNS = 2     /* times work was queued on the second stream (H applications, energies, forces) */
+};
+long long sdft_ctx_info(const sdft_ctx *ctx, int what);
 /* CUDA stream priority of the context's stream (lower = more urgent, 0 =
  * default; clamped to the device's range).  Call while the context is idle:
  * the stream is replaced.  A server gives cheap requests the urgent

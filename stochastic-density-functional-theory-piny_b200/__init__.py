@@ -134,6 +134,7 @@ _sig("sdft_event_synchronize", C.c_int, [_vp])
 _sig("sdft_event_elapsed_ms", C.c_int, [_vp, _vp, C.POINTER(C.c_float)])
 _sig("sdft_event_destroy", C.c_int, [_vp])
 _sig("sdft_launch_count", C.c_longlong, [_vp])
+_sig("sdft_ctx_info", C.c_longlong, [_vp, C.c_int])
 _sig("sdft_ctx_set_timing", C.c_int, [_vp, C.c_int])
 _sig("sdft_ctx_read_timing", C.c_int, [_vp, _dp, C.POINTER(C.c_longlong)])
 _sig("sdft_ctx_set_gemm_split", C.c_int, [_vp, C.c_int])
@@ -420,6 +421,21 @@ class Context:
     @property
     def launches(self):
         return int(lib.sdft_launch_count(self._p))
+
+    @property
+    def digit_gemms(self):
+        """Whether the projections run as INT8 digit GEMMs (mixed precision, enough projection work)."""
+        return bool(lib.sdft_ctx_info(self._p, 0))
+
+    @property
+    def column_pairs(self):
+        """Column pairs per CTA of the column stages."""
+        return int(lib.sdft_ctx_info(self._p, 1))
+
+    @property
+    def side_runs(self):
+        """Times the context queued work on its second stream."""
+        return int(lib.sdft_ctx_info(self._p, 2))
 
     def sync(self):
         _chk(lib.sdft_sync(self._p))

@@ -474,6 +474,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   if (fork) {
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+    ctx->side_runs++;
   }
   r = run_kb(ctx, cur, nstate, want_enl, true, fork ? ctx->st_kb : nullptr);
   if (fork) CK(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
@@ -962,6 +963,15 @@ extern "C" int sdft_ctx_set_vks(sdft_ctx *ctx, const double *v) {
 extern "C" long long sdft_ctx_device_bytes(const sdft_ctx *ctx) { return ctx ? ctx->dev_bytes : 0; }
 extern "C" void *sdft_ctx_stream(sdft_ctx *ctx) { return ctx ? (void *)ctx->st : nullptr; }
 extern "C" long long sdft_launch_count(const sdft_ctx *ctx) { return ctx ? ctx->launches : 0; }
+extern "C" long long sdft_ctx_info(const sdft_ctx *ctx, int what) {
+  if (!ctx) return -1;
+  switch (what) {
+    case SDFT_INFO_DIGIT_GEMMS: return ctx->oz;
+    case SDFT_INFO_COLUMN_PAIRS: return ctx->g.cpb;
+    case SDFT_INFO_SIDE_RUNS: return ctx->side_runs;
+    default: return -1;
+  }
+}
 extern "C" int sdft_ctx_set_timing(sdft_ctx *ctx, int enable) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   ctx->timing = enable != 0;
@@ -1527,6 +1537,7 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   if (beside) {  // the projection's first pass and the kinetic sum each read c; the sum hides behind the GEMM
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+    ctx->side_runs++;
     r = run_kb(ctx, v, nstate, true, false, ctx->st_kb);
     CK(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
   }
@@ -1615,6 +1626,7 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
       if (beside && k < 3) {  // d[(k + 1) & 1] is free: st has the GEMM that read it behind it
         CKG(cudaEventRecord(ctx->ev_fork, ctx->st));
         CKG(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
+        ctx->side_runs++;
         digits(k + 1, ctx->st_kb);
         CKG(cudaEventRecord(ctx->ev_kb, ctx->st_kb));
       } else if (!beside && k) {

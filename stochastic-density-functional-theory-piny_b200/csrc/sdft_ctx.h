@@ -77,6 +77,7 @@ struct sdft_ctx {
   // runs on st; between the two events of apply_h, so st alone orders the rest
   cudaStream_t st_kb = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_kb = nullptr;
+  long long side_runs = 0;  // times work was queued on st_kb
   bool shares = false;    // stream priority set: one of several contexts at work
   bool in_batch = false;  // being captured into a graph with other contexts
   bool fast = false;  // compile-time-edge FFT kernels available
