@@ -27,8 +27,10 @@ def _system(wl, grid, reps, holes, ecut=10.0):
     return s
 
 
-def _results(pkg, s, prec, ns):
-    ctx = pkg.Context(*s["grid"], s["ka"], s["kb"], s["kc"], s["hmat"], precision=prec, max_states=ns)
+def _results(pkg, s, prec, ns, nmax=None, pairs=8):
+    """Results of ns orbitals in a context for nmax, whose column stages take `pairs` column pairs a CTA."""
+    ctx = pkg.Context(*s["grid"], s["ka"], s["kb"], s["kc"], s["hmat"], precision=prec, max_states=nmax or ns)
+    assert ctx.column_pairs == pairs
     ctx.set_vks(s["vks"])
     ctx.set_kb(s["kb_desc"])
     out = {}
@@ -49,7 +51,8 @@ def _results(pkg, s, prec, ns):
 
 
 # every edge with a compile-time plan on every axis, the plane pairs with stage-B
-# instances of their own, and spheres narrower and wider than 3/8 of the planes
+# instances of their own, and spheres narrower and wider than 3/8 of the planes;
+# the few orbitals make every context take the column stages of 8 pairs a CTA
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("grid,reps,ns,holes", [
     ((12, 12, 12), 1, 3, False), ((24, 24, 32), 1, 3, False), ((32, 32, 24), 1, 5, True),
@@ -64,6 +67,22 @@ def _results(pkg, s, prec, ns):
 def test_compile_time_edges_match_run_time_sizes(pkg, wl, monkeypatch, prec, grid, reps, ns, holes):
     s = _system(wl, grid, reps, holes, ECUT.get(grid, 10.0))
     fast = _results(pkg, s, prec, ns)
+    monkeypatch.setenv("SDFT_GENERIC_FFT", "1")
+    slow = _results(pkg, s, prec, ns)
+    for k, v in slow.items():
+        assert rel_l2(fast[k], v) < (1e-12 if prec == 0 or k in ("noise", "density") else 5e-6), k
+
+
+# the column stages of contexts with many orbitals: 32 column pairs a CTA below
+# edge 36, 16 below 72 (43 and 87 column pairs here: the last CTA is partly empty)
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("grid,reps,ns,holes", [
+    ((12, 12, 12), 1, 3, False), ((24, 24, 16), 1, 2, False), ((24, 24, 18), 1, 3, True), ((24, 24, 24), 1, 4, False),
+    ((24, 24, 27), 1, 3, False), ((24, 24, 32), 1, 5, True), ((24, 24, 36), 1, 3, False),
+    ((24, 24, 48), (1, 1, 2), 2, False), ((24, 24, 54), (1, 1, 2), 3, True), ((24, 24, 64), (1, 1, 2), 3, False)])
+def test_columns_of_contexts_with_many_orbitals(pkg, wl, monkeypatch, prec, grid, reps, ns, holes):
+    s = _system(wl, grid, reps, holes, ECUT.get(grid, 10.0))
+    fast = _results(pkg, s, prec, ns, 1024, 32 if grid[2] < 36 else 16)
     monkeypatch.setenv("SDFT_GENERIC_FFT", "1")
     slow = _results(pkg, s, prec, ns)
     for k, v in slow.items():
