@@ -55,6 +55,26 @@ def test_fp64_tiles_of_a_larger_cell(pkg, wl):
     ctx.close()
 
 
+def test_fp64_split_of_more_orbitals_than_a_grid_dimension(pkg, wl):
+    """A split projection of 65544 orbitals: the reduction's grid holds 65535 of
+    them.  Eight orbitals repeated: every copy's force is the first one's, bit for
+    bit (the same sums at another place), and equal to a context for eight."""
+    s = wl.make_system(1, (12, 12, 12), ecut=5.0)
+    nc, rep = s["ncoef"], 8193
+    cr, ci = _orbitals(nc, 8)
+    small = _ctx(pkg, s, pkg.SDFT_PREC_FP64, 8)
+    ref = small.calc_coef_force(cr, ci)
+    small.close()
+    ctx = _ctx(pkg, s, pkg.SDFT_PREC_FP64, 8 * rep)
+    ctx.set_gemm_split(3)
+    got = ctx.calc_coef_force(np.tile(cr, rep), np.tile(ci, rep))
+    ctx.close()
+    for g, r in zip(got, ref):
+        g = g.reshape(rep, 8 * nc)
+        assert rel_l2(g[0], r) < 1e-12
+        assert np.array_equal(g, np.broadcast_to(g[0], g.shape))
+
+
 @pytest.mark.parametrize("nmax", [4, 1800])  # P K max_states = 2e5 and 9.6e7: DMMA and digit GEMMs
 def test_mixed_on_both_sides_of_the_digit_limit(pkg, sys1, nmax):
     cr, ci = _orbitals(sys1["ncoef"], 4)
