@@ -1675,8 +1675,8 @@ out:
 extern "C" int sdft_ctx_set_plane_threads(sdft_ctx *ctx, int nt) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   if (nt != 0 && nt != 128 && nt != 256) return set_error(SDFT_ERR_ARG, "plane_threads: 0 (default), 128 or 256");
-  if (nt == 128 && (is_fp64(ctx) || !ctx->fast || !plane_size_settable(ctx->n1, ctx->n2, ctx->n3)))
-    return set_error(SDFT_ERR_UNSUPPORTED, "plane_threads: 128 exists for the FP32 fast plane stage only");
+  if (nt == 128 && (is_fp64(ctx) || !ctx->fast))
+    return set_error(SDFT_ERR_UNSUPPORTED, "plane_threads: 128 exists for the FP32 compile-time-edge plane stage only");
   ctx->g.plane_nt = nt == 0 ? default_plane_threads(ctx) : nt;
   return SDFT_OK;
 }

@@ -6,9 +6,6 @@
 
 namespace sdft {
 bool fast_supported(int n1, int n2, int n3);
-// grids of edges 24, 48, 72, 96 whose plane has an instance of its own: those
-// whose FP32 plane CTA size can be set
-bool plane_size_settable(int n1, int n2, int n3);
 // column stages of edge N3 (sdft_cols.cuh, instantiated in sdft_cols_*.cu)
 template <typename T, int N3>
 void cols_launch_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st);

@@ -195,11 +195,6 @@ __global__ void kf_vks_perm(const double *__restrict__ v, T *__restrict__ Vp, in
 // ---------------------------------------------------------------------------
 bool fast_supported(int n1, int n2, int n3) { return plan_rt(n1).r1 && plan_rt(n2).r1 && plan_rt(n3).r1; }
 
-bool plane_size_settable(int n1, int n2, int n3) {
-  auto small = [](int n) { return n == 24 || n == 48 || n == 72; };
-  return (small(n3) || n3 == 96) && ((small(n1) && small(n2)) || (n1 == 96 && n2 == 96));
-}
-
 template <typename T>
 void fast_stage_a(const DevGeom &g, const double *C, int nstate, int pair0, int npairs, void *X, cudaStream_t st) {
   switch (g.n3) {

@@ -87,3 +87,20 @@ def test_columns_of_contexts_with_many_orbitals(pkg, wl, monkeypatch, prec, grid
     slow = _results(pkg, s, prec, ns)
     for k, v in slow.items():
         assert rel_l2(fast[k], v) < (1e-12 if prec == 0 or k in ("noise", "density") else 5e-6), k
+
+
+# planes with an instance of their own and without one, most with 128 threads as
+# the default: either CTA size can be set, and set back
+@pytest.mark.parametrize("grid,reps", [((64, 64, 24), (2, 2, 1)), ((54, 64, 24), (2, 2, 1)), ((32, 32, 32), 1),
+                                       ((32, 96, 24), (1, 3, 1)), ((108, 81, 32), (3, 2, 1))])
+def test_plane_cta_sizes_give_the_same_result(pkg, wl, grid, reps):
+    s = _system(wl, grid, reps, False)
+    ctx = pkg.Context(*s["grid"], s["ka"], s["kb"], s["kc"], s["hmat"], precision=pkg.SDFT_PREC_MIXED, max_states=3)
+    ctx.set_vks(s["vks"])
+    ctx.set_kb(s["kb_desc"])
+    cr, ci = ctx.genNoiseOrbitalReal(3, seed=5.0)
+    ref = ctx.calc_coef_force(cr, ci)
+    for nt in (256, 128, 0):
+        ctx.set_plane_threads(nt)
+        assert all(np.array_equal(a, b) for a, b in zip(ctx.calc_coef_force(cr, ci), ref)), nt
+    ctx.close()
