@@ -1,7 +1,8 @@
 """Autotuner for the per-system launch shapes of the filter.
 
 Three shapes are tuned per problem shape:
-* the orbital columns per tile of the mixed-precision KB GEMMs, 128 or 64:
+* the orbital columns per tile of the INT8 digit KB GEMMs, 128 or 64 (the FP64
+  GEMM, which small mixed contexts take too, picks its tile per call):
   the orbital count is padded to the tile width, so 64 wastes less on small
   or just-over-128 counts, while 128 reads each projector tile fewer times
   (timed first, at the cost model's split);
@@ -18,8 +19,10 @@ context's resident orbitals: the filter kernels themselves, device time by
 CUDA events on the context stream, through the library's own event calls.
 The library's own choice (0) is a candidate in each list, and another is set
 only when it is more than 2 % faster, so timing noise cannot pick a slower
-shape.  Results are cached per problem shape (grid, projectors, orbital
-tiles of 64, precision), in memory and optionally in a JSON file.
+shape.  Results are cached per problem shape (grid, coefficients to a ninth of
+an octave, projectors, orbital tiles of 64, precision and the form of the
+projection GEMM with what sizes its workspace), in memory and optionally in a
+JSON file.
 
 Tuning overwrites the context's filter accumulators: run it before the real
 filter.
@@ -27,6 +30,7 @@ filter.
 from __future__ import annotations
 
 import json
+import math
 import os
 
 import numpy as np
@@ -62,9 +66,13 @@ class Tuner:
 
     @staticmethod
     def key(ctx, nstate, nproj):
-        # the GEMM tile grid depends on the projector count and the orbitals
-        # in 64-wide tiles; K (2 ncoef) follows from the grid
-        return f"{ctx.n[0]}x{ctx.n[1]}x{ctx.n[2]}/P{nproj}/N{(nstate + 63) // 64}/prec{ctx.precision}"
+        # the GEMM tile grid depends on the projector count and the orbitals in
+        # 64-wide tiles, its K on the coefficients (binned, so that strained
+        # cells share an entry).  Which GEMM a mixed context takes depends on the
+        # orbitals it is made for, and so does the room for the FP64 GEMM's splits
+        form = "digits" if ctx.digit_gemms else f"fp64w{(ctx.max_states + 63) // 64}"
+        return (f"{ctx.n[0]}x{ctx.n[1]}x{ctx.n[2]}/K{round(9 * math.log2(ctx.ncoef))}/P{nproj}"
+                f"/N{(nstate + 63) // 64}/prec{ctx.precision}/{form}")
 
     def _time(self, ctx, nstate, split, scale, emean, reps=2):
         """Device time of a short filter under split-K `split`: the best of
@@ -92,7 +100,7 @@ class Tuner:
         k = self.key(ctx, nstate, nproj)
         if k not in self.cache:
             bn = {}
-            if ctx.precision != self.pkg.SDFT_PREC_FP64:  # the FP64 GEMM has one tile shape
+            if ctx.digit_gemms:
                 for w in GEMM_BN:
                     ctx.set_gemm_bn(w)
                     bn[str(w)] = self._time(ctx, nstate, 0, scale, emean)

@@ -83,3 +83,52 @@ def test_serving_and_tuning_need_no_torch(pkg, mod):
         elif isinstance(node, ast.ImportFrom) and node.module:
             names.add(node.module.split(".")[0])
     assert "torch" not in names
+
+
+class _Ctx:
+    """What the autotuner's cache key reads of a context, and the calls it makes."""
+    n, precision = (48, 48, 48), 1
+
+    def __init__(self, ncoef, max_states, digits):
+        self.ncoef, self.max_states, self.digit_gemms, self.calls = ncoef, max_states, digits, []
+
+    def set_gemm_bn(self, bn):
+        self.calls.append(("bn", bn))
+
+    def set_gemm_split(self, split):
+        self.calls.append(("split", split))
+
+    def set_plane_threads(self, nt):
+        self.calls.append(("plane", nt))
+
+
+def _tuner(pkg, path=None):
+    mod = importlib.import_module(pkg.__name__ + ".tuner")
+    t = mod.Tuner(pkg, path)
+    t._time = lambda ctx, nstate, split, scale, emean: 1.0 if split in (0, 8) else 2.0
+    return t
+
+
+def test_tuned_shapes_are_kept_per_projection_gemm(pkg, tmp_path):
+    """A split tuned on the digit GEMMs is not set on a context of the same grid
+    and orbital tiles that projects with the FP64 GEMM, or the other way round;
+    a file written before the key told them apart has no entry that matches."""
+    import json
+    digits, fp64 = _Ctx(6500, 40, True), _Ctx(6500, 20, False)
+    t = _tuner(pkg)
+    assert t.key(digits, 20, 256) != t.key(fp64, 20, 256)
+    assert t.key(fp64, 20, 256) != t.key(_Ctx(6500, 200, False), 20, 256)  # more room for splits
+    assert t.key(fp64, 20, 256) != t.key(_Ctx(13000, 20, False), 20, 256)  # twice the cutoff's K
+    assert t.key(digits, 20, 256) == t.key(_Ctx(6500, 400, True), 20, 256)
+    path = tmp_path / "shapes.json"
+    path.write_text(json.dumps({"48x48x48/P256/N1/prec1": {"split": 32, "gemm_bn": 64}}))
+    assert _tuner(pkg, str(path)).tune(fp64, 20, 256) == 0
+
+
+def test_tile_widths_are_timed_for_digit_gemms_only(pkg):
+    for digits in (True, False):
+        ctx = _Ctx(6500, 40, digits)
+        t = _tuner(pkg)
+        t.tune(ctx, 40, 256)
+        assert any(c[0] == "bn" for c in ctx.calls) == digits
+        assert ("gemm_bn" in t.cache[t.key(ctx, 40, 256)]) == digits
