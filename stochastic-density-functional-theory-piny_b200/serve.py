@@ -88,26 +88,51 @@ def estimate_spec_bytes(spec, nsto, ecut=10.0, a0=10.26):
     return int(1.15 * _bytes(spec["grid"], ncoef, cols, natm, nsto))
 
 
-def _bytes(grid, ncoef, cols, natm, nsto):
+_PLAN_EDGES = (12, 16, 18, 24, 27, 32, 36, 48, 54, 64, 72, 81, 96, 108, 128)
+
+
+def _density_grids(grid, npairs):
+    """Partial density grids of a context: one per pair group, as
+    fast_density_max_groups (csrc/sdft_planes.cu) bounds them, or one per pair on
+    edges without a compile-time plan."""
     n1, n2, n3 = grid
-    spad = (nsto + 127) // 128 * 128
-    vec = spad * 2 * ncoef * 8
-    npairs = (nsto + 1) // 2
-    P = 4 * natm
-    ppad = (P + 127) // 128 * 128
-    kp = (2 * ncoef + 63) // 64 * 64
-    mpad = (2 * ncoef + 127) // 128 * 128
-    # projector bytes per value: four digits, or FP64 where the projections are
-    # small (csrc/sdft_kb.cu kOzMinWork, 9e7; with room for padding)
-    pv = 8 if P * kp * nsto < 1.0e8 else 4
-    return int(5 * vec + npairs * n3 * cols * 8 + npairs * n1 * n2 * n3 * 8 + pv * (ppad * kp + mpad * ppad)
-               + 4 * spad * (kp + ppad) + 32 * spad * ppad * 8 + 64 * 2 ** 20)
+    if not all(n in _PLAN_EDGES for n in grid):
+        return npairs
+    plane = 16 * ((n1 + 1) // 2 + n1 * (n2 | 1))
+    slots = 148 * (2 if 2 * (plane + 1024) <= 228 * 1024 else 1)
+    return min(npairs, -(-3 * slots // n3))
+
+
+def _bytes(grid, ncoef, cols, natm, nsto):
+    def up(a, b):
+        return (a + b - 1) // b * b
+
+    n1, n2, n3 = grid
+    N, npairs, P, K = n1 * n2 * n3, (nsto + 1) // 2, 4 * natm, 2 * up(ncoef, 16)
+    s64, s128, ppad, kp, mpad = up(nsto, 64), up(nsto, 128), up(P, 128), up(K, 64), up(K, 128)
+    vec = s64 * K * 8
+    after = vec + max(npairs, 2) * n3 * up(cols, 4) * 8 + npairs * (cols // 16 + 1) * 24
+    after += _density_grids(grid, npairs) * N * 8 + N * 8 + nsto * N  # the last: noise signs
+    f64 = 8 * (ppad * K + mpad * ppad)
+    digits = 4 * (ppad * kp + mpad * ppad) + 4 * s128 * (kp + ppad) + 32 * s128 * ppad * 8
+    # digit or FP64 projectors (kOzMinWork in csrc/sdft_kb.cu, 9e7); the larger where
+    # a coefficient count that is itself an estimate leaves it open
+    proj = digits if P * K * nsto >= 8e7 else 0
+    if P * K * nsto < 1.1e8:
+        proj = max(proj, f64)
+    # the digit form is made from the FP64 one: both at once, before the buffers of
+    # the filter (accumulators, columns, density) exist
+    building = f64 + digits if P * K * nsto >= 8e7 else f64
+    # throughout: three orbital blocks and the nonlocal force, V_KS, Z and the FP64
+    # split partials (17 times Z; those past 16 splits are below 32 MB)
+    held = 4 * vec + N * 12 + 17 * s64 * ppad * 8
+    return int(held + max(after + proj, building) + 64 * 2 ** 20)
 
 
 def estimate_bytes(s, nsto):
     """Device footprint of one request's context (mixed precision), from the
-    sizes the library allocates: orbital blocks, FFT column scratch, density
-    partials, KB digit arrays and split-K partials."""
+    sizes the library allocates: orbital blocks, FFT column scratch, noise signs,
+    density group grids, projectors (digits or FP64) and split-K partials."""
     cols = len(set(zip(s["ka"][:-1].tolist(), s["kb"][:-1].tolist()))) * 2 + 1
     return _bytes(s["grid"], s["ncoef"], cols, s["natm"], nsto)
 

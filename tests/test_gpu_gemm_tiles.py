@@ -88,13 +88,35 @@ def test_mixed_on_both_sides_of_the_digit_limit(pkg, sys1, nmax):
 
 
 @pytest.mark.parametrize("cells,grid,ns", [((2, 2, 2), (48, 48, 48), 2), ((3, 3, 3), (72, 72, 72), 2),
-                                           ((3, 3, 3), (72, 72, 72), 4)])  # FP64, FP64 and digit projectors
+                                           ((3, 3, 3), (72, 72, 72), 4),  # FP64, FP64 and digit projectors
+                                           ((2, 2, 2), (48, 48, 48), 256), ((3, 2, 1), (72, 48, 24), 96),
+                                           ((4, 4, 4), (96, 96, 96), 512)])
 def test_estimate_covers_either_form(pkg, wl, cells, grid, ns):
+    """The admission estimate of a request covers all it allocates from the context
+    to the density, set-up included, by no more than a tenth beside its fixed
+    64 MB: under a limit of the estimate the calls succeed, under 0.9 of the rest
+    one of them is refused its memory."""
     serve = __import__(pkg.__name__ + ".serve", fromlist=["estimate_bytes"])
     s = wl.make_system(cells, grid)
-    ctx = _ctx(pkg, s, pkg.SDFT_PREC_MIXED, ns)
-    ctx.noise_dev(ns)
-    ctx.filter_cheby_dev(ns, np.ones(3), 1, 0.1, 2.0)
-    ctx.density_dev(ns, want=False)
-    assert ctx.device_bytes <= serve.estimate_bytes(s, ns)
-    ctx.close()
+    est = serve.estimate_bytes(s, ns)
+
+    def request(limit):
+        pkg.set_device_memory_limit(0, pkg.device_memory_in_use(0) + int(limit))
+        ctx = None
+        try:
+            ctx = _ctx(pkg, s, pkg.SDFT_PREC_MIXED, ns)
+            ctx.lanczos_bounds(3)
+            ctx.noise_dev(ns)
+            ctx.moments_dev(ns, 4, 0.1, 2.0)
+            ctx.filter_cheby_dev(ns, np.ones(3), 1, 0.1, 2.0)
+            ctx.density_dev(ns, want=False)
+            return ctx.device_bytes
+        finally:
+            pkg.set_device_memory_limit(0, 0)
+            if ctx:
+                ctx.close()
+
+    assert request(est) <= est
+    with pytest.raises(pkg.SdftError) as e:
+        request(0.9 * (est - 64 * 2 ** 20))
+    assert e.value.code == 3  # SDFT_ERR_NOMEM
