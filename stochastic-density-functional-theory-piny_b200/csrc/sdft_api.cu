@@ -457,6 +457,18 @@ static bool fork_ok(const sdft_ctx *ctx, int nstate) {
          (double)((nstate + 1) / 2) * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
 }
 
+// The second stream and its events, made when a call first wants them: a stream
+// takes 50 us to make and 50 to destroy (creating a context of 8 to 96 atoms, mean
+// of six: 0.345 ms with it, 0.287 without), and contexts of small systems, of graphs
+// of several and with a priority never use it.  Not while a stream is captured.
+static int ensure_side(sdft_ctx *ctx) {
+  if (ctx->st_kb) return SDFT_OK;
+  if (!ctx->ev_fork) CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+  if (!ctx->ev_kb) CK(cudaEventCreateWithFlags(&ctx->ev_kb, cudaEventDisableTiming));
+  CK(cudaStreamCreateWithPriority(&ctx->st_kb, cudaStreamNonBlocking, -1));
+  return SDFT_OK;
+}
+
 // st goes on when the nonlocal chain is done; stage C then has two kernels to
 // wait for and starts ordinarily.
 static int join_kb(sdft_ctx *ctx) {
@@ -472,6 +484,7 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   if ((r = ensure_x(ctx, npairs))) return r;  // (on st, so before the fork)
   const bool fork = fork_ok(ctx, nstate);
   if (fork) {
+    if ((r = ensure_side(ctx))) return r;
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
     ctx->side_runs++;
@@ -734,10 +747,7 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   ctx->npairs_max = (max_states + 1) / 2;
   ctx->vec_elems = (size_t)ctx->s_pad * 2 * ctx->ngp;
   if (cudaSetDevice(device) != cudaSuccess) return fail(set_error(SDFT_ERR_CUDA, "cudaSetDevice failed"));
-  if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithPriority(&ctx->st_kb, cudaStreamNonBlocking, -1) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_kb, cudaEventDisableTiming) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess)
     return fail(set_error(SDFT_ERR_CUDA, "stream create failed"));
   std::vector<int> cpg, cpc, colab;
   int r = build_columns(ctx, cpg, cpc, colab);
@@ -754,8 +764,6 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
     const char *ev = getenv("SDFT_GENERIC_FFT");  // force the runtime-size kernels (testing)
     ctx->fast = fast_supported(n1, n2, n3) && !(ev && ev[0] == '1');
   }
-  std::vector<int> gkc(ncoef);
-  for (int i = 0; i < ncoef; i++) gkc[i] = kc[i];
   std::vector<double> ak2(ncoef);
   sdft_ak2_kinetic(hmat, ncoef, ka, kb, kc, 0.0, ak2.data());
   std::vector<double2> tw(n1 + n2 + n3);
@@ -771,20 +779,6 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   }
 #define DMF(ptr, bytes) do { int r__ = dmalloc(ctx, (void **)&(ptr), (bytes)); if (r__) return fail(r__); } while (0)
 #define CKF(call) do { cudaError_t e__ = (call); if (e__ != cudaSuccess) return fail(set_error(SDFT_ERR_CUDA, cudaGetErrorString(e__))); } while (0)
-  DMF(ctx->d_cp_gstart, cpg.size() * sizeof(int));
-  DMF(ctx->d_cp_gcount, cpc.size() * sizeof(int));
-  DMF(ctx->d_col_ab, colab.size() * sizeof(int));
-  DMF(ctx->d_gkc, ncoef * sizeof(int));
-  DMF(ctx->d_ak2, ncoef * sizeof(double));
-  DMF(ctx->d_tw, tw.size() * sizeof(double2));
-  DMF(ctx->d_twf, twf.size() * sizeof(float2));
-  CKF(cudaMemcpyAsync(ctx->d_cp_gstart, cpg.data(), cpg.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_cp_gcount, cpc.data(), cpc.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_col_ab, colab.data(), colab.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_gkc, gkc.data(), ncoef * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_ak2, ak2.data(), ncoef * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
-  CKF(cudaMemcpyAsync(ctx->d_twf, twf.data(), twf.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->st));
   DevGeom &g = ctx->g;
   g.n1 = n1; g.n2 = n2; g.n3 = n3; g.N = ctx->N;
   g.plane_nt = default_plane_threads(ctx);
@@ -806,14 +800,11 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
   }
   g.cpb = cpb;
   g.nbatch = (g.ncp + cpb - 1) / cpb;
-  g.cp_gstart = ctx->d_cp_gstart; g.cp_gcount = ctx->d_cp_gcount; g.col_ab = ctx->d_col_ab;
-  g.gkc = ctx->d_gkc; g.ak2 = ctx->d_ak2;
-  g.tw1 = ctx->d_tw; g.tw2 = ctx->d_tw + n1; g.tw3 = ctx->d_tw + n1 + n2;
-  g.tw1f = ctx->d_twf; g.tw2f = ctx->d_twf + n1; g.tw3f = ctx->d_twf + n1 + n2;
   // signed kb range of the sphere columns on each plane row a (a = ka mod n1),
   // and whether every row's columns fill their range
+  std::vector<int2> kb_rng(n1, make_int2(1, 0));
   {
-    std::vector<int2> rng(n1, make_int2(1, 0));
+    std::vector<int2> &rng = kb_rng;
     std::vector<int> cnt(n1, 0);
     for (int ab : colab) {
       const int a = ab >> 16, b = ab & 0xffff;
@@ -828,16 +819,15 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
       if (cnt[a]) g.kbmax = std::max(g.kbmax, std::max(std::abs(rng[a].x), std::abs(rng[a].y)));
     }
     g.prune34 = (8 * g.kamax < 3 * n1 && 8 * g.kbmax < 3 * n2) ? (4 * g.kamax >= n1 ? 2 : 1) : 0;
-    DMF(ctx->d_kb_rng, n1 * sizeof(int2));
-    CKF(cudaMemcpyAsync(ctx->d_kb_rng, rng.data(), n1 * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
-    CKF(cudaStreamSynchronize(ctx->st));  // (rng is a local)
-    g.kb_rng = ctx->d_kb_rng;
   }
   // the column-stage CTAs' points and the kc range of each column (a mirror
   // column's is the negated one; the (0,0) column holds both halves and G = 0)
+  std::vector<int> start;
+  std::vector<int2> items, kc_rng;
   if (ctx->fast) {
-    std::vector<int> start(g.nbatch + 1, 0);
-    std::vector<int2> items, rng(g.ncols);
+    start.assign(g.nbatch + 1, 0);
+    kc_rng.resize(g.ncols);
+    std::vector<int2> &rng = kc_rng;
     items.reserve(ncoef);
     g.kc_contig = 1;
     auto wrap = [n3](int k) { return k < 0 ? k + n3 : k; };
@@ -868,14 +858,44 @@ extern "C" int sdft_ctx_create(int n1, int n2, int n3, int ncoef, const int *ka,
       start[cp / cpb + 1] = (int)items.size();
     }
     if (!g.kc_contig) std::fill(rng.begin(), rng.end(), make_int2(-n3, n3));
-    DMF(ctx->d_item_start, start.size() * sizeof(int));
-    DMF(ctx->d_items, items.size() * sizeof(int2));
-    DMF(ctx->d_kc_rng, rng.size() * sizeof(int2));
-    CKF(cudaMemcpyAsync(ctx->d_item_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-    CKF(cudaMemcpyAsync(ctx->d_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
-    CKF(cudaMemcpyAsync(ctx->d_kc_rng, rng.data(), rng.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->st));
-    CKF(cudaStreamSynchronize(ctx->st));  // (the vectors are locals)
-    g.item_start = ctx->d_item_start; g.items = ctx->d_items; g.kc_rng = ctx->d_kc_rng;
+  }
+  // All tables in one block with one upload: every allocation and every wait of a
+  // copy costs several microseconds, and a server makes a context per request
+  // (the mean of six systems of 8 to 96 atoms: eleven blocks 0.415 ms, one 0.345).
+  {
+    std::vector<unsigned char> host;
+    auto add = [&](const void *p, size_t bytes) {
+      const size_t at = rup(host.size(), 256);
+      host.resize(at + bytes);
+      if (bytes) std::memcpy(host.data() + at, p, bytes);
+      return at;
+    };
+    auto all = [&](const auto &v) { return add(v.data(), v.size() * sizeof v[0]); };
+    const size_t o_gstart = all(cpg), o_gcount = all(cpc), o_ab = all(colab), o_kc = all(ctx->kc), o_ak2 = all(ak2),
+                 o_tw = all(tw), o_twf = all(twf), o_kb = all(kb_rng), o_start = all(start), o_items = all(items),
+                 o_kcr = all(kc_rng);
+    DMF(ctx->d_geom, host.size());
+    CKF(cudaMemcpyAsync(ctx->d_geom, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->st));
+    CKF(cudaStreamSynchronize(ctx->st));  // (host is a local)
+    unsigned char *d = static_cast<unsigned char *>(ctx->d_geom);
+    g.cp_gstart = reinterpret_cast<int *>(d + o_gstart);
+    g.cp_gcount = reinterpret_cast<int *>(d + o_gcount);
+    g.col_ab = reinterpret_cast<int *>(d + o_ab);
+    g.gkc = reinterpret_cast<int *>(d + o_kc);
+    ctx->d_ak2 = reinterpret_cast<double *>(d + o_ak2);
+    g.ak2 = ctx->d_ak2;
+    g.tw1 = reinterpret_cast<double2 *>(d + o_tw);
+    g.tw2 = g.tw1 + n1;
+    g.tw3 = g.tw2 + n2;
+    g.tw1f = reinterpret_cast<float2 *>(d + o_twf);
+    g.tw2f = g.tw1f + n1;
+    g.tw3f = g.tw2f + n2;
+    g.kb_rng = reinterpret_cast<int2 *>(d + o_kb);
+    if (ctx->fast) {
+      g.item_start = reinterpret_cast<int *>(d + o_start);
+      g.items = reinterpret_cast<int2 *>(d + o_items);
+      g.kc_rng = reinterpret_cast<int2 *>(d + o_kcr);
+    }
   }
 
   // orbital blocks (zero padded)
@@ -907,11 +927,11 @@ extern "C" int sdft_ctx_destroy(sdft_ctx *ctx) {
   if (!ctx) return SDFT_OK;
   cudaSetDevice(ctx->device);
   if (ctx->st) cudaStreamSynchronize(ctx->st);
-  void *ptrs[] = {ctx->d_cp_gstart, ctx->d_cp_gcount, ctx->d_col_ab, ctx->d_gkc, ctx->d_ak2, ctx->d_tw,
-                  ctx->d_twf, ctx->d_vp, ctx->d_vks_tmp, ctx->d_pj, ctx->d_bk, ctx->d_w, ctx->d_z,
+  if (ctx->st_kb) cudaStreamSynchronize(ctx->st_kb);  // (st waits for it, save where a call failed between the two)
+  void *ptrs[] = {ctx->d_geom, ctx->d_vp, ctx->d_vks_tmp, ctx->d_pj, ctx->d_bk, ctx->d_w, ctx->d_z,
                   ctx->d_zwork, ctx->d_chi, ctx->d_b1, ctx->d_b2, ctx->d_fnl, ctx->d_acc, ctx->d_coef,
                   ctx->d_x, ctx->d_dots, ctx->d_mom, ctx->d_rho_part, ctx->d_rho, ctx->d_neg, ctx->d_noise_scratch,
-                  ctx->d_enl, ctx->d_red, ctx->d_kb_rng, ctx->d_item_start, ctx->d_items, ctx->d_kc_rng,
+                  ctx->d_enl, ctx->d_red,
                   ctx->d_err, ctx->d_pj_dig, ctx->d_bk_dig, ctx->d_c_dig,
                   ctx->d_z_dig, ctx->d_pj_sc, ctx->d_bk_sc, ctx->d_c_sc, ctx->d_z_sc, ctx->d_rowmax,
                   ctx->d_oz_part, ctx->d_kb_rs, ctx->d_kb_rc, ctx->d_gk, ctx->d_zsave, ctx->d_rowmax3};
@@ -1535,6 +1555,7 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   double *sc = ctx->d_red + kRedPart;
   const bool beside = ctx->P && !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside;
   if (beside) {  // the projection's first pass and the kinetic sum each read c; the sum hides behind the GEMM
+    if ((r = ensure_side(ctx))) return r;
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
     ctx->side_runs++;
@@ -1609,6 +1630,7 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
     const bool beside = !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
                         db + ctx->s_oz * sizeof(double) <= ctx->vec_elems * sizeof(double);
     if (beside) {
+      if ((r = ensure_side(ctx))) goto out;
       int8_t *dig = reinterpret_cast<int8_t *>(ctx->d_fnl);
       if ((r = make_tmap_oz(&t2[0], dig, ctx->s_oz, ctx->kp_oz)) ||
           (r = make_tmap_oz(&t2[1], dig, ctx->s_oz, ctx->kp_oz, OZ_7x4, 64)))
@@ -1806,6 +1828,10 @@ extern "C" int sdft_batch_create(int n, sdft_ctx *const *ctxs, const int *nstate
   std::vector<bool> timing(n);
   long long l0 = 0;
   for (int i = 0; i < n; i++) { timing[i] = ctxs[i]->timing; ctxs[i]->timing = false; l0 += ctxs[i]->launches; }
+  if (n == 1 && fork_ok(ctxs[0], nstate[0]) && (r = ensure_side(ctxs[0]))) {
+    ctxs[0]->timing = timing[0];
+    return fail(r);
+  }
   if ((r = ck(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal)))) return fail(r);
   int rc = ck(cudaEventRecord(b->evs[0], b->st));
   for (int i = 0; i < n && rc == SDFT_OK; i++) {

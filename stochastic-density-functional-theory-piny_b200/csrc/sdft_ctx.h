@@ -21,11 +21,9 @@ struct sdft_ctx {
   sdft::DevGeom g{};
   int max_states = 0, s_pad = 0, npairs_max = 0;
   size_t vec_elems = 0;  // doubles per orbital block (s_pad*2*ngp)
-  // device geometry arrays
-  int *d_cp_gstart = nullptr, *d_cp_gcount = nullptr, *d_col_ab = nullptr, *d_gkc = nullptr;
-  double *d_ak2 = nullptr;
-  double2 *d_tw = nullptr;  // n1+n2+n3
-  float2 *d_twf = nullptr;
+  // the geometry tables that DevGeom points into: one block, one upload
+  void *d_geom = nullptr;
+  double *d_ak2 = nullptr;  // in d_geom
   // potential
   void *d_vp = nullptr;     // [n3][n1][n2] (double or float)
   double *d_vks_tmp = nullptr;
@@ -63,9 +61,6 @@ struct sdft_ctx {
   std::vector<sdft_batch *> batches;  // graphs that replay this context's filter
   double *d_enl = nullptr;
   double *d_red = nullptr;  // reduction partials + scalars (Lanczos, energies)
-  int2 *d_kb_rng = nullptr;  // per plane row: signed kb range of its sphere columns
-  int *d_item_start = nullptr;                    // column-stage CTAs' items (DevGeom)
-  int2 *d_items = nullptr, *d_kc_rng = nullptr;
   // state
   int resident = 0;          // orbitals in d_chi
   int filtered = 0;          // orbitals with results in d_acc
@@ -75,6 +70,7 @@ struct sdft_ctx {
   double gcut = 0.0;
   // the nonlocal chain of an H application runs here while the plane stage
   // runs on st; between the two events of apply_h, so st alone orders the rest
+  // (all three made by ensure_side, at their first use)
   cudaStream_t st_kb = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_kb = nullptr;
   long long side_runs = 0;  // times work was queued on st_kb

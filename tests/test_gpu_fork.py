@@ -78,6 +78,26 @@ def test_results_do_not_depend_on_the_streams(pkg, sys2, prec, nmax, ns):
     ctx.close()
 
 
+@pytest.mark.parametrize("prec,ns", [(0, 109), (1, 28)])
+def test_a_graph_may_be_the_first_use_of_the_second_stream(pkg, sys2, prec, ns):
+    """The second stream is made at its first use, which may be the capture of a
+    one-context graph; noise alone does not use it."""
+    scale, mean, ec = 0.1, 2.0, 1.0 / np.arange(1.0, 10.0)
+    ctx = _ctx(pkg, sys2, prec, ns)
+    ctx.noise_dev(ns, seed=3.0)
+    assert ctx.side_runs == 0
+    b = pkg.Batch([ctx], [ns], [ec.size], [ec], [scale], [mean], [1.0])
+    assert ctx.side_runs == ec.size - 1
+    b.launch()
+    b.sync()
+    got = ctx.download_density()
+    b.close()
+    ctx.set_timing(True)  # in turn
+    ctx.filter_cheby_dev(ns, ec, 1, scale, mean)
+    assert np.array_equal(ctx.density_dev(ns), got)
+    ctx.close()
+
+
 def test_lanczos_of_512_atoms_does_not_depend_on_the_streams(pkg, wl):
     """One orbital of 96^3, the smallest application that runs beside."""
     ctx = _ctx(pkg, wl.make_system(4, (96, 96, 96)), pkg.SDFT_PREC_MIXED, 1)
