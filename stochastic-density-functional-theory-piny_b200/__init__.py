@@ -812,9 +812,11 @@ class Batch:
         _chk(lib.sdft_batch_sync(self._p))
 
     def set_plane_threads(self, nt):
-        """Threads per CTA of the FP32 plane stage: 128, 256, or 0 = the
-        library's default (128 for 48 x 48 to 72 x 72 planes, 256 otherwise)."""
-        _chk(lib.sdft_ctx_set_plane_threads(self._p, int(nt)))
+        """Threads per CTA of the FP32 plane stage (Context.set_plane_threads) on
+        every context of the batch, for their later calls and graphs; this graph
+        keeps what it was captured with."""
+        for c in self._ctxs:
+            c.set_plane_threads(nt)
 
     def set_priority(self, priority):
         """CUDA priority of the stream the graph is launched into; idle only."""
