@@ -5,6 +5,8 @@ mixed contexts on both sides of the digit GEMMs' size limit.
 FP64: sums of at most 1664 products in another order than the oracle's, 1e-12
 as for every FP64 H psi.  Mixed: FP32 transforms and, above the limit, 28-bit
 projections, 2e-7 as for every mixed H psi."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -99,6 +101,8 @@ def test_estimate_covers_either_form(pkg, wl, cells, grid, ns):
     serve = __import__(pkg.__name__ + ".serve", fromlist=["estimate_bytes"])
     s = wl.make_system(cells, grid)
     est = serve.estimate_bytes(s, ns)
+
+    gc.collect()  # contexts that earlier tests left would be released meanwhile
 
     def request(limit):
         pkg.set_device_memory_limit(0, pkg.device_memory_in_use(0) + int(limit))
