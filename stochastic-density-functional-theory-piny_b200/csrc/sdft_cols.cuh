@@ -39,7 +39,7 @@ namespace sdft {
 // transforms -- took 0.965 ms, 42.4 us at 48^3 and 64 pairs (28.7 now) and
 // 65.7 us at N3 = 24 with moment dots (19.3 now).  (All before the order of the
 // epilogue's loads, 682 -> 611 us, see epilogue_pair.)  Bound: 2.98 GB at 96^3,
-// 4.9 TB/s, 0.73 of a copy; the waits for those loads.
+// 4.9 TB/s, 0.75 of a copy; the waits for those loads.
 // FP64: 128 x 5 46.5 us at 72^3 and 32 pairs, 256 x 3 53.3, 192 x 4 49.0.
 template <typename T, int N3, int CPB> struct ColCfg {
   static constexpr int NL = 2 * CPB;

@@ -261,11 +261,6 @@ struct UnitIter {
   }
 };
 
-// Twiddle source of dif/dit: exp(-2 pi i t/N) from a shared-memory table
-// (pointer) or from an accessor object with operator()(t).
-template <typename C, typename P> __device__ __forceinline__ C tw_at(P *tw, int t) { return lds_tw(tw + t); }
-template <typename C, typename TW> __device__ __forceinline__ C tw_at(const TW &tw, int t) { return tw(t); }
-
 // Elements of a line that hold data (mask.line(l)(k) for natural index k of
 // line l): dif reads only those on input (the others count as zero and need
 // not be stored), dit writes only those on output.  AllElems: every element.
@@ -284,7 +279,7 @@ template <int R1> __device__ __forceinline__ constexpr bool band34(bool p34, int
   return p34 && R1 == 8 && (j1 == 3 || j1 == 4);
 }
 
-// natural -> permuted.  twN: exp(-2 pi i t/N) (shared-memory table or accessor).
+// natural -> permuted.  twN(t): exp(-2 pi i t/N) (TwC, sdft_tw_edges.cuh).
 template <int N, int ES, int DIR, bool P34 = false, typename C, typename LM, typename TW, typename MK = AllElems>
 __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN, int tid, int nthr,
                                     const MK &mask = MK{}, int es_rt = ES) {
@@ -308,7 +303,7 @@ __device__ __forceinline__ void dif(C *buf, const LM &lm, int nl, const TW &twN,
       p[j2 * es] = v[0];
 #pragma unroll
       for (int k1 = 1; k1 < R1; k1++) {
-        C w = tw_at<C>(twN, j2 * k1);
+        C w = twN(j2 * k1);
         if (DIR > 0) w.y = -w.y;
         p[(j2 + R2 * k1) * es] = cmul(v[k1], w);
       }
@@ -352,7 +347,7 @@ __device__ __forceinline__ void dit(C *buf, const LM &lm, int nl, const TW &twN,
       p[0] = v[0];
 #pragma unroll
       for (int j2 = 1; j2 < R2; j2++) {
-        C w = tw_at<C>(twN, j2 * k1);
+        C w = twN(j2 * k1);
         if (DIR > 0) w.y = -w.y;
         p[j2 * es] = cmul(v[j2], w);
       }

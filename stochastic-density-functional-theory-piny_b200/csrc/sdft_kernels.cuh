@@ -8,9 +8,9 @@ namespace sdft {
 
 // Column-pair batch of the column stages.
 constexpr int kCPB = 8;          // column pairs per CTA (16 columns), generic path
-// column pairs per CTA of the compile-time-edge column stages: 1.1 to 1.6
-// thousand points, so that a transform pass has one or two units per thread of
-// 128 and the item phase one or two points, at every edge
+// column pairs per CTA of the compile-time-edge column stages: 0.8 to 2.0
+// thousand points (1.2 to 2.0 from edge 36 on), 1 to 2.25 transform units per
+// thread of 128 and pass from edge 36 on, 1.5 to 4.5 below
 constexpr int col_cpb(int n3) { return n3 >= 72 ? 8 : (n3 >= 36 ? 16 : 32); }
 // and of the contexts whose orbitals would not fill the SMs with such CTAs
 constexpr int kCPBSmall = 8;

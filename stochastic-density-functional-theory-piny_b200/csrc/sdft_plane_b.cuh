@@ -70,9 +70,10 @@ kf_stage_b(DevGeom g, typename CT<T>::type *__restrict__ X, const T *__restrict_
 // ---------------------------------------------------------------------------
 // Plane edges with instances of their own: the 24-per-cell grids of one to
 // three cells per axis and 96 x 96, and the density grids' 32 and 64 and their
-// pairs with 96.  Every other pair takes the run-time-edge kernel
-// (sdft_planes.cu), which pays for its row pitch and the registers of the
-// largest radix: 64 x 64, 49 pairs, FP32, 58.0 us there and 46.8 here.
+// pairs with 96.  Every other pair -- also an uneven cell's 96 with 24, 48 or 72 --
+// takes the run-time-edge kernel (sdft_planes.cu), which pays for its row pitch
+// and the registers of the largest radix: 64 x 64, 49 pairs, FP32, 58.0 us there
+// and 46.8 here (the only pair timed both ways).
 #define SDFT_FOR_PLANE(X)                                                     \
   do {                                                                        \
     switch (g.n1 * 1000 + g.n2) {                                             \

@@ -89,7 +89,7 @@ __device__ __forceinline__ void plane_a_vmul(C2 *pl, int P2, int nl, int N2, con
     p[j2 * P2] = v[0];
 #pragma unroll
     for (int k1 = 1; k1 < R1; k1++) {
-      C2 w = tw_at<C2>(tw1, j2 * k1);
+      C2 w = tw1(j2 * k1);
       w.y = -w.y;
       p[(j2 + R2 * k1) * P2] = cmul(v[k1], w);
     }
@@ -109,7 +109,7 @@ __device__ __forceinline__ void plane_a_vmul(C2 *pl, int P2, int nl, int N2, con
     dftr<R2, -1>(v);
     p[0] = v[0];
 #pragma unroll
-    for (int j2 = 1; j2 < R2; j2++) p[j2 * P2] = cmul(v[j2], tw_at<C2>(tw1, j2 * k1));
+    for (int j2 = 1; j2 < R2; j2++) p[j2 * P2] = cmul(v[j2], tw1(j2 * k1));
   }
   __syncthreads();
 #pragma unroll 1
