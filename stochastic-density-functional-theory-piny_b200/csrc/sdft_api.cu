@@ -456,7 +456,7 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
 // among them 549.1 -> 546.1, 12 systems 62.9 -> 61.5.
 constexpr double kForkPoints = 8e5, kForkPointsF64 = 6e6;
 static bool fork_ok(const sdft_ctx *ctx, int nstate) {
-  return ctx->P && ctx->fast && !ctx->timing && !ctx->in_batch &&
+  return ctx->P && ctx->st_kb && ctx->fast && !ctx->timing && !ctx->in_batch &&
          (double)((nstate + 1) / 2) * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
 }
 
@@ -476,12 +476,19 @@ static int replace_stream(cudaStream_t *st, int priority) {
   return SDFT_OK;
 }
 
-// The second stream and its events, made when a call first wants them: a stream
-// takes 50 us to make and 50 to destroy (creating a context of 8 to 96 atoms, mean
-// of six: 0.345 ms with it, 0.287 without), and contexts of small systems and of graphs
-// of several never use it.  Not while a stream is captured.
+// Values of c from which the energies and forces run passes beside projections.
+// In turn -> beside: 512 atoms x 256 orbitals, both calls 2.43 -> 2.35 ms; 64 atoms
+// x 512 energies 120 -> 110 us, forces 310 -> 277; x 128 (1.7e6) 81 -> 74, 171 ->
+// 157; 8 atoms x 512 (8e5) 62 -> 64, forces 110 both.
+constexpr double kForceBeside = 1e6;
+
+// The second stream and its events, for contexts large enough that some call
+// uses them: a stream takes 50 us to make and 50 to destroy (creating a context
+// of 8 to 96 atoms, mean of six: 0.345 ms with it, 0.287 without), and a first
+// call that made it would take that longer.
 static int ensure_side(sdft_ctx *ctx) {
-  if (ctx->st_kb) return SDFT_OK;
+  const bool h = ctx->fast && (double)ctx->npairs_max * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
+  if (ctx->st_kb || !ctx->P || !(h || (double)ctx->max_states * 2 * ctx->ngp >= kForceBeside)) return SDFT_OK;
   if (!ctx->ev_fork) CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   if (!ctx->ev_kb) CK(cudaEventCreateWithFlags(&ctx->ev_kb, cudaEventDisableTiming));
   return replace_stream(&ctx->st_kb, ctx->priority - 1);
@@ -502,7 +509,6 @@ static int apply_h(sdft_ctx *ctx, const double *cur, int nstate, EpiArgs e, bool
   if ((r = ensure_x(ctx, npairs))) return r;  // (on st, so before the fork)
   const bool fork = fork_ok(ctx, nstate);
   if (fork) {
-    if ((r = ensure_side(ctx))) return r;
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
     ctx->side_runs++;
@@ -1144,7 +1150,9 @@ int sdft_build_kb_device(sdft_ctx *ctx, const sdft_kb_desc *kb);  // sdft_kb.cu
 extern "C" int sdft_ctx_set_kb(sdft_ctx *ctx, const sdft_kb_desc *kb) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   cudaSetDevice(ctx->device);
-  return sdft_build_kb_device(ctx, kb);
+  int r = sdft_build_kb_device(ctx, kb);
+  if (!r && (r = ensure_side(ctx))) sdft_build_kb_device(ctx, nullptr);
+  return r;
 }
 
 // ---- hot path ---------------------------------------------------------------
@@ -1555,11 +1563,6 @@ extern "C" int sdft_lanczos_bounds(sdft_ctx *ctx, int nstep, const double *v0re,
   return SDFT_OK;
 }
 
-// Values of c from which the energies and forces run passes beside projections.
-// In turn -> beside: 512 atoms x 256 orbitals, both calls 2.43 -> 2.35 ms; 64 atoms
-// x 512 energies 120 -> 110 us, forces 310 -> 277; x 128 (1.7e6) 81 -> 74, 171 ->
-// 157; 8 atoms x 512 (8e5) 62 -> 64, 110.
-constexpr double kForceBeside = 1e6;
 extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, double occ, int nsto_total,
                                        double *energy_ke, double *energy_pnl) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
@@ -1571,9 +1574,8 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   if (r) return r;
   const double *v = ctx->d_acc + (size_t)imu * ctx->vec_elems;
   double *sc = ctx->d_red + kRedPart;
-  const bool beside = ctx->P && !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside;
+  const bool beside = ctx->P && ctx->st_kb && !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside;
   if (beside) {  // the projection's first pass and the kinetic sum each read c; the sum hides behind the GEMM
-    if ((r = ensure_side(ctx))) return r;
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
     ctx->side_runs++;
@@ -1645,10 +1647,9 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
     OzDigits d[2] = {own, own};
     CUtensorMap t2[2];
     const size_t db = (size_t)kOzSlices * ctx->s_oz * ctx->kp_oz;
-    const bool beside = !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
+    const bool beside = ctx->st_kb && !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
                         db + ctx->s_oz * sizeof(double) <= ctx->vec_elems * sizeof(double);
     if (beside) {
-      if ((r = ensure_side(ctx))) goto out;
       int8_t *dig = reinterpret_cast<int8_t *>(ctx->d_fnl);
       if ((r = make_tmap_oz(&t2[0], dig, ctx->s_oz, ctx->kp_oz)) ||
           (r = make_tmap_oz(&t2[1], dig, ctx->s_oz, ctx->kp_oz, OZ_7x4, 64)))
@@ -1832,10 +1833,6 @@ extern "C" int sdft_batch_create(int n, sdft_ctx *const *ctxs, const int *nstate
   std::vector<bool> timing(n);
   long long l0 = 0;
   for (int i = 0; i < n; i++) { timing[i] = ctxs[i]->timing; ctxs[i]->timing = false; l0 += ctxs[i]->launches; }
-  if (n == 1 && fork_ok(ctxs[0], nstate[0]) && (r = ensure_side(ctxs[0]))) {
-    ctxs[0]->timing = timing[0];
-    return fail(r);
-  }
   if ((r = ck(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal)))) return fail(r);
   int rc = ck(cudaEventRecord(b->evs[0], b->st));
   for (int i = 0; i < n && rc == SDFT_OK; i++) {

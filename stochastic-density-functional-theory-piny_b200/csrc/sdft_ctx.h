@@ -70,7 +70,7 @@ struct sdft_ctx {
   double gcut = 0.0;
   // the nonlocal chain of an H application runs here while the plane stage
   // runs on st; between the two events of apply_h, so st alone orders the rest
-  // (all three made by ensure_side, at their first use)
+  // (all three made by ensure_side with the projectors, where some call can use them)
   cudaStream_t st_kb = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_kb = nullptr;
   long long side_runs = 0;  // times work was queued on st_kb

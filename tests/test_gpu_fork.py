@@ -79,8 +79,9 @@ def test_results_do_not_depend_on_the_streams(pkg, sys2, prec, nmax, ns):
 
 @pytest.mark.parametrize("prec,ns", [(0, 109), (1, 28)])
 def test_a_graph_may_be_the_first_use_of_the_second_stream(pkg, sys2, prec, ns):
-    """The second stream is made at its first use, which may be the capture of a
-    one-context graph; noise alone does not use it."""
+    """The second stream comes with the projectors, so that the capture of a
+    one-context graph may be its first use; noise alone does not use it, nor does
+    a context without projectors."""
     scale, mean, ec = 0.1, 2.0, 1.0 / np.arange(1.0, 10.0)
     ctx = _ctx(pkg, sys2, prec, ns)
     ctx.noise_dev(ns, seed=3.0)
@@ -94,6 +95,14 @@ def test_a_graph_may_be_the_first_use_of_the_second_stream(pkg, sys2, prec, ns):
     ctx.set_timing(True)  # in turn
     ctx.filter_cheby_dev(ns, ec, 1, scale, mean)
     assert np.array_equal(ctx.density_dev(ns), got)
+    ctx.set_timing(False)
+    n = ctx.side_runs
+    ctx.set_kb(None)
+    ctx.filter_cheby_dev(ns, ec, 1, scale, mean)
+    assert ctx.side_runs == n
+    ctx.set_kb(sys2["kb_desc"])
+    ctx.filter_cheby_dev(ns, ec, 1, scale, mean)
+    assert ctx.side_runs == n + ec.size - 1 and np.array_equal(ctx.density_dev(ns), got)
     ctx.close()
 
 
