@@ -415,8 +415,7 @@ enum {
 long long sdft_ctx_info(const sdft_ctx *ctx, int what);
 /* CUDA stream priority of the context's stream (lower = more urgent, 0 =
  * default; clamped to the device's range).  Call while the context is idle:
- * the stream is replaced (and the second stream that large H applications
- * run their projections on, which is one level more urgent).  A server gives cheap requests the urgent
+ * the stream is replaced.  A server gives cheap requests the urgent
  * priorities so they are not queued behind large ones on a shared GPU. */
 int sdft_ctx_set_priority(sdft_ctx *ctx, int priority);
 /* One CUDA graph running, for every context i (orbitals resident, V and KB

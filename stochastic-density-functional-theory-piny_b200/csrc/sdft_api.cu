@@ -297,9 +297,7 @@ static int default_plane_threads(const sdft_ctx *c) {
 // applications spend (per filter step: 64 atoms x 128 orbitals 116 -> 100 us, 8 x
 // 16 FP64 26.8 -> 17.4); at 512 atoms x 512 orbitals, 24576 planes, the waiting CTAs
 // cost 1 to 2 % instead, and in a graph of several systems they hold SMs that
-// another system's kernel could use (six uneven systems 2 % slower).  Graphs of one
-// system each replayed side by side do gain: 6 and 12 systems 60.9 -> 60.1 and 63.9
-// -> 62.8 ms, 16 the same.
+// another system's kernel could use (six uneven systems 2 % slower).
 constexpr long long kEarlyPlanes = 8192;
 static bool early_ok(const sdft_ctx *ctx, int nstate) {
   return !ctx->in_batch && (long long)((nstate + 1) / 2) * ctx->n3 <= kEarlyPlanes;
@@ -450,30 +448,13 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
 // pipe and a displaced round of plane CTAs can cost more than it hides (48^3 x 10
 // pairs 53 -> 59 us a step, 72 x 48 x 48 x 28 pairs 167 -> 184), up to 5.3e6,
 // against gains of 1 to 24 % from 6e6 on (cells of 8 to 512 atoms).  Not while kernels are
-// timed one by one, and not in a graph of several systems, which fill the SMs.
-// Graphs of one system each replayed side by side at the serving loop's
-// priorities still gain, 1 to 2 %: 16 systems 147.7 -> 145.2 ms, with 512-atom ones
-// among them 549.1 -> 546.1, 12 systems 62.9 -> 61.5.
+// timed one by one, and not where other systems fill the SMs: in a graph of
+// several, and in a context whose stream was given a priority, one of several at
+// work.
 constexpr double kForkPoints = 8e5, kForkPointsF64 = 6e6;
 static bool fork_ok(const sdft_ctx *ctx, int nstate) {
-  return ctx->P && ctx->st_kb && ctx->fast && !ctx->timing && !ctx->in_batch &&
+  return ctx->P && ctx->st_kb && ctx->fast && !ctx->timing && !ctx->in_batch && !ctx->shares &&
          (double)((nstate + 1) / 2) * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
-}
-
-// Replace an idle stream by one of the given CUDA priority (lower = more
-// urgent), clamped to the device's range.
-static int replace_stream(cudaStream_t *st, int priority) {
-  int least = 0, greatest = 0;
-  CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-  priority = std::min(least, std::max(greatest, priority));
-  cudaStream_t ns = nullptr;
-  CK(cudaStreamCreateWithPriority(&ns, cudaStreamNonBlocking, priority));
-  if (*st) {
-    cudaStreamSynchronize(*st);
-    cudaStreamDestroy(*st);
-  }
-  *st = ns;
-  return SDFT_OK;
 }
 
 // Values of c from which the energies and forces run passes beside projections.
@@ -483,15 +464,16 @@ static int replace_stream(cudaStream_t *st, int priority) {
 constexpr double kForceBeside = 1e6;
 
 // The second stream and its events, for contexts large enough that some call
-// uses them: a stream takes 50 us to make and 50 to destroy (creating a context
+// uses them (not once a priority was set): a stream takes 50 us to make and 50 to destroy (creating a context
 // of 8 to 96 atoms, mean of six: 0.345 ms with it, 0.287 without), and a first
 // call that made it would take that longer.
 static int ensure_side(sdft_ctx *ctx) {
   const bool h = ctx->fast && (double)ctx->npairs_max * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
-  if (ctx->st_kb || !ctx->P || !(h || (double)ctx->max_states * 2 * ctx->ngp >= kForceBeside)) return SDFT_OK;
+  if (ctx->st_kb || ctx->shares || !ctx->P || !(h || (double)ctx->max_states * 2 * ctx->ngp >= kForceBeside)) return SDFT_OK;
   if (!ctx->ev_fork) CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   if (!ctx->ev_kb) CK(cudaEventCreateWithFlags(&ctx->ev_kb, cudaEventDisableTiming));
-  return replace_stream(&ctx->st_kb, ctx->priority - 1);
+  CK(cudaStreamCreateWithPriority(&ctx->st_kb, cudaStreamNonBlocking, -1));
+  return SDFT_OK;
 }
 
 // st goes on when the nonlocal chain is done; stage C then has two kernels to
@@ -1574,7 +1556,7 @@ extern "C" int sdft_energy_chempot_dev(sdft_ctx *ctx, int nstate, int imu, doubl
   if (r) return r;
   const double *v = ctx->d_acc + (size_t)imu * ctx->vec_elems;
   double *sc = ctx->d_red + kRedPart;
-  const bool beside = ctx->P && ctx->st_kb && !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside;
+  const bool beside = ctx->P && ctx->st_kb && !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside;
   if (beside) {  // the projection's first pass and the kinetic sum each read c; the sum hides behind the GEMM
     CK(cudaEventRecord(ctx->ev_fork, ctx->st));
     CK(cudaStreamWaitEvent(ctx->st_kb, ctx->ev_fork, 0));
@@ -1647,7 +1629,7 @@ extern "C" int sdft_nl_force_dev(sdft_ctx *ctx, int nstate, int imu, double occ,
     OzDigits d[2] = {own, own};
     CUtensorMap t2[2];
     const size_t db = (size_t)kOzSlices * ctx->s_oz * ctx->kp_oz;
-    const bool beside = ctx->st_kb && !ctx->timing && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
+    const bool beside = ctx->st_kb && !ctx->timing && !ctx->shares && (double)nstate * 2 * ctx->ngp >= kForceBeside &&
                         db + ctx->s_oz * sizeof(double) <= ctx->vec_elems * sizeof(double);
     if (beside) {
       int8_t *dig = reinterpret_cast<int8_t *>(ctx->d_fnl);
@@ -1736,13 +1718,27 @@ extern "C" int sdft_ctx_set_gemm_split(sdft_ctx *ctx, int split) {
   return SDFT_OK;
 }
 
+// Replace an idle stream by one of the given CUDA priority (lower = more
+// urgent), clamped to the device's range.
+static int replace_stream(cudaStream_t *st, int priority) {
+  int least = 0, greatest = 0;
+  CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  priority = std::min(least, std::max(greatest, priority));
+  cudaStream_t ns = nullptr;
+  CK(cudaStreamCreateWithPriority(&ns, cudaStreamNonBlocking, priority));
+  if (*st) {
+    cudaStreamSynchronize(*st);
+    cudaStreamDestroy(*st);
+  }
+  *st = ns;
+  return SDFT_OK;
+}
+
 extern "C" int sdft_ctx_set_priority(sdft_ctx *ctx, int priority) {
   if (!ctx) return set_error(SDFT_ERR_ARG, "null context");
   cudaSetDevice(ctx->device);
-  int r = replace_stream(&ctx->st, priority);
-  if (r) return r;
-  ctx->priority = std::max(priority, -100);  // (no device has as many levels; one less must not overflow)
-  return ctx->st_kb ? replace_stream(&ctx->st_kb, ctx->priority - 1) : SDFT_OK;
+  ctx->shares = true;
+  return replace_stream(&ctx->st, priority);
 }
 
 struct sdft_batch {

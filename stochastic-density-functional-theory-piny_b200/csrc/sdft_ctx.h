@@ -74,7 +74,7 @@ struct sdft_ctx {
   cudaStream_t st_kb = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_kb = nullptr;
   long long side_runs = 0;  // times work was queued on st_kb
-  int priority = 0;       // of st; st_kb is one level more urgent, as far as the device goes
+  bool shares = false;    // stream priority set: one of several contexts at work
   bool in_batch = false;  // being captured into a graph with other contexts
   bool fast = false;  // compile-time-edge FFT kernels available
   bool fft64 = true;  // FFT scratch / V_KS in FP64 (plain form)

@@ -1,8 +1,9 @@
 """The nonlocal chain beside the plane stage, from 8e5 grid points times pairs
 on with the digit GEMMs and 6e6 with the FP64 one, and the digit passes and the
 kinetic sum beside the projections, from 1e6 values on.  While kernels are timed
-one by one they run in turn on one stream: the same kernels on the same data, so
-every result is equal bit for bit, also replayed from a graph, at any priority.  Each test checks which of the two ran by the
+one by one, and once the stream was given a priority, they run in turn on one
+stream: the same kernels on the same data, so every result is equal bit for bit,
+also replayed from a graph.  Each test checks which of the two ran by the
 context's count of work queued on its second stream."""
 import numpy as np
 import pytest
@@ -68,12 +69,12 @@ def test_results_do_not_depend_on_the_streams(pkg, sys2, prec, nmax, ns):
         b.sync()
         assert np.array_equal(ctx.download_density(), ref[-1])
     b.close()
-    for priority in (-2, 0, -9):  # no other effect than the streams' priorities (the last past their range)
+    n = ctx.side_runs
+    for priority in (-2, 0):  # either marks the context as one of several at work
         ctx.sync()
-        n = ctx.side_runs
         ctx.set_priority(priority)
         equal(results())
-        assert (ctx.side_runs > n) == beside
+    assert ctx.side_runs == n
     ctx.close()
 
 
