@@ -416,7 +416,12 @@ long long sdft_ctx_info(const sdft_ctx *ctx, int what);
 /* CUDA stream priority of the context's stream (lower = more urgent, 0 =
  * default; clamped to the device's range).  Call while the context is idle:
  * the stream is replaced.  A server gives cheap requests the urgent
- * priorities so they are not queued behind large ones on a shared GPU. */
+ * priorities so they are not queued behind large ones on a shared GPU.
+ * Any call, priority 0 included, also marks the context, for as long as it
+ * lives, as one of several at work on the device: its projections then stay on
+ * that one stream, where a context on its own runs large ones on a second
+ * stream beside the plane transforms.  Results are the same bit for bit; a
+ * context that has the device to itself is faster unmarked. */
 int sdft_ctx_set_priority(sdft_ctx *ctx, int priority);
 /* One CUDA graph running, for every context i (orbitals resident, V and KB
  * set), the Chebyshev filter of nstate[i] orbitals with the L[i]

@@ -582,7 +582,10 @@ class Context:
         _chk(lib.sdft_ctx_set_plane_threads(self._p, int(nt)))
 
     def set_priority(self, priority):
-        """CUDA priority of the context's stream (lower = more urgent); idle only."""
+        """CUDA priority of the context's stream (lower = more urgent); idle only.
+        Any call, 0 included, marks the context for good as one of several at work
+        on the device, which keeps its projections on that one stream: not for a
+        context that has the device to itself."""
         _chk(lib.sdft_ctx_set_priority(self._p, int(priority)))
 
     def lanczos_bounds(self, nstep=20, seed=15, margin=0.1, v0=None):

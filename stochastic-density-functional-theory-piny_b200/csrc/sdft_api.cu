@@ -297,7 +297,9 @@ static int default_plane_threads(const sdft_ctx *c) {
 // applications spend (per filter step: 64 atoms x 128 orbitals 116 -> 100 us, 8 x
 // 16 FP64 26.8 -> 17.4); at 512 atoms x 512 orbitals, 24576 planes, the waiting CTAs
 // cost 1 to 2 % instead, and in a graph of several systems they hold SMs that
-// another system's kernel could use (six uneven systems 2 % slower).
+// another system's kernel could use (six uneven systems 2 % slower).  Contexts of
+// their own at work at once keep it: the serving loop at 4 requests/s has a p50 of
+// 0.16 s with and 0.18 without, 48 requests at 50/s 1075 and 1100 orbitals/s.
 constexpr long long kEarlyPlanes = 8192;
 static bool early_ok(const sdft_ctx *ctx, int nstate) {
   return !ctx->in_batch && (long long)((nstate + 1) / 2) * ctx->n3 <= kEarlyPlanes;
@@ -450,7 +452,10 @@ static int run_kb(sdft_ctx *ctx, const double *vec, int nstate, bool want_enl, b
 // against gains of 1 to 24 % from 6e6 on (cells of 8 to 512 atoms).  Not while kernels are
 // timed one by one, and not where other systems fill the SMs: in a graph of
 // several, and in a context whose stream was given a priority, one of several at
-// work.
+// work.  The serving loop with it: 4 requests/s p50 0.16 -> 0.37 s, 64 requests
+// queued at once 777 -> 675 orbitals/s; its preparing and capturing wait for the
+// device longer (0.02 -> 0.1 s each), though the same graphs replayed side by side
+// with nothing else take 1 to 2 % less.
 constexpr double kForkPoints = 8e5, kForkPointsF64 = 6e6;
 static bool fork_ok(const sdft_ctx *ctx, int nstate) {
   return ctx->P && ctx->st_kb && ctx->fast && !ctx->timing && !ctx->in_batch && !ctx->shares &&
@@ -464,9 +469,9 @@ static bool fork_ok(const sdft_ctx *ctx, int nstate) {
 constexpr double kForceBeside = 1e6;
 
 // The second stream and its events, for contexts large enough that some call
-// uses them (not once a priority was set): a stream takes 50 us to make and 50 to destroy (creating a context
-// of 8 to 96 atoms, mean of six: 0.345 ms with it, 0.287 without), and a first
-// call that made it would take that longer.
+// uses them, unless a priority was set: a stream takes 50 us to make and 50 to
+// destroy (creating a context of 8 to 96 atoms, mean of six: 0.345 ms with it,
+// 0.287 without), and a first call that made it would take that longer.
 static int ensure_side(sdft_ctx *ctx) {
   const bool h = ctx->fast && (double)ctx->npairs_max * ctx->N >= (ctx->oz ? kForkPoints : kForkPointsF64);
   if (ctx->st_kb || ctx->shares || !ctx->P || !(h || (double)ctx->max_states * 2 * ctx->ngp >= kForceBeside)) return SDFT_OK;

@@ -46,7 +46,8 @@ def prepare(pkg, wl, s, nsto, L, precision, seed, device=0, tuner=None, mu=None,
     """Context with resident noise orbitals and filter coefficients for one
     system (steps 2 of the request life cycle).  mu, if given, replaces the
     bisection result (the moments are still computed); priority, if given,
-    is the CUDA priority of the context's stream."""
+    is the CUDA priority of the context's stream, which also marks the context as
+    one of several at work."""
     t = [time.perf_counter()]
     ctx = pkg.Context(*s["grid"], s["ka"], s["kb"], s["kc"], s["hmat"], precision=precision, max_states=nsto,
                       device=device)
@@ -185,7 +186,7 @@ class Server:
         tb = time.perf_counter()
         s = self.wl.build_spec(r["spec"])
         build_s = time.perf_counter() - tb
-        prio = request_priority(s["grid"], r["nsto"], r["L"]) if self.priorities else None
+        prio = request_priority(s["grid"], r["nsto"], r["L"]) if self.priorities else 0
         p = prepare(pkg, self.wl, s, r["nsto"], r["L"], self.precision, r["seed"], self.device, self.tuner,
                     mu=r.get("mu"), priority=prio)
         ctx = p["ctx"]
@@ -193,8 +194,7 @@ class Server:
             tc = time.perf_counter()
             if self.graph:  # one captured graph per request, replayed once
                 b = pkg.Batch([ctx], [r["nsto"]], [r["L"]], [p["ec"]], [p["scale"]], [p["emean"]], [p["occ_over"]])
-                if prio is not None:
-                    b.set_priority(prio)
+                b.set_priority(prio)
                 st = b.stream_ptr
                 b.launch()
             else:  # the same kernels issued directly on the context's stream (no capture / instantiation)

@@ -132,3 +132,34 @@ def test_tile_widths_are_timed_for_digit_gemms_only(pkg):
         t.tune(ctx, 40, 256)
         assert any(c[0] == "bn" for c in ctx.calls) == digits
         assert ("gemm_bn" in t.cache[t.key(ctx, 40, 256)]) == digits
+
+
+@pytest.mark.parametrize("priorities,want", [(True, -5), (False, 0)])
+def test_served_contexts_are_marked_as_several_at_work(serve, monkeypatch, priorities, want):
+    """A context without a priority counts as alone on the device and takes a
+    second stream, which slows the others' preparation: a server without stream
+    priorities gives every context the default one."""
+    class Stop(Exception):
+        pass
+
+    class Pkg:
+        @staticmethod
+        def set_device(device):
+            pass
+
+    class Wl:
+        @staticmethod
+        def build_spec(spec):
+            return spec
+
+    seen = []
+
+    def prepare(*a, priority=None, **k):
+        seen.append(priority)
+        raise Stop
+
+    monkeypatch.setattr(serve, "prepare", prepare)
+    srv = serve.Server(Pkg, Wl, 1, priorities=priorities)
+    with pytest.raises(Stop):
+        srv._start(0, dict(spec=dict(grid=(24, 24, 24)), nsto=16, L=128, seed=1.0), 0.0)
+    assert seen == [want]
