@@ -105,16 +105,17 @@ def setup_system(cfg_name, rank):
     return wl, cfg, s
 
 
-def algorithmic(kind, s, nsto, csz):
-    """Compulsory bytes (or flops) of one launch of `kind` over nsto orbitals.
+def algorithmic(kind, s, nsto, csz, digits):
+    """Compulsory bytes (or flops) of one launch of `kind` over nsto orbitals
+    (digits: the KB GEMMs are INT8 digit GEMMs, not FP64).
 
     stage A: read the orbitals (16 B/coef) + write the column scratch;
     stage B: read + write the column scratch + V_KS once;
     stage C: read the scratch, c and T_{k-2}, write T_k (FP64 orbitals);
-    read FNL (FP32 in mixed precision, FP64 otherwise); the filter sum is
+    read FNL (FP32 from the digit GEMMs, FP64 otherwise); the filter sum is
     read and written every other step (one orbital block per step on
-    average); mixed precision also packs the next step's columns (write one
-    column scratch) in place of a stage A launch;
+    average); it also packs the next step's columns (write one column scratch)
+    in place of a stage A launch;
     GEMMs: 2*P*nsto*2*ncoef flops."""
     npairs = (nsto + 1) // 2
     n1, n2, n3 = s["grid"]
@@ -127,9 +128,7 @@ def algorithmic(kind, s, nsto, csz):
     if kind == "stage_b_plane_fft_vks":
         return "hbm", 2 * xb + n1 * n2 * n3 * (csz // 2)
     if kind == "stage_c_cfft_unpack_recur":
-        if csz == 8:
-            return "hbm", 2 * xb + 4.5 * vec
-        return "hbm", xb + 5 * vec
+        return "hbm", 2 * xb + (4.5 if digits else 5) * vec
     if kind in ("kb_proj_gemm", "kb_back_gemm"):
         return "tensor", 2.0 * s["_P"] * nsto * 2 * ncoef
     if kind == "density_planes":
@@ -181,10 +180,10 @@ def fp64_gemm_peak(local):
     return 2.0 * n ** 3 / (best * 1e-3) / 1e12
 
 
-def rooflines(timing, s, nsto, mixed, back_products=10, fp64_peak=None):
+def rooflines(timing, s, nsto, mixed, back_products=10, fp64_peak=None, digits=None):
     """Roofline of every kernel function with an algorithmic model, largest
     total time first.  Tensor: the KB GEMMs (projection and back projection,
-    one kernel) -- mixed: int8 tcgen05 ops (10 digit products per FP64-
+    one kernel) -- digit GEMMs (digits; mixed contexts with enough projection work): int8 tcgen05 ops (10 digit products per FP64-
     equivalent multiply-add) against 2 x the measured bf16 burst peak (B200's
     dense int8 rate is twice its bf16 rate); FP64: DMMA flops against the
     FP64 tensor (DMMA) rate measured by fp64_gemm_peak (fp64_peak), else the
@@ -193,12 +192,13 @@ def rooflines(timing, s, nsto, mixed, back_products=10, fp64_peak=None):
     of the back projection (10, or 6 with the 24-bit digits of mixed_fast)."""
     pk, src = peaks()
     csz = 8 if mixed else 16
+    digits = mixed if digits is None else digits
     agg = {}
     for kind, (ms, n) in timing.items():
         kern = KERNEL_OF.get(kind)
         if kern is None or n == 0:
             continue
-        bound, work = algorithmic(kind, s, nsto, csz)
+        bound, work = algorithmic(kind, s, nsto, csz, digits)
         a = agg.setdefault(kern, [bound, 0.0, 0, 0.0, 0.0])
         a[1] += ms
         a[2] += n
@@ -218,7 +218,7 @@ def rooflines(timing, s, nsto, mixed, back_products=10, fp64_peak=None):
             if kern in PROFILED_LIMITER:
                 out[-1]["limiter"] = PROFILED_LIMITER[kern]
         else:
-            if mixed:
+            if digits:
                 ach = ops8 / t / 1e12
                 peak = 2.0 * pk["bf16_tflops"]
                 psrc = f"int8 dense = 2 x {src} bf16 burst ({pk['bf16_tflops']})"
@@ -230,10 +230,10 @@ def rooflines(timing, s, nsto, mixed, back_products=10, fp64_peak=None):
                         if fp64_peak else "nominal FP64 tensor (DMMA) rate")
                 name = "kb_gemm (k_gemm_nt_f64, DMMA)"
             out.append({"kernel": name, "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
-                        "frac": ach / peak, "traffic": PROFILED_GEMM_TRAFFIC.get((tuple(s["grid"]), mixed, nsto)),
+                        "frac": ach / peak, "traffic": PROFILED_GEMM_TRAFFIC.get((tuple(s["grid"]), digits, nsto)),
                         "peak_source": psrc, "ms_total": ms, "launches": n,
                         "fp64_equivalent_tflops": work / t / 1e12})
-            if mixed and pk.get("bf16_tflops_sustained"):
+            if digits and pk.get("bf16_tflops_sustained"):
                 # the same against the sustained bf16 loop (its clocks sat near 1.33 GHz under the
                 # power cap; this step runs near 1.75-1.8 GHz, so the burst figure is the stricter one)
                 out[-1]["frac_vs_sustained"] = ach / (2.0 * pk["bf16_tflops_sustained"])
@@ -498,15 +498,17 @@ def run_ours(args):
         f64f, fms64 = force_ms(c64)
         fmxf, fmsmx = force_ms(ctx)
         # four projections (c and i G_d c, d = x, y, z), each 2 P S (2 ncoef) FP64-equivalent flops;
-        # the mixed ones execute 10 int8 digit products per FP64-equivalent multiply-add
+        # digit GEMMs execute 10 int8 products per FP64-equivalent multiply-add
         pk, psrc = peaks()
         f_flops = 4 * 2.0 * s["_P"] * nsto * 2 * s["ncoef"]
         nl_force = {"natm": int(f64f.shape[0]), "ms_fp64": fms64, "ms_mixed": fmsmx,
                     "max_abs_err_mixed_vs_fp64_over_max_force":
                         float(np.abs(fmxf - f64f).max() / max(1e-300, np.abs(f64f).max())) if f64f.size else 0.0,
-                    "fp64_equiv_tflops_mixed": f_flops / (fmsmx * 1e-3) / 1e12,
-                    "frac_of_int8_peak_mixed": 10.0 * f_flops / (fmsmx * 1e-3) / 1e12 / (2.0 * pk["bf16_tflops"]),
-                    "peak_source": f"int8 dense = 2 x {psrc} bf16 burst ({pk['bf16_tflops']})"}
+                    "fp64_equiv_tflops_mixed": f_flops / (fmsmx * 1e-3) / 1e12}
+        if ctx.digit_gemms:
+            nl_force.update(
+                frac_of_int8_peak_mixed=10.0 * f_flops / (fmsmx * 1e-3) / 1e12 / (2.0 * pk["bf16_tflops"]),
+                peak_source=f"int8 dense = 2 x {psrc} bf16 burst ({pk['bf16_tflops']})")
         fp64 = {"orbitals_per_s": nsto * world / (ms64 / 1e3), "ms_per_step": ms64,
                 "mixed_speedup": (nsto * world / (ms64 / 1e3)) and value / (nsto * world / (ms64 / 1e3)),
                 "density_rel_l2_mixed_vs_fp64": float(np.linalg.norm(rhom - rho64) / np.linalg.norm(rho64)),
@@ -518,7 +520,7 @@ def run_ours(args):
 
     # ---- roofline: per kernel function, the dominant one first
     roof_all = rooflines(timing, s, nsto, prec != pkg.SDFT_PREC_FP64,
-                         back_products=6 if prec == pkg.SDFT_PREC_MIXED_FAST else 10)
+                         back_products=6 if prec == pkg.SDFT_PREC_MIXED_FAST else 10, digits=ctx.digit_gemms)
     roof = roof_all[0] if roof_all else None
     kernel_table = {k: {"ms_total": v[0], "launches": v[1], "share": v[0] / max(1e-9, sum(x[0] for x in
                     timing.values()))} for k, v in timing.items() if v[1]}
@@ -531,9 +533,10 @@ def run_ours(args):
         "metric": "filtered stochastic orbitals/s (512-atom Si, mixed vs FP64 GPU); p50/p99 latency",
         "value": value, "unit": "orbitals/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": tot_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": ("mixed(fp32 fft, int8-ozaki kb gemm, fp64 recurrence)" if prec == pkg.SDFT_PREC_MIXED else
-                  "mixed_fast(fp32 fft, int8-ozaki kb gemm with 24-bit back projection, fp64 recurrence)"
-                  if prec == pkg.SDFT_PREC_MIXED_FAST else "f64"),
+        "dtype": ("f64" if prec == pkg.SDFT_PREC_FP64 else
+                  "mixed(fp32 fft, fp64 kb gemm, fp64 recurrence)" if not ctx.digit_gemms else
+                  "mixed(fp32 fft, int8-ozaki kb gemm, fp64 recurrence)" if prec == pkg.SDFT_PREC_MIXED else
+                  "mixed_fast(fp32 fft, int8-ozaki kb gemm with 24-bit back projection, fp64 recurrence)"),
         "data": "synthetic (seeded Si supercell, Gaussian V_loc, Gaussian s+p KB, +-1 noise)",
         "config": {"workload": f"{args.config}: {s['natm']}-atom Si, grid {s['grid'][0]}x{s['grid'][1]}x{s['grid'][2]}, "
                                f"{nsto} orbitals/GPU, Chebyshev L={L}, ncoef={s['ncoef']}, P={s['_P']}",
