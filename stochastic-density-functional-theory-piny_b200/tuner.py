@@ -14,9 +14,12 @@ Three shapes are tuned per problem shape:
 * the CTA size of the FP32 plane FFT stage (one CTA per plane and orbital
   pair): 256 threads, or 128, which fits twice the CTAs per SM and can be
   faster on small planes (mixed contexts on the fast FFT path).
-Each candidate is timed (best of two) on a short Chebyshev filter of the
-context's resident orbitals: the filter kernels themselves, device time by
-CUDA events on the context stream, through the library's own event calls.
+Each candidate is timed (best of two) on a short Chebyshev filter + density of
+the context's resident orbitals, replayed as a graph: device time by CUDA events
+through the library's own event calls.  Not issued call by call: on small systems
+that takes as long as the host needs for the launches, whatever the shape (8
+atoms, 16 orbitals: 6 steps 0.110 ms at the library's split and 0.110 at 8, whose
+graph of 63 steps takes 0.99 ms instead of 0.89).
 The library's own choice (0) is a candidate in each list, and another is set
 only when it is more than 2 % faster, so timing noise cannot pick a slower
 shape.  Results are cached per problem shape (grid, coefficients to a ninth of
@@ -24,8 +27,8 @@ an octave, projectors, orbital tiles of 64, precision and the form of the
 projection GEMM with what sizes its workspace), in memory and optionally in a
 JSON file.
 
-Tuning overwrites the context's filter accumulators: run it before the real
-filter.
+Tuning overwrites the context's filter accumulators and density: run it before
+the real filter.
 """
 from __future__ import annotations
 
@@ -79,20 +82,22 @@ class Tuner:
         `reps` runs after a warm-up run."""
         ctx.set_gemm_split(split)
         ec = np.full(self.steps + 1, 1.0 / (self.steps + 1))
-        ctx.filter_cheby_dev(nstate, ec, 1, scale, emean)  # warm (buffers, caches)
+        g = self.pkg.Batch([ctx], [nstate], [ec.size], [ec], [scale], [emean], [1.0])
         a, b = self.pkg.Event(ctx.device), self.pkg.Event(ctx.device)
         try:
+            g.launch()  # warm (caches)
             best = float("inf")
             for _ in range(reps):
-                a.record(ctx.stream_ptr)
-                ctx.filter_cheby_dev(nstate, ec, 1, scale, emean)
-                b.record(ctx.stream_ptr)
-                ctx.sync()
+                a.record(g.stream_ptr)
+                g.launch()
+                b.record(g.stream_ptr)
+                g.sync()
                 best = min(best, a.elapsed_ms(b))
             return best
         finally:
             a.close()
             b.close()
+            g.close()
 
     def tune(self, ctx, nstate, nproj, scale=0.1, emean=0.0):
         """Pick and set the KB GEMM tile width, the projection split-K and

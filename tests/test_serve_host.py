@@ -163,3 +163,47 @@ def test_served_contexts_are_marked_as_several_at_work(serve, monkeypatch, prior
     with pytest.raises(Stop):
         srv._start(0, dict(spec=dict(grid=(24, 24, 24)), nsto=16, L=128, seed=1.0), 0.0)
     assert seen == [want]
+
+
+def test_candidates_are_timed_as_replayed_graphs(pkg):
+    """Not call by call, where a small system's launches by the host hide the shape."""
+    log = []
+
+    class Event:
+        def __init__(self, device):
+            pass
+
+        def record(self, stream):
+            log.append(("record", stream))
+
+        def elapsed_ms(self, other):
+            return 1.5
+
+        def close(self):
+            pass
+
+    class Batch:
+        stream_ptr = 7
+
+        def __init__(self, ctxs, nstate, L, coeffs, scale, emean, occ):
+            log.append(("graph", nstate[0], L[0], len(coeffs[0])))
+
+        def launch(self):
+            log.append("launch")
+
+        def sync(self):
+            log.append("sync")
+
+        def close(self):
+            log.append("close")
+
+    class Pkg:
+        pass
+
+    Pkg.Event, Pkg.Batch = Event, Batch
+    ctx = _Ctx(6500, 40, True)
+    ctx.device = 0
+    t = importlib.import_module(pkg.__name__ + ".tuner").Tuner(Pkg, steps=6)
+    assert t._time(ctx, 40, 4, 0.1, 0.0, reps=1) == 1.5
+    assert ctx.calls == [("split", 4)]
+    assert log == [("graph", 40, 7, 7), "launch", ("record", 7), "launch", ("record", 7), "sync", "close"]
