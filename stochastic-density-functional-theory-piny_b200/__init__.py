@@ -196,7 +196,9 @@ def _out(like, n):
     """An array like `like` whose first n values the call will write: not
     cleared first, since on a large result that costs as much as the copy that
     fills it (V_KS at 128^3, 16.8 MB: 1.13 ms a call with cleared arrays, 0.60
-    without; six filters of 48 to 216 atoms 6.3 and 5.8)."""
+    without; six filters of 48 to 216 atoms 6.3 and 5.8).  That is on repeated calls,
+    where the allocator hands back mapped pages; a page mapped anew is cleared by
+    the system either way."""
     a = np.empty_like(like)
     if a.size > n:
         a.reshape(-1)[n:] = 0.0
