@@ -508,30 +508,29 @@ k_gemm_nt_f64(const double *__restrict__ A, int lda, const double *__restrict__ 
 
 // Split partials summed per output: kRedZ threads share the splits of one output
 // (each a contiguous run, in order), then their sums are added in order.
-// Orbitals on grid.y, in steps of its limit where there are more.
+// Orbitals on grid.y, and on grid.z in steps of its limit where there are more.
 constexpr int kRedZ = 8, kMaxGridY = 65535;
 __global__ void __launch_bounds__(32 * kRedZ)
 k_split_reduce(const double *__restrict__ work, int split, size_t stride, int ldo, int Mst, int Nst,
                double *__restrict__ out) {
   const int m = blockIdx.x * 32 + threadIdx.x, z = threadIdx.y;
+  const int n = blockIdx.z * kMaxGridY + blockIdx.y;
+  const size_t idx = (size_t)n * ldo + m;
   const int z0 = split * z / kRedZ, z1 = split * (z + 1) / kRedZ;
   __shared__ double sh[kRedZ][32];
   pdl_trigger();
   pdl_wait();
-  for (int n = blockIdx.y; n < Nst; n += gridDim.y) {
-    const size_t idx = (size_t)n * ldo + m;
-    double s = 0.0;
-    if (m < Mst) {
+  if (n >= Nst) return;
+  double s = 0.0;
+  if (m < Mst) {
 #pragma unroll 4
-      for (int i = z0; i < z1; i++) s += work[i * stride + idx];
-    }
-    sh[z][threadIdx.x] = s;
-    __syncthreads();
-    if (z == 0 && m < Mst) {
-      for (int i = 1; i < kRedZ; i++) s += sh[i][threadIdx.x];
-      out[idx] = s;
-    }
-    __syncthreads();
+    for (int i = z0; i < z1; i++) s += work[i * stride + idx];
+  }
+  sh[z][threadIdx.x] = s;
+  __syncthreads();
+  if (z == 0 && m < Mst) {
+    for (int i = 1; i < kRedZ; i++) s += sh[i][threadIdx.x];
+    out[idx] = s;
   }
 }
 
@@ -828,8 +827,8 @@ int launch_gemm_nt_f64(const GemmPlan &p, bool early, const double *A, int lda, 
   }
 #undef SDFT_G
   if (p.split > 1)
-    launch_pdl(early, k_split_reduce, dim3((Mst + 31) / 32, std::min(Nst, kMaxGridY)), dim3(32, kRedZ), 0, st,
-               (const double *)work, p.split, stride, ldo, Mst, Nst, out);
+    launch_pdl(early, k_split_reduce, dim3((Mst + 31) / 32, std::min(Nst, kMaxGridY), (Nst + kMaxGridY - 1) / kMaxGridY),
+               dim3(32, kRedZ), 0, st, (const double *)work, p.split, stride, ldo, Mst, Nst, out);
   return p.split > 1 ? 2 : 1;
 }
 
